@@ -1,7 +1,8 @@
 // li_paged_attention: attention of the step's tokens over the paged cache,
 // chosen by dtype and batch shape.
 //
-//   float32                          -> general kernel (attention_generic.cu)
+//   float32                          -> the 32-bit kernel (attention_f32.cu): heads of up to 128 elements, a multiple of 4, one map a
+//                                       query row; the sizes decide, never the batch, so that a token's output does not depend on it
 //   bfloat16, every item one token   -> split-context decode kernel (attention_decode.cu)
 //   bfloat16, long portions          -> tcgen05 kernel (attention_tcgen05.cu): head_dim 64 or 128, a portion of
 //                                       at least 64 tokens in the batch
@@ -20,6 +21,10 @@
 int li_attention_generic(const void* qkv, void* out, const void* kcache, const void* vcache, int dtype, const int* block_table,
                          int max_blocks, const int* seq_of_token, const int* positions, int T, int nh, int nkv, int dh,
                          int page_size, int num_pages, float scale, int window, const AttentionOptions& opt, cudaStream_t stream);
+bool li_attention_f32_accepts(const void* qkv, const void* kcache, const void* vcache, int nh, int nkv, int dh, int page_size, const AttentionOptions& opt);
+int li_attention_f32(const void* qkv, void* out, const void* kcache, const void* vcache, const int* block_table, int max_blocks, const int* seq_of_token,
+                     const int* positions, int T, int nh, int nkv, int dh, int page_size, int num_pages, float scale, int window,
+                     const AttentionOptions& opt, cudaStream_t stream);
 bool li_attention_decode_accepts(int nh, int nkv, int dh, int page_size);
 int li_attention_decode(const void* qkv, void* out, const void* kcache, const void* vcache, const int* block_table, int max_blocks,
                         const int* ctx_lens, const int* old_lens, const int* q_start, int S, int nh, int nkv, int dh, int page_size, int num_pages,
@@ -116,6 +121,9 @@ LI_EXPORT int li_paged_attention(const void* qkv, void* out, const void* kcache,
                                           opt, &done, stream);
         if (rc || done) return rc;
     }
+    if (dtype == LI_F32 && li_attention_f32_accepts(qkv, kcache, vcache, nh, nkv, dh, page_size, opt))
+        return li_attention_f32(qkv, out, kcache, vcache, block_table, max_blocks, seq_of_token, positions, T, nh, nkv, dh, page_size, num_pages,
+                                scale, window, opt, stream);
     return li_attention_generic(qkv, out, kcache, vcache, dtype, block_table, max_blocks, seq_of_token, positions, T, nh, nkv, dh,
                                 page_size, num_pages, scale, window, opt, stream);
 }
@@ -124,7 +132,7 @@ LI_EXPORT int li_paged_attention(const void* qkv, void* out, const void* kcache,
 // last one, which is so when every sequence of the step is a request of its own.  The decode kernel may read those
 // keys while the kernel that writes the step's keys is still running.
 //
-// Force one implementation, for tests of each kernel alone: 0 general, 1 decode, 2 prefill (mma.sync), 3 prefill (tcgen05).
+// Force one implementation, for tests of each kernel alone: 0 general, 1 decode, 2 prefill (mma.sync), 3 prefill (tcgen05), 4 float32.
 // With `singles` 2 and 3 leave the sequences of one token to the decode kernel, as li_paged_attention does.
 LI_EXPORT int li_paged_attention_with(int which, const void* qkv, void* out, const void* kcache, const void* vcache, int dtype,
                                       const int* block_table, int max_blocks, const int* q_start, const int* ctx_lens,
@@ -139,6 +147,12 @@ LI_EXPORT int li_paged_attention_with(int which, const void* qkv, void* out, con
     if (which == 0)
         return li_attention_generic(qkv, out, kcache, vcache, dtype, block_table, max_blocks, seq_of_token, positions, T, nh, nkv,
                                     dh, page_size, num_pages, scale, window, opt, stream);
+    if (which == 4) {
+        LI_REQUIRE(dtype == LI_F32 && li_attention_f32_accepts(qkv, kcache, vcache, nh, nkv, dh, page_size, opt),
+                   "attention: the float32 kernel refuses heads=%d/%d head_dim=%d page=%d maps=%d", nh, nkv, dh, page_size, opt.maps);
+        return li_attention_f32(qkv, out, kcache, vcache, block_table, max_blocks, seq_of_token, positions, T, nh, nkv, dh, page_size, num_pages,
+                                scale, window, opt, stream);
+    }
     LI_REQUIRE(dtype == LI_BF16, "attention: implementation %d takes bfloat16 only", which);
     LI_REQUIRE(dh % (8 * maps) == 0, "attention: the tensor-core kernels take maps of multiples of 8 elements, not %d / %d", dh, maps);
     if (which == 1) {

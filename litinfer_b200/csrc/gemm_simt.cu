@@ -1,6 +1,5 @@
-// out[M, N] = a[M, K] w[N, K]^T (+ bias[N]) on the CUDA cores: the matrix
-// product of the true 32-bit path (no tensor-core mode that would round the
-// operands), and of sizes the tensor-core kernels refuse.
+// out[M, N] = a[M, K] w[N, K]^T (+ bias[N]) on the CUDA cores for bfloat16 operands
+// whose sizes the tensor-core kernels refuse.
 //
 // As LitInfer's linear (src/ops/linear/cpu/linear_cpu.cpp:45-60): both
 // operands row-major with K contiguous, accumulation in float, bias added in
@@ -84,9 +83,11 @@ static int launch(const void* a, const void* w, const float* bias, void* out, in
     return li_check_launch("linear (simt)");
 }
 
+int li_linear_f32(const float* a, const float* w, const float* bias, float* out, int M, int N, int K, cudaStream_t stream);
+
 int li_linear_simt(const void* a, const void* w, const float* bias, void* out, int dtype_in, int dtype_out, int M, int N, int K,
                    cudaStream_t stream) {
-    if (dtype_in == LI_F32 && dtype_out == LI_F32) return launch<float, float>(a, w, bias, out, M, N, K, stream);
+    if (dtype_in == LI_F32 && dtype_out == LI_F32) return li_linear_f32((const float*)a, (const float*)w, bias, (float*)out, M, N, K, stream);
     if (dtype_in == LI_BF16 && dtype_out == LI_BF16) return launch<bf16, bf16>(a, w, bias, out, M, N, K, stream);
     if (dtype_in == LI_BF16 && dtype_out == LI_F32) return launch<bf16, float>(a, w, bias, out, M, N, K, stream);
     return li_fail("linear: unsupported dtypes in=%d out=%d", dtype_in, dtype_out);

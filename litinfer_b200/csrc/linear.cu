@@ -1,6 +1,6 @@
 // li_linear: out[M, N] = a[M, K] w[N, K]^T (+ bias[N]), chosen by dtype and size.
 //
-//   float32            -> CUDA-core kernel (gemm_simt.cu), always: a true 32-bit product
+//   float32            -> CUDA-core kernels (gemm_f32.cu), always: a true 32-bit product
 //   bfloat16, M <= 64  -> decode is bound by reading every weight once: wide matrices go to
 //                         the tcgen05 kernel with swapped operands (gemv_tcgen05.cu), narrow
 //                         ones to the register-fed weight-streaming kernel (gemv_bf16.cu)

@@ -445,7 +445,7 @@ def rope_table(positions: torch.Tensor, denominators: torch.Tensor, out: torch.T
     _check(library().li_rope_table(_p(positions), _p(denominators), _i(half), _p(out), _i(T), _stream(out)), "rope_table")
 
 
-ATTENTION_IMPLEMENTATIONS = {"general": 0, "decode": 1, "prefill": 2, "prefill_tcgen05": 3}
+ATTENTION_IMPLEMENTATIONS = {"general": 0, "decode": 1, "prefill": 2, "prefill_tcgen05": 3, "float32": 4}
 
 
 def paged_attention(qkv: torch.Tensor, out: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor,
@@ -463,7 +463,7 @@ def paged_attention(qkv: torch.Tensor, out: torch.Tensor, k_cache: torch.Tensor,
     Queries are the first ``num_heads * head_dim`` columns of ``qkv`` (already
     rotated).  The token at position p of sequence s sees the cached keys
     ``max(0, p - window + 1) .. p`` of s, found through ``block_table[s]``.
-    ``implementation`` (``general``, ``decode``, ``prefill``, ``prefill_tcgen05``) forces one kernel, for
+    ``implementation`` (``general``, ``decode``, ``prefill``, ``prefill_tcgen05``, ``float32``) forces one kernel, for
     tests and measurements; it is an error if that kernel refuses the sizes.
     ``old_lens`` (int32 ``[S]``): how many keys of each sequence were in the cache before this step; needed when
     several sequences of the step are tokens of one request (None: all but each sequence's last key).

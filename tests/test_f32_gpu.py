@@ -1,0 +1,124 @@
+"""The kernels of the 32-bit path where they can go wrong: remainders of chunks, segments and tiles, every cut of the rows,
+operands that are not aligned, and attention against the general kernel with every option."""
+
+from __future__ import annotations
+
+import pytest
+import torch
+
+from test_kernels_gpu import make_attention_case
+
+pytestmark = pytest.mark.gpu
+
+EPS = 2.0 ** -24
+
+
+def K():
+    from litinfer_b200 import kernels
+    return kernels
+
+
+def on_device(c):
+    """The case of make_attention_case on the GPU; pages that no request holds are full of NaN."""
+    kc = torch.full((c["pages"], c["nkv"], c["page"], c["dh"]), float("nan"))
+    vc = torch.full((c["pages"], c["nkv"], c["dh"], c["page"]), float("nan"))
+    for s in range(c["S"]):
+        t = torch.arange(c["ctx_lens"][s])
+        pages, offs = c["bt"][s].long()[t // c["page"]], t % c["page"]
+        kc[pages.unique()], vc[pages.unique()] = 0.0, 0.0
+        kc[pages, :, offs], vc[pages, :, :, offs] = c["keys"][s], c["vals"][s]
+
+    def ints(x):
+        return torch.as_tensor(x, dtype=torch.int32).cuda()
+
+    return dict(qkv=c["qkv"].cuda(), k_cache=kc.cuda(), v_cache=vc.cuda(), block_table=ints(c["bt"]), q_start=ints(c["q_start"]),
+                ctx_lens=ints(c["ctx_lens"]), seq_of_token=ints(c["seq_of"]), positions=ints(c["pos"]))
+
+
+def product(a, w, bias):
+    out = torch.full((a.shape[0], w.shape[0]), float("nan"), dtype=torch.float32, device="cuda")
+    K().linear(a, w, bias, out)
+    return out
+
+
+def unaligned(t):
+    """The same values four bytes behind a 16-byte boundary."""
+    buf = torch.empty(t.numel() + 4, dtype=t.dtype, device=t.device)
+    view = buf[1:1 + t.numel()].view(t.shape)
+    view.copy_(t)
+    return view
+
+
+@pytest.mark.parametrize("N", [1, 33, 160, 1536, 4800])
+@pytest.mark.parametrize("Kd", [4, 7, 64, 68, 512, 1000, 1540, 4612, 8960])
+def test_product_every_cut_and_its_error(N, Kd):
+    g = torch.Generator(device="cuda").manual_seed(Kd * 7 + N)
+    a = torch.randn((150, Kd), generator=g, device="cuda")
+    w = torch.randn((N, Kd), generator=g, device="cuda")
+    bias = torch.randn(N, generator=g, device="cuda")
+    whole = product(a, w, bias)
+    exact = a.double() @ w.double().T + bias.double()
+    # a chain of 32 products, 16 chunks, the segments, the bias: each term is rounded at most that often
+    depth = 32 + 16 + -(-Kd // 512) + 1
+    bound = depth * EPS * (a.double().abs() @ w.double().abs().T + bias.double().abs())
+    assert bool(((whole.double() - exact).abs() <= bound).all())
+    for rows in (1, 3, 4, 5, 8, 9, 16, 17, 32, 33, 64, 65, 70, 81, 145):
+        assert torch.equal(product(a[:rows].contiguous(), w, bias), whole[:rows]), f"{rows} rows differ from 150"
+    last = product(a[149:].contiguous(), w, bias)
+    assert torch.equal(last, whole[149:])
+    assert torch.equal(product(unaligned(a[:3]), unaligned(w), bias), whole[:3])
+    assert torch.equal(product(a[:6].contiguous(), w, None) + bias, whole[:6])
+
+
+OPTIONS = [
+    {}, {"window": 70}, {"window": 33, "keep_first": 5}, {"window": 200, "keep_first": 150}, {"chunk": 48}, {"softcap": 20.0}, {"slopes": True},
+    {"sinks": True, "window": 1}, {"gate": "heads"}, {"gate": "elements", "slopes": True, "window": 130, "keep_first": 70},
+]
+
+
+@pytest.mark.parametrize("heads", [(12, 2, 128, 16), (4, 4, 16, 32), (9, 1, 36, 16), (20, 2, 64, 64)])
+@pytest.mark.parametrize("opt", OPTIONS, ids=str)
+def test_attention_against_the_general_kernel(heads, opt):
+    nh, nkv, dh, page = heads
+    for q_lens, ctx_lens in (([1, 1, 1], [1, 700, 65]), ([40, 1, 70], [40, 333, 150])):
+        c = on_device(make_attention_case(q_lens, ctx_lens, nh, nkv, dh, page, torch.float32, seed=3))
+        T = c["qkv"].shape[0]
+        g = torch.Generator(device="cuda").manual_seed(5)
+        kw = {k: opt[k] for k in ("keep_first", "chunk", "softcap") if k in opt}
+        if opt.get("slopes"):
+            kw["slopes"] = torch.rand(nh, generator=g, device="cuda") * 0.1
+        if opt.get("sinks"):
+            kw["sinks"] = torch.randn(nh, generator=g, device="cuda")
+        if opt.get("gate"):
+            elements = opt["gate"] == "elements"
+            kw.update(gate=torch.randn((T, nh * (dh if elements else 1)), generator=g, device="cuda"), gate_elements=elements)
+
+        def run(which, rows=None):
+            out = torch.full((T, nh * dh), float("nan"), device="cuda")
+            K().paged_attention(c["qkv"], out, c["k_cache"], c["v_cache"], c["block_table"], c["q_start"], c["ctx_lens"], c["seq_of_token"],
+                                c["positions"], nh, nkv, dh, dh ** -0.5, opt.get("window"), max(q_lens), max(ctx_lens), implementation=which, **kw)
+            return out
+
+        ref, got = run("general"), run("float32")
+        # probabilities and weighted sums of up to 700 keys, each in float32 on both sides, values about 1
+        assert torch.isfinite(got).all()
+        assert float((got - ref).abs().max()) <= 2e-5
+        assert torch.equal(run(None), got)
+
+
+def test_attention_does_not_depend_on_the_batch():
+    """A token alone (its units over a cluster of eight blocks) and among a hundred (one block): the same bits."""
+    nh, nkv, dh, page = 12, 2, 128, 16
+    c = on_device(make_attention_case([100], [2500], nh, nkv, dh, page, torch.float32, seed=8))
+
+    def run(lo, hi):
+        n = hi - lo
+        out = torch.empty((n, nh * dh), device="cuda")
+        K().paged_attention(c["qkv"][lo:hi].contiguous(), out, c["k_cache"], c["v_cache"], c["block_table"],
+                            torch.tensor([0, n], dtype=torch.int32, device="cuda"), c["ctx_lens"], c["seq_of_token"][lo:hi].contiguous(),
+                            c["positions"][lo:hi].contiguous(), nh, nkv, dh, dh ** -0.5, None, n, 2500, implementation="float32")
+        return out
+
+    whole = run(0, 100)
+    for lo, hi in ((0, 1), (57, 60), (99, 100)):
+        assert torch.equal(run(lo, hi), whole[lo:hi])
