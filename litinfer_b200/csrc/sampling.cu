@@ -19,7 +19,17 @@
 // (seed, index of the output token, i): exact sampling from the candidates'
 // softmax that depends on nothing outside the request.  The first maximum wins
 // ties (src/ops/argmax/op.cpp:28-33).  All sums are in a fixed order.
+//
+// Large vocabularies with a small top_k (sample_topk_kernel, the usual options): a cluster of blocks a row, one pass.  Each
+// thread keeps the maximum of its elements; the k-th largest of a block's thread maxima is a bound below the row's
+// k-th largest value, and only the few threads whose maximum reaches it are looked through again, by their whole warp.
+// The candidates, the sums over them (the same order, so the same bits) and the draw are those of the general kernel,
+// which takes whatever this one leaves (NaN, too many equal values, other options).  64 rows of 151,936, top-k 50 and
+// top-p 0.8: 20 us (two blocks a row); six passes by one block a row and 32 block-wide sums for the second threshold took
+// 136 us.
 #include "common.cuh"
+
+#include <cooperative_groups.h>
 
 namespace {
 
@@ -354,10 +364,183 @@ __device__ unsigned block_exclusive_scan(unsigned v, SelectShared& sh, unsigned*
     return r;
 }
 
+// The rows that sample_topk_kernel looks at (a vocabulary that leaves every thread of its blocks something).
+constexpr int kFastK = 256, kFastCand = 1024, kFastVocab = 16384;
+__device__ __forceinline__ bool fast_options(float temperature, int top_k, int V) {
+    return temperature > 0.0f && top_k > 1 && top_k <= kFastK && V >= kFastVocab;
+}
+
+struct FastShared {
+    unsigned key[kFastCand], okey[kFastCand];
+    int idx[kFastCand], oidx[kFastCand];
+    float e[kFastCand];
+    float x[kFastCand];
+    unsigned count, keep, keep_from;
+    float bound;                                          // this block's bound below the k-th largest (NaN: the row has one)
+    float fscratch[32];
+    Best scratch[32];
+};
+
+// out[r] = the row's token, or -1: sample_kernel, launched behind this one, takes the row.
+template <bool kVec>
+__global__ void __launch_bounds__(kThreads) sample_topk_kernel(const float* __restrict__ logits, const int* __restrict__ params, int* __restrict__ out, int V) {
+    namespace cg = cooperative_groups;
+    __shared__ FastShared sh;
+    cg::cluster_group cluster = cg::this_cluster();
+    pdl_launch_dependents();
+    pdl_wait();
+    const int blocks = (int)gridDim.x, rank = (int)blockIdx.x, r = (int)blockIdx.y;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int* pr = params + r * 6;
+    const float temperature = __int_as_float(pr[0]);
+    const int top_k = pr[1];
+    const float top_p = __int_as_float(pr[2]);
+    if (!fast_options(temperature, top_k, V)) {           // (the whole cluster agrees)
+        if (rank == 0 && tid == 0) out[r] = -1;
+        return;
+    }
+    const float* row = logits + (size_t)r * V;
+    const int per = ((V + blocks - 1) / blocks + 3) & ~3;
+    const int lo = min(V, rank * per), hi = min(V, lo + per);
+    // a thread's elements: four in a row at 4 (tid + 1024 j)
+    auto load4 = [&](int i) {
+        float4 v = make_float4(-INFINITY, -INFINITY, -INFINITY, -INFINITY);
+        if constexpr (kVec) {
+            if (i < hi) v = __ldcg(reinterpret_cast<const float4*>(row + i));
+        } else {
+            if (i < hi) v.x = __ldcg(row + i);
+            if (i + 1 < hi) v.y = __ldcg(row + i + 1);
+            if (i + 2 < hi) v.z = __ldcg(row + i + 2);
+            if (i + 3 < hi) v.w = __ldcg(row + i + 3);
+        }
+        return v;
+    };
+    if (tid == 0) sh.count = 0, sh.keep = 0, sh.keep_from = 0xFFFFFFFFu;
+    float mx = -INFINITY;
+    bool odd = false;
+    constexpr int U = 8;
+    for (int i0 = lo + 4 * tid; i0 < hi; i0 += U * 4 * kThreads) {
+        float4 v[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) v[u] = load4(i0 + u * 4 * kThreads);
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            mx = fmaxf(mx, fmaxf(fmaxf(v[u].x, v[u].y), fmaxf(v[u].z, v[u].w)));
+            odd |= (v[u].x != v[u].x) | (v[u].y != v[u].y) | (v[u].z != v[u].z) | (v[u].w != v[u].w);
+        }
+    }
+    // the top_k-th largest of the block's thread maxima
+    const unsigned mkey = sortable(mx);
+    unsigned a = 0, b = 0xFFFFFFFFu;
+    while (a < b) {
+        const unsigned mid = a + ((b - a) >> 1);
+        if (__syncthreads_count(mkey > mid) < top_k) b = mid;
+        else a = mid + 1;
+    }
+    const bool any_odd = __syncthreads_or(odd);
+    if (tid == 0) sh.bound = any_odd ? __int_as_float(0x7fc00000) : unsortable(a);
+    cluster.sync();
+    float bound = -INFINITY;
+    bool give_up = false;
+    for (int k = 0; k < blocks; ++k) {
+        const float o = *cluster.map_shared_rank(&sh.bound, k);
+        give_up |= o != o;
+        bound = fmaxf(bound, o);
+    }
+    // Candidates are chosen by z = x / temperature, which may round different x together: elements a few units in the last
+    // place below the bound are looked at too.  (Where z overflows or becomes so small that more falls together, or the bound
+    // says nothing, the general kernel decides.)
+    const float zb = fabsf(bound / temperature);
+    give_up |= !(fabsf(bound) < INFINITY) || !(zb < 1e30f) || (bound != 0.0f && zb < 1e-30f) || (bound == 0.0f && !(temperature < 1e30f));
+    const float from = bound - fabsf(bound) * 1e-6f;
+    if (!give_up) {
+        FastShared* first = cluster.map_shared_rank(&sh, 0);
+        unsigned flagged = __ballot_sync(0xffffffffu, mx >= from);
+        while (flagged) {
+            const int l = __ffs(flagged) - 1;
+            flagged &= flagged - 1;
+            const int t = (tid & ~31) + l;
+            for (int i = lo + 4 * t + lane * 4 * kThreads; i < hi; i += 32 * 4 * kThreads) {
+                const float4 v = load4(i);
+                const float x[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+                for (int q = 0; q < 4; ++q)
+                    if (x[q] >= from && i + q < hi) {
+                        const unsigned at = atomicAdd(&first->count, 1u);
+                        if (at < (unsigned)kFastCand) first->x[at] = x[q], first->idx[at] = i + q;
+                    }
+            }
+        }
+    }
+    cluster.sync();
+    if (rank != 0) return;
+    const int n = (int)sh.count;
+    if (give_up || n > kFastCand || n < top_k) {          // (uniform)
+        if (tid == 0) out[r] = -1;
+        return;
+    }
+    const unsigned key = tid < n ? sortable(sh.x[tid] / temperature) : 0u;
+    const int idx = tid < n ? sh.idx[tid] : 0;
+    sh.key[tid] = key;
+    __syncthreads();
+    int above = 0;
+    for (int j = 0; j < n; ++j) above += sh.key[j] > key ? 1 : 0;
+    const bool stays = tid < n && above < top_k;          // the k-th largest and what equals it stay together
+    __syncthreads();
+    sh.idx[tid] = stays ? idx : -1;
+    __syncthreads();
+    // in the order of the general kernel: by the element's place modulo 1024, then by the element
+    if (stays) {
+        int before = 0;
+        for (int j = 0; j < n; ++j) {
+            const int o = sh.idx[j];
+            before += (o >= 0 && ((o & (kThreads - 1)) < (idx & (kThreads - 1)) || ((o & (kThreads - 1)) == (idx & (kThreads - 1)) && o < idx))) ? 1 : 0;
+        }
+        sh.okey[before] = key;
+        sh.oidx[before] = idx;
+    }
+    const int C = __syncthreads_count(stays);
+    const unsigned mine = tid < C ? sh.okey[tid] : 0u;
+    // the largest of all: z of the row's maximum
+    if (tid < C) atomicMax(&sh.keep, mine);
+    __syncthreads();
+    const float zmax = unsortable(sh.keep);
+    unsigned keep_from = 0;
+    if (top_p > 0.0f && top_p < 1.0f) {
+        const float e = tid < C ? expf(unsortable(mine) - zmax) : 0.0f;
+        sh.e[tid] = e;
+        const float target = top_p * block_sum(e, sh.fscratch);      // (its barriers also publish sh.e)
+        // The smallest threshold whose mass above it is below the target is one of the candidates' keys: a warp a key, its
+        // sum in the order of block_sum.
+        for (int j = warp; j < C; j += kThreads / 32) {
+            const unsigned t = sh.okey[j];
+            float part = 0.0f;
+            for (int g = 0; 32 * g < C; ++g) {
+                const int q = 32 * g + lane;
+                const float v = warp_sum(q < C && sh.okey[q] > t ? sh.e[q] : 0.0f);
+                if (lane == g) part = v;
+            }
+            const float mass = warp_sum(part);
+            if (lane == 0 && mass < target) atomicMin(&sh.keep_from, t);
+        }
+        __syncthreads();
+        keep_from = sh.keep_from;
+    }
+    const unsigned long long seed = (unsigned long long)(unsigned)pr[3] | ((unsigned long long)(unsigned)pr[4] << 32);
+    const unsigned long long hash = splitmix64(seed ^ splitmix64((unsigned long long)(long long)pr[5]));
+    Best best{-INFINITY, 0x7fffffff};
+    if (tid < C && mine >= keep_from) {
+        const float v = unsortable(mine) + gumbel(hash, sh.oidx[tid]);
+        if (v > best.v) best = Best{v, sh.oidx[tid]};
+    }
+    best = block_best(best, sh.scratch);
+    if (tid == 0) out[r] = best.i == 0x7fffffff ? -1 : best.i;
+}
+
 // chunked_plain: rows with temperature alone are drawn by sample_temperature_chunks_kernel, launched after this kernel; here
 // they only get the first maximum as a stand-in (which stays if the row has nothing finite).
 __global__ void __launch_bounds__(kThreads) sample_kernel(const float* __restrict__ logits, const int* __restrict__ params,
-                                                          int* __restrict__ out, int V, int chunked_plain) {
+                                                          int* __restrict__ out, int V, int chunked_plain, int fast) {
     __shared__ Best scratch[32];
     __shared__ float fscratch[32];
     __shared__ SelectShared sh;
@@ -373,6 +556,7 @@ __global__ void __launch_bounds__(kThreads) sample_kernel(const float* __restric
     const unsigned long long index = (unsigned long long)(long long)pr[5];
 
     const bool use_k = top_k > 0 && top_k < V, use_p = top_p > 0.0f && top_p < 1.0f;
+    if (fast && fast_options(temperature, top_k, V) && out[r] >= 0) return;
     if (chunked_plain && temperature > 0.0f && top_k != 1 && !use_k && !use_p) {
         if (threadIdx.x == 0) out[r] = 0;                // stands only if the row has nothing finite (what the first maximum would give)
         return;
@@ -480,7 +664,17 @@ LI_EXPORT int li_sample(const float* logits, const int* params, int* out, int R,
     if (R == 0) return 0;
     // few rows of a large vocabulary: rows with temperature alone are drawn over many CTAs by a second kernel
     const int chunked_plain = (R <= 64 && R <= kChunkRows && V >= 16384) ? 1 : 0;
-    li_launch_pdl(sample_kernel, dim3(R), dim3(kThreads), 0, stream, logits, params, out, V, chunked_plain);
+    // rows with a small top-k: two to eight blocks a row, as many as fill the GPU once (from 65 rows on one block a row does)
+    const int fast = (R <= 64 && V >= kFastVocab) ? 1 : 0;
+    if (fast) {
+        const int blocks = R > 32 ? 2 : R > 16 ? 4 : 8;
+        if (V % 4 == 0 && (uintptr_t)logits % 16 == 0)
+            li_launch_pdl(sample_topk_kernel<true>, dim3(blocks, R), dim3(kThreads), 0, stream, dim3(blocks, 1, 1), logits, params, out, V);
+        else
+            li_launch_pdl(sample_topk_kernel<false>, dim3(blocks, R), dim3(kThreads), 0, stream, dim3(blocks, 1, 1), logits, params, out, V);
+        if (int rc = li_check_launch("sample (top-k)")) return rc;
+    }
+    li_launch_pdl(sample_kernel, dim3(R), dim3(kThreads), 0, stream, logits, params, out, V, chunked_plain, fast);
     if (int rc = li_check_launch("sample")) return rc;
     if (chunked_plain) {
         li_launch_pdl(sample_temperature_chunks_kernel, dim3(kDrawChunks, R), dim3(256), 0, stream, logits, params, out, V);

@@ -1,0 +1,82 @@
+"""Branches that a rule on sizes or options chooses, against the general way to the same result."""
+
+from __future__ import annotations
+
+import pytest
+import torch
+
+import test_kernels_gpu as T
+
+pytestmark = pytest.mark.gpu
+
+
+def K():
+    from litinfer_b200 import kernels
+    return kernels
+
+
+def params(rows):
+    """(temperature, top_k, top_p, seed, output index) per row, as the sampler packs them."""
+    out = torch.zeros((len(rows), 6), dtype=torch.int32)
+    f = out.view(torch.float32)
+    for i, (temperature, top_k, top_p, seed, index) in enumerate(rows):
+        f[i, 0], out[i, 1], f[i, 2], out[i, 3], out[i, 5] = temperature, top_k, top_p, seed, index
+    return out.cuda()
+
+
+@pytest.mark.parametrize("R", [64, 32, 7])
+@pytest.mark.parametrize("V", [16384, 16387, 50001, 151936])
+def test_top_k_by_a_cluster_is_the_general_kernels_token(V, R):
+    """Up to 64 rows the rows with a small top-k go to the kernel with several blocks a row; 65 and more go to the general one."""
+    g = torch.Generator(device="cuda").manual_seed(V + R)
+    x = torch.randn((R, V), generator=g, device="cuda") * 2.5
+    options = [(0.7, 50, 0.8), (1.0, 256, 1.0), (0.3, 2, 0.999), (1.3, 20, 0.1), (1.0, 257, 0.9), (0.0, 50, 0.8), (1.0, 1, 1.0), (0.9, 0, 0.9), (1.0, 0, 1.0),
+               (1e-6, 50, 0.8), (1e30, 50, 0.8)]
+    rows = [(*options[i % len(options)], 100 + i, i) for i in range(R)]
+    # rows in which thresholds meet equal values, masks, infinities and no numbers (the options of those rows differ with R)
+    x[1] = x[1].round()                                  # hundreds of equal values at the threshold
+    x[2, V // 3:] = torch.finfo(torch.float32).min
+    x[3, 100:] = float("-inf")
+    x[4] = 1.5
+    x[5, 17] = float("inf")
+    x[6, V - 1] = float("nan")
+    if R > 8:
+        rows[8:14] = [(0.7, 50, 0.8, 5, 1)] * 6
+        x[8] = x[8].round()
+        x[9, 30:] = torch.finfo(torch.float32).min       # fewer than top_k that are not masked
+        x[10] = 0.0
+        x[11, 3] = float("nan")
+        x[12, V - 1] = float("inf")
+        x[13] = float("-inf")
+    p = params(rows)
+    got = torch.full((R,), -7, dtype=torch.int32, device="cuda")
+    K().sample(x, p, got)
+    more = -(-65 // R)
+    ref = torch.full((R * more,), -7, dtype=torch.int32, device="cuda")
+    K().sample(x.repeat(more, 1), p.repeat(more, 1), ref)
+    assert got.tolist() == ref[:R].tolist()
+
+
+@pytest.mark.parametrize("cfg", [(28, 4, 128, 264, 1800), (40, 8, 128, 136, 1300), (28, 4, 128, 264, 2049)])
+def test_rotation_in_the_epilogue_of_wide_long_steps(cfg):
+    """q|k|v of so many rows that the plain product would go to the persistent kernel."""
+    T.test_linear_rope_kv_fused(torch.bfloat16, cfg)
+
+
+@pytest.mark.parametrize("shape", [(640, 15360, 4224), (520, 13000, 4168), (769, 12800, 5120)])
+@pytest.mark.parametrize("epilogue", [None, "swiglu"])
+def test_product_with_a_long_k_on_either_side_of_the_persistent_rule(shape, epilogue):
+    M, N, Kd = shape
+    N -= N % 16
+    g = torch.Generator(device="cuda").manual_seed(M)
+    a = torch.randn((M, Kd), generator=g, device="cuda").to(torch.bfloat16)
+    w = (torch.randn((N, Kd), generator=g, device="cuda") * Kd ** -0.5).to(torch.bfloat16)
+    ref = a.float() @ w.float().T
+    if epilogue:
+        r = ref.view(M, N // 16, 2, 8)
+        ref = (torch.nn.functional.silu(r[:, :, 0]) * r[:, :, 1]).reshape(M, N // 2)
+    out = torch.full(ref.shape, float("nan"), dtype=torch.bfloat16, device="cuda")
+    K().linear(a, w, None, out, epilogue=epilogue)
+    assert torch.isfinite(out).all()
+    # one rounding to bfloat16 of a float32 sum; the sums themselves are within a few 1e-6 of each other
+    assert bool(((out.float() - ref).abs() <= 2.0 ** -8 * ref.abs() + 1e-3).all())
