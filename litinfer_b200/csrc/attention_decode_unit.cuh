@@ -199,6 +199,7 @@ __device__ __forceinline__ void decode_attention_unit(int split, int kvh, int s,
         }
     }
     sync();
+    const bool alone = k_begin <= lo && k_end == ctx;      // the only unit of its sequence and key/value head: nothing to merge
     // partial layout per (sequence, head, split): DH floats of O, then m, l
     for (int e = tid; e < G * DH; e += kWarps * 32) {
         const int r = e / DH, d = e - r * DH;
@@ -212,12 +213,29 @@ __device__ __forceinline__ void decode_attention_unit(int split, int kvh, int s,
             O += sm_o[((size_t)w * G + r) * DH + d] * f;
             L += sm_l[w * 16 + r] * f;
         }
+        if (alone) {
+            if constexpr (kMod)
+                if (mod.sinks) {
+                    const float sink = mod.sinks[kvh * G + r], M2 = fmaxf(M, sink), f = expf(M - M2);
+                    O *= f;
+                    L = L * f + expf(sink - M2);
+                }
+            float res = L > 0.0f ? O / L : 0.0f;
+            if constexpr (kMod)
+                if (mod.gate) res *= mod.gate_of(tok, kvh * G + r, DH, d);
+            out[((size_t)tok * nh + kvh * G + r) * DH + d] = __float2bfloat16_rn(res);
+            continue;
+        }
         float* dst = part + (((size_t)s * nh + kvh * G + r) * nsplit + split) * (DH + 2);
         dst[d] = O;
         if (d == 0) {
             dst[DH] = M;
             dst[DH + 1] = L;
         }
+    }
+    if (alone) {
+        sync();                                            // (the fused step's next unit writes the scratch)
+        return;
     }
     // the CTA that finishes last for this (sequence, kv head) merges the splits, in split order
     int first, last;
