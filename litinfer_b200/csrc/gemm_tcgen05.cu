@@ -579,25 +579,22 @@ int launch(const void* a, const void* w, const float* bias, void* out, int M, in
 
 int g_forced_tile = 0;
 
-// whether `launch` takes paired tiles (one accumulator a CTA) for this shape by itself
-bool pair_tiles_chosen(int M, int N, int K) {
-    const long long big_ctas = (long long)ceil_div(M, 256) * ceil_div(N, 256);
-    const long long pair_ctas = (long long)((ceil_div(M, 128) + 1) & ~1) * ceil_div(N, 256);
-    (void)K;
-    return g_forced_tile == 0 && g_forced_ksplit == 0 && big_ctas < 120 && pair_ctas >= 74 && M > 128;
-}
-
 }  // namespace
 
-// The q|k|v product with rotary encoding and the cache writes as its epilogue (rope_epilogue.cuh): where the shape takes
-// the paired tiles anyway, and on single 128 x 128 tiles (a head each) for steps too short for those: there the two
+// The q|k|v product with rotary encoding and the cache writes as its epilogue (rope_epilogue.cuh): on paired tiles where
+// there are enough of them (also where the plain product would go to the persistent kernel: 2,048 rows, N 4608, K 3584
+// that kernel and the two behind it took 63 + 28 + 17 us), and on single 128 x 128 tiles (a head each) for steps too short for those: there the two
 // kernels that would rotate and write the cache cost more than the narrower column tiles of the plain product gain.
 int g_rope_single_tiles = 1;      // 0: the rope epilogue only on paired tiles (measurements)
 LI_EXPORT void li_tcgen05_rope_single_tiles(int on) { g_rope_single_tiles = on; }
 
+static bool rope_pairs(int M, int N) {
+    return g_forced_tile == 0 && g_forced_ksplit == 0 && M > 128 && (long long)((ceil_div(M, 128) + 1) & ~1) * ceil_div(N, 256) >= 74;
+}
+
 bool li_tcgen05_rope_wanted(const void* a, const void* w, const void* out, int M, int N, int K) {
-    if (!li_tcgen05_accepts(a, w, out, LI_BF16, M, N, K) || N % 128 != 0 || li_tcgen05_persistent_wanted(M, N, K)) return false;
-    return g_forced_tile == 0 && g_forced_ksplit == 0 && (g_rope_single_tiles || pair_tiles_chosen(M, N, K));
+    if (!li_tcgen05_accepts(a, w, out, LI_BF16, M, N, K) || N % 128 != 0) return false;
+    return rope_pairs(M, N) || (g_forced_tile == 0 && g_forced_ksplit == 0 && g_rope_single_tiles && !li_tcgen05_persistent_wanted(M, N, K));
 }
 
 int li_linear_tcgen05_rope(const void* a, const void* w, const float* bias, void* out, int M, int N, int K, const RopeEpilogue& rope,
@@ -605,7 +602,7 @@ int li_linear_tcgen05_rope(const void* a, const void* w, const float* bias, void
     LI_REQUIRE(li_tcgen05_rope_wanted(a, w, out, M, N, K), "linear + rope (tcgen05): refuses M=%d N=%d K=%d", M, N, K);
     LI_REQUIRE(N == (rope.nh + 2 * rope.nkv) * 128 && rope.cos_sin && rope.slot_mapping && rope.kcache && rope.vcache,
                "linear + rope (tcgen05): N=%d does not match %d + 2 x %d heads of 128, or a null operand", N, rope.nh, rope.nkv);
-    if (pair_tiles_chosen(M, N, K)) return launch_tile<128, 256, bf16, false, true, true>(a, w, bias, out, M, N, K, stream, 1, rope);
+    if (rope_pairs(M, N)) return launch_tile<128, 256, bf16, false, true, true>(a, w, bias, out, M, N, K, stream, 1, rope);
     return launch_tile<128, 128, bf16, false, false, true>(a, w, bias, out, M, N, K, stream, 1, rope);
 }
 
