@@ -9,15 +9,22 @@
 // Grid (tiles of 128 weight rows, splits of k).  Warp 0: producer (TMA), warp 1:
 // tensor-memory allocation and MMA issue, warps 2-5: epilogue.  The weight tiles of
 // the first stages are requested before griddepcontrol.wait (weights do not depend
-// on the kernel before), the activation tiles after it.  With several splits each
-// CTA writes its float partial tile to a workspace and the one that arrives last
-// (a counter per tile) adds them in split order; the number of splits depends on N
-// and K only, so a token's result does not depend on the batch it is in.
+// on the kernel before), the activation tiles after it.  With several splits the
+// CTAs of a tile form clusters of up to eight: each leaves its float partial tile
+// in its shared memory, and CTA r of a cluster takes the tokens r, r + size, ...,
+// adds their sums in split order through distributed shared memory and does their
+// epilogue.  More than eight splits: clusters of four, whose sums meet in a
+// workspace where the last one to arrive (a counter per tile and place in the
+// cluster) adds them in order.  The number of splits depends on N, K and the token
+// tile only, so a token's result does not depend on the batch it is in.  (One CTA
+// that read every split's partial tile from the workspace took several round trips
+// for itself: 64 tokens, eight splits, 262 KB.)
 // Epilogue: bias, or the SwiGLU of gate and up rows interleaved in groups of 8
 // (up * gate / (1 + exp(-gate)), src/ops/swiglu/op.cpp:17-23).
 //
 // K a multiple of 8; waits bounded as in the other tcgen05 kernel.
 #define LI_PDL_KIND 2
+#include "gemv_epilogue.cuh"
 #include "row_scale.cuh"
 #include "tcgen05.cuh"
 
@@ -26,7 +33,6 @@ namespace {
 using namespace tc;
 
 constexpr int BR = 128;                  // weight rows per CTA
-constexpr int kStages = 6;
 constexpr int kThreads = 192;
 constexpr int kTargetCtas = 148;
 constexpr size_t kWorkspaceFloats = 4u << 20;
@@ -34,6 +40,9 @@ constexpr int kMaxTiles = 1 << 16;
 
 template <int BT>
 struct __align__(1024) Smem {
+    // as many stages as two CTAs a multiprocessor leave room for: the next tile, or the next kernel's first one, streams in
+    // while the other's epilogue runs (64 tokens with six stages had room for one: N 37888, K 3584 61 -> 49 us)
+    static constexpr int kStages = BT <= 16 ? 6 : BT <= 32 ? 5 : 4;
     unsigned char w[kStages][BR * BK * 2];
     unsigned char x[kStages][BT * BK * 2];
     unsigned long long full[kStages];
@@ -82,14 +91,31 @@ __device__ __forceinline__ void tmem_ld<64>(unsigned taddr, float (&v)[64]) {
     }
 }
 
-enum { kEpiNone = 0, kEpiSwiglu = 1, kEpiAddScaled = 2, kEpiGluClamped = 3, kEpiGeglu = 4 };     // (the last two: SwiGLU's layout, another activation)
+// All threads of a cluster's CTAs, each warp by itself.
+__device__ __forceinline__ void cluster_arrive_wait() {
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ unsigned peer_address(unsigned addr, unsigned rank) {
+    unsigned r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ float peer_load(unsigned addr) {
+    float v;
+    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
+    return v;
+}
 
-template <int BT, typename Tout, int kEpi>
+enum { kEpiNone = 0, kEpiSwiglu = 1, kEpiAddScaled = 2, kEpiGluClamped = 3, kEpiGeglu = 4, kEpiRope = 5 };     // (3 and 4: SwiGLU's layout, another activation)
+
+// kSplit: k is split over the CTAs of clusters of `csize` (the grid's y: splits, a cluster's consecutive).
+template <int BT, typename Tout, int kEpi, bool kSplit>
 __global__ void __launch_bounds__(kThreads)
 gemv_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
                     const float* __restrict__ bias, Tout* __restrict__ out, float* __restrict__ partial,
-                    unsigned* __restrict__ counters, int M, int N, int K, int ksplit, int* __restrict__ error_flag, const RowScale rs,
-                    const AddScaled add) {
+                    unsigned* __restrict__ counters, int M, int N, int K, int ksplit, int csize, int* __restrict__ error_flag, const RowScale rs,
+                    const AddScaled add, const RopeArgs rope) {
     constexpr int kSwiglu = kEpi == kEpiSwiglu ? LI_EPILOGUE_SWIGLU : kEpi == kEpiGluClamped ? LI_EPILOGUE_GLU_CLAMPED : kEpi == kEpiGeglu ? LI_EPILOGUE_GEGLU : 0;
     constexpr bool kAdd = kEpi == kEpiAddScaled;
     extern __shared__ unsigned char smem_raw[];
@@ -102,6 +128,8 @@ gemv_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
     const int nkb = kb1 - kb0;
     constexpr unsigned kStageBytes = BR * BK * 2 + BT * BK * 2;
     constexpr unsigned kCols = BT < 32 ? 32 : BT;
+    constexpr int kStages = Smem<BT>::kStages;
+    constexpr int kMine = kSplit ? BT / 2 : BT;            // tokens a CTA finishes at most (a cluster has at least two)
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < kStages; ++s) {
@@ -181,102 +209,167 @@ gemv_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
             row_scales_of_warp<8>(rs, M, warp - 2, 4, lane, sm.factor);
             asm volatile("bar.sync 1, 128;" ::: "memory");
         }
-        float xold[kAdd ? BT : 1];
+        // the tokens this CTA finishes: all of them, or every csize-th of a cluster's
+        const int rank = kSplit ? split % csize : 0, step = kSplit ? csize : 1;
+        float xold[kAdd ? kMine : 1];
         if constexpr (kAdd) {
 #pragma unroll
-            for (int j = 0; j < BT; ++j) xold[j] = (j < M && row < N) ? __ldcg(add.x32 + (size_t)j * N + row) : 0.0f;
+            for (int i = 0; i < kMine; ++i) {
+                const int j = rank + i * step;
+                xold[i] = (j < M && row < N) ? __ldcg(add.x32 + (size_t)j * N + row) : 0.0f;
+            }
         }
         const bool ok = mbar_wait(&sm.accum, 0);
-        if (!ok) {
-            if (lane == 0) atomicExch(error_flag, 33);
-        } else {
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            float v[BT];
-            tmem_ld<BT>(tmem_acc + ((unsigned)(quarter * 32) << 16), v);
-            bool write = true;
-            if (ksplit > 1) {
-                const size_t tiles = gridDim.x;
-                float* mine = partial + (((size_t)split * tiles + tile) * BT) * BR + r_in_tile;
+        if (!ok && lane == 0) atomicExch(error_flag, 33);
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        float v[BT];
+        tmem_ld<BT>(tmem_acc + ((unsigned)(quarter * 32) << 16), v);
+        bool write = ok;
+        if constexpr (kSplit) {
+            // (every load into the stages has been multiplied: their room holds the partial tile [token][row] now)
+            float* mine = reinterpret_cast<float*>(sm.w[0]) + r_in_tile;
 #pragma unroll
-                for (int j = 0; j < BT; ++j)
-                    if (j < M) mine[(size_t)j * BR] = v[j];
+            for (int j = 0; j < BT; ++j)
+                if (j < M) mine[j * BR] = v[j];
+            cluster_arrive_wait();
+            float t[kMine];
+#pragma unroll
+            for (int i = 0; i < kMine; ++i) t[i] = 0.0f;
+            for (int r = 0; r < csize; ++r) {
+                const unsigned src = peer_address(smem_u32(mine), (unsigned)r);
+#pragma unroll
+                for (int i = 0; i < kMine; ++i) {
+                    const int j = rank + i * step;
+                    if (j < M) t[i] += peer_load(src + (unsigned)j * (BR * 4));
+                }
+            }
+#pragma unroll
+            for (int i = 0; i < kMine; ++i) v[i] = t[i];
+            const int groups = ksplit / csize;
+            if (groups > 1) {
+                const int group = split / csize;
+                const size_t tiles = gridDim.x;
+                float* to = partial + (((size_t)group * tiles + tile) * BT) * BR + r_in_tile;
+#pragma unroll
+                for (int i = 0; i < kMine; ++i)
+                    if (rank + i * step < M) to[(size_t)(rank + i * step) * BR] = v[i];
                 __threadfence();
                 asm volatile("bar.sync 1, 128;" ::: "memory");
                 if (warp == 2 && lane == 0) {
-                    const unsigned prev = atomicAdd(&counters[tile], 1u);
-                    sm.is_last = (prev == (unsigned)(ksplit - 1));
+                    const unsigned prev = atomicAdd(&counters[tile * csize + rank], 1u);
+                    sm.is_last = (prev == (unsigned)(groups - 1));
                 }
                 asm volatile("bar.sync 1, 128;" ::: "memory");
-                write = sm.is_last != 0;
-                if (write) {
+                write = write && sm.is_last != 0;
+                if (sm.is_last != 0) {
                     __threadfence();
 #pragma unroll
-                    for (int j = 0; j < BT; ++j) v[j] = 0.0f;
-                    // several splits' loads in flight at once (64 values a thread), added in split order
-                    constexpr int SU = 64 / BT;
-                    for (int s0 = 0; s0 < ksplit; s0 += SU) {
-                        float p[SU][BT];
+                    for (int i = 0; i < kMine; ++i) v[i] = 0.0f;
+                    for (int g = 0; g < groups; ++g) {
+                        const float* src = partial + (((size_t)g * tiles + tile) * BT) * BR + r_in_tile;
 #pragma unroll
-                        for (int u = 0; u < SU; ++u) {
-                            const float* src = partial + (((size_t)(s0 + u) * tiles + tile) * BT) * BR + r_in_tile;
-#pragma unroll
-                            for (int j = 0; j < BT; ++j) p[u][j] = (s0 + u < ksplit && j < M) ? __ldcg(src + (size_t)j * BR) : 0.0f;
-                        }
-#pragma unroll
-                        for (int u = 0; u < SU; ++u)
-#pragma unroll
-                            for (int j = 0; j < BT; ++j) v[j] += p[u][j];
+                        for (int i = 0; i < kMine; ++i)
+                            if (rank + i * step < M) v[i] += __ldcg(src + (size_t)(rank + i * step) * BR);
                     }
                     asm volatile("bar.sync 1, 128;" ::: "memory");
-                    if (warp == 2 && lane == 0) counters[tile] = 0;          // ready for the next launch on this stream
+                    if (warp == 2 && lane == 0) counters[tile * csize + rank] = 0;          // ready for the next launch on this stream
                 }
             }
-            if (write && rs.ssq) {
+        }
+        if (write && rs.ssq) {
 #pragma unroll
-                for (int j = 0; j < BT; ++j)
-                    if (j < M) v[j] *= sm.factor[j];
-            }
-            if (write) {
-                if constexpr (kAdd) {
-                    // into the residual stream, and on to the next product as bfloat16(norm_weight * x) with the sums of x^2
-                    const float b = (bias && row < N) ? bias[row] : 0.0f;
-                    const float nw = row < N ? add.norm_weight[row] : 0.0f;
+            for (int i = 0; i < kMine; ++i)
+                if (rank + i * step < M) v[i] *= sm.factor[rank + i * step];
+        }
+        if (write) {
+            if constexpr (kAdd) {
+                // into the residual stream, and on to the next product as bfloat16(norm_weight * x) with the sums of x^2
+                const float b = (bias && row < N) ? bias[row] : 0.0f;
+                const float nw = row < N ? add.norm_weight[row] : 0.0f;
 #pragma unroll
-                    for (int j = 0; j < BT; ++j) {
-                        if (j < M) {                                       // uniform
-                            const float x = row < N ? xold[j] + (v[j] + b) : 0.0f;
-                            if (row < N) {
-                                __stcg(add.x32 + (size_t)j * N + row, x);
-                                add.hprime[(size_t)j * N + row] = __float2bfloat16_rn(nw * x);
-                            }
-                            const float sq = warp_sum(x * x);
-                            if (lane == 0) sm.squares[quarter][j] = sq;
+                for (int i = 0; i < kMine; ++i) {
+                    const int j = rank + i * step;
+                    if (j < M) {                                           // uniform
+                        const float x = row < N ? xold[i] + (v[i] + b) : 0.0f;
+                        if (row < N) {
+                            __stcg(add.x32 + (size_t)j * N + row, x);
+                            add.hprime[(size_t)j * N + row] = __float2bfloat16_rn(nw * x);
                         }
+                        const float sq = warp_sum(x * x);
+                        if (lane == 0) sm.squares[quarter][j] = sq;
                     }
-                    asm volatile("bar.sync 1, 128;" ::: "memory");
-                    const int tid = (int)threadIdx.x - 64;
-                    if (tid < M)
-                        add.ssq_out[(size_t)tid * gridDim.x + tile] = ((sm.squares[0][tid] + sm.squares[1][tid]) + sm.squares[2][tid]) + sm.squares[3][tid];
-                } else if constexpr (kSwiglu == 0) {
-                    const float b = (bias && row < N) ? bias[row] : 0.0f;
+                }
+                asm volatile("bar.sync 1, 128;" ::: "memory");
+                const int j = rank + ((int)threadIdx.x - 64) * step;
+                if (j < M) add.ssq_out[(size_t)j * gridDim.x + tile] = ((sm.squares[0][j] + sm.squares[1][j]) + sm.squares[2][j]) + sm.squares[3][j];
+            } else if constexpr (kEpi == kEpiRope) {
+                // the tile is one head: rotation, then q into its row, k and v (transposed) into the paged cache (rope.cu)
+                const int head = tile, d = r_in_tile;
+                const float b = bias ? bias[row] : 0.0f;
+                const bool rotate = rope.denom != nullptr && head < rope.nh + rope.nkv;
+                float* both = reinterpret_cast<float*>(sm.x[0]) + d;       // the other half of a pair is 64 rows, two warps, away
 #pragma unroll
-                    for (int j = 0; j < BT; ++j)
-                        if (j < M && row < N) out[(size_t)j * N + row] = from_float<Tout>(v[j] + b);
-                } else {
-                    // rows come as 8 gate, 8 up, ...: lanes 0-7 and 16-23 hold gates, the lane 8 further on the matching up
-                    const int half_n = N >> 1;
-                    const int col = (row >> 4) * 8 + (row & 7);
+                for (int i = 0; i < kMine; ++i) {
+                    v[i] += b;
+                    // q and k are rounded to bfloat16 by the projection before they are rotated, as in the unfused path
+                    both[i * BR] = rotate ? __bfloat162float(__float2bfloat16_rn(v[i])) : v[i];
+                }
+                asm volatile("bar.sync 1, 128;" ::: "memory");
+                const float den = rotate ? rope.denom[d & 63] : 1.0f;
+                const size_t ld = (size_t)(rope.nh + 2 * rope.nkv) * BR;
+#pragma unroll 1
+                for (int i = 0; i < kMine; ++i) {
+                    const int j = rank + i * step;
+                    if (j >= M) break;
+                    float y = both[i * BR];
+                    if (rotate) {
+                        float sn, cs;
+                        sincosf((float)rope.positions[j] / den, &sn, &cs);
+                        const float other = d < 64 ? both[i * BR + 64] : both[i * BR - 64];
+                        y = d < 64 ? y * cs - other * sn : y * cs + other * sn;
+                    }
+                    const bf16 r = __float2bfloat16_rn(y);
+                    if (head >= rope.nh + 2 * rope.nkv) {
+                        rope.extra_out[((size_t)j * rope.extra + (head - rope.nh - 2 * rope.nkv)) * BR + d] = r;
+                    } else if (head < rope.nh) {
+                        reinterpret_cast<bf16*>(out)[j * ld + (size_t)head * BR + d] = r;
+                    } else if (rope.write) {
+                        const int slot = rope.slot_mapping[j];
+                        const int page = slot / rope.page_size, off = slot - page * rope.page_size;
+                        if (slot < 0 || page >= rope.num_pages) continue;      // validated on the host; never write outside the cache
+                        if (head < rope.nh + rope.nkv)
+                            rope.kcache[(((size_t)page * rope.nkv + (head - rope.nh)) * rope.page_size + off) * BR + d] = r;
+                        else
+                            rope.vcache[((size_t)page * rope.nkv + (head - rope.nh - rope.nkv)) * BR * rope.page_size + (size_t)d * rope.page_size + off] = r;
+                    }
+                }
+            } else if constexpr (kSwiglu == 0) {
+                const float b = (bias && row < N) ? bias[row] : 0.0f;
 #pragma unroll
-                    for (int j = 0; j < BT; ++j) {
-                        const float up = __shfl_down_sync(0xffffffffu, v[j], 8);
-                        if (j < M && (lane & 8) == 0 && row + 8 < N) {
-                            const float gate = v[j];
-                            out[(size_t)j * half_n + col] = from_float<Tout>(glu_of<Tout, kSwiglu>(gate, up, bias));
-                        }
+                for (int i = 0; i < kMine; ++i) {
+                    const int j = rank + i * step;
+                    if (j < M && row < N) out[(size_t)j * N + row] = from_float<Tout>(v[i] + b);
+                }
+            } else {
+                // rows come as 8 gate, 8 up, ...: lanes 0-7 and 16-23 hold gates, the lane 8 further on the matching up
+                const int half_n = N >> 1;
+                const int col = (row >> 4) * 8 + (row & 7);
+#pragma unroll
+                for (int i = 0; i < kMine; ++i) {
+                    const int j = rank + i * step;
+                    const float up = __shfl_down_sync(0xffffffffu, v[i], 8);
+                    if (j < M && (lane & 8) == 0 && row + 8 < N) {
+                        const float gate = v[i];
+                        out[(size_t)j * half_n + col] = from_float<Tout>(glu_of<Tout, kSwiglu>(gate, up, bias));
                     }
                 }
             }
         }
+    }
+    if constexpr (kSplit) {
+        __syncwarp();
+        if (warp < 2) cluster_arrive_wait();               // (the epilogue warps met there for the partial tiles)
+        cluster_arrive_wait();                             // nobody leaves while its partial tile may be read
     }
     __syncwarp();
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -316,17 +409,19 @@ int choose_ksplit(int N, int K, int bt) {
     } else {
         ks = kTargetCtas / tiles;
         if (ks < 1) ks = 1;
-        if (bt == 64 && ks > 8) ks = 8;                               // 32 KB of partial sums a split: the merge by one CTA grows with them (measured)
         const int by_work = nkb / 2 > 0 ? nkb / 2 : 1;                // at least two k-blocks a CTA
         if (ks > by_work) ks = by_work;
     }
     while (ks > 1 && (size_t)ks * tiles * 64 * BR > kWorkspaceFloats) --ks;      // the partial sums fit the workspace: sized for 64 tokens whatever M is
+    // many tokens: one cluster a tile (64 tokens, N 1536, K 8960: 21.8 us with three clusters of four, whose sums meet in the workspace)
+    if (bt == 64 && ks > 8) ks = 8;
+    if (ks > 8) ks -= ks % 4;                                         // clusters of four
     return ks;
 }
 
 template <int BT, typename Tout, int kEpi>
 int launch(const void* a, const void* w, const float* bias, void* out, int M, int N, int K, cudaStream_t stream, const RowScale& rs,
-           const AddScaled& add) {
+           const AddScaled& add, const RopeArgs& rope) {
     EncodeTiledFn encode = nullptr;
     int *err_host = nullptr, *err_dev = nullptr;
     if (int rc = setup(&encode, &err_host, &err_dev)) return rc;
@@ -345,21 +440,29 @@ int launch(const void* a, const void* w, const float* bias, void* out, int M, in
     const size_t smem = sizeof(Smem<BT>) + 1024;
     static bool raised = false;
     if (!raised) {
-        cudaError_t e = cudaFuncSetAttribute(gemv_tcgen05_kernel<BT, Tout, kEpi>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaError_t e = cudaFuncSetAttribute(gemv_tcgen05_kernel<BT, Tout, kEpi, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(gemv_tcgen05_kernel<BT, Tout, kEpi, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return li_fail("linear (tcgen05 gemv): cannot raise shared memory to %zu: %s", smem, cudaGetErrorString(e));
         raised = true;
     }
-    li_launch_pdl(gemv_tcgen05_kernel<BT, Tout, kEpi>, dim3(tiles, ksplit), dim3(kThreads), smem, stream, map_w, map_x, bias, (Tout*)out,
-                  ws->partial, ws->counters, M, N, K, ksplit, err_dev, rs, add);
+    if (ksplit == 1) {
+        li_launch_pdl(gemv_tcgen05_kernel<BT, Tout, kEpi, false>, dim3(tiles, 1), dim3(kThreads), smem, stream, map_w, map_x, bias, (Tout*)out,
+                      ws->partial, ws->counters, M, N, K, 1, 1, err_dev, rs, add, rope);
+    } else {
+        const int csize = ksplit <= 8 ? ksplit : 4;
+        LI_REQUIRE(tiles * csize <= kMaxTiles, "linear (tcgen05 gemv): N=%d has too many tiles for a split of k", N);
+        li_launch_pdl(gemv_tcgen05_kernel<BT, Tout, kEpi, true>, dim3(tiles, ksplit), dim3(kThreads), smem, stream, dim3(1, csize, 1), map_w, map_x, bias,
+                      (Tout*)out, ws->partial, ws->counters, M, N, K, ksplit, csize, err_dev, rs, add, rope);
+    }
     return li_check_launch("linear (tcgen05 gemv)");
 }
 
 template <typename Tout, int kEpi>
 int launch_bt(const void* a, const void* w, const float* bias, void* out, int M, int N, int K, cudaStream_t stream, const RowScale& rs,
-              const AddScaled& add = AddScaled{}) {
-    if (M <= 16) return launch<16, Tout, kEpi>(a, w, bias, out, M, N, K, stream, rs, add);
-    if (M <= 32) return launch<32, Tout, kEpi>(a, w, bias, out, M, N, K, stream, rs, add);
-    return launch<64, Tout, kEpi>(a, w, bias, out, M, N, K, stream, rs, add);
+              const AddScaled& add = AddScaled{}, const RopeArgs& rope = RopeArgs{}) {
+    if (M <= 16) return launch<16, Tout, kEpi>(a, w, bias, out, M, N, K, stream, rs, add, rope);
+    if (M <= 32) return launch<32, Tout, kEpi>(a, w, bias, out, M, N, K, stream, rs, add, rope);
+    return launch<64, Tout, kEpi>(a, w, bias, out, M, N, K, stream, rs, add, rope);
 }
 
 }  // namespace
@@ -384,6 +487,17 @@ int li_linear_gemv_tcgen05(const void* a, const void* w, const float* bias, void
     if (dtype_out == LI_BF16) return launch_bt<bf16, kEpiNone>(a, w, bias, out, M, N, K, stream, rs);
     if (dtype_out == LI_F32) return launch_bt<float, kEpiNone>(a, w, bias, out, M, N, K, stream, rs);
     return li_fail("linear (tcgen05 gemv): unsupported output dtype %d", dtype_out);
+}
+
+// The fused q|k|v projection with rotary encoding and cache write in its epilogue: heads of 128 (rotated whole or not at all),
+// a tile a head.  Against the register-fed kernel's (li_linear_gemv_rope) where its rows are long: linear.cu says from where.
+bool li_gemv_tcgen05_rope_accepts(const void* a, const void* w, int M, int N, int K, int nh, int nkv, int dh, int rotary_dim) {
+    return li_gemv_tcgen05_accepts(a, w, M, N, K) && dh == BR && (rotary_dim == dh || rotary_dim == 0) && N == (nh + 2 * nkv) * dh;
+}
+
+int li_linear_gemv_tcgen05_rope(const void* a, const void* w, const float* bias, void* out, int M, int N, int K, const RopeArgs& rope, const RowScale& rs,
+                                cudaStream_t stream) {
+    return launch_bt<bf16, kEpiRope>(a, w, bias, out, M, N + rope.extra * BR, K, stream, rs, AddScaled{}, rope);
 }
 
 // x32 += a w^T (+ bias), hprime = bfloat16(norm_weight * x32), ssq_out[token, tile] = sums of squares (row_scale.cuh).
