@@ -10,7 +10,9 @@
 // one CTA per (sequence, kv head) whose warps walk every 8th block of 32 keys;
 // nothing to merge across CTAs.  Either way a warp works for all query heads of
 // one key/value head at once (they share every K and V byte read; heads are the
-// 16 rows of a tensor-core tile).  Per block a warp computes S = Q K^T and
+// 16 rows of a tensor-core tile; up to 8 of them are the 8 columns instead,
+// attention_mma.cuh: 64 sequences of 12 heads on 2 at 2,176 keys 31.4 -> 27.7 us
+// with twelve warps).  Per block a warp computes S = Q K^T and
 // O += P V with mma.sync m16n8k16 (bfloat16 in, float accumulate), softmax
 // online in float as in LitInfer's kernel (src/ops/paged_attention/op.cpp:194-234).
 // All operands go from global memory straight into fragment registers with
@@ -50,7 +52,7 @@ Workspace g_ws[16];
 using namespace attn;
 using namespace attn_decode;
 
-template <int DH, int KB, bool kCut, bool kMod>
+template <int DH, int KB, bool kCut, bool kMod, bool kColumns>
 __global__ void __launch_bounds__(kWarps * 32, 1)
 decode_attention_kernel(const bf16* __restrict__ qkv, const bf16* __restrict__ kcache, const bf16* __restrict__ vcache,
                         const int* __restrict__ block_table, int max_blocks, const int* __restrict__ ctx_lens,
@@ -60,7 +62,7 @@ decode_attention_kernel(const bf16* __restrict__ qkv, const bf16* __restrict__ k
     extern __shared__ float sm[];
     __shared__ int is_last;
     pdl_launch_dependents();
-    decode_attention_unit<DH, KB, kCut, kMod>((int)blockIdx.x, (int)blockIdx.y, (int)blockIdx.z, (int)threadIdx.x, qkv, kcache, vcache, block_table, max_blocks,
+    decode_attention_unit<DH, KB, kCut, kMod, kColumns>((int)blockIdx.x, (int)blockIdx.y, (int)blockIdx.z, (int)threadIdx.x, qkv, kcache, vcache, block_table, max_blocks,
                                   ctx_lens, old_lens, q_start, part, counters, out, nh, nkv, page_size, num_pages, scale, window, nsplit, sm,
                                   &is_last, [] { __syncthreads(); }, [] { pdl_wait(); }, want, mod);
 }
@@ -69,7 +71,7 @@ decode_attention_kernel(const bf16* __restrict__ qkv, const bf16* __restrict__ k
 // context over CTAs would only add partial results to write, merge and wait for.  Each of the CTA's warps
 // walks every WARPS-th block of 16 keys with a running softmax; the warps are merged through shared memory in
 // warp order at the end.  The assignment of blocks to warps depends on the sequence alone.
-template <int DH, int WARPS, int KB, bool kMod>
+template <int DH, int WARPS, int KB, bool kMod, bool kColumns>
 __global__ void __launch_bounds__(WARPS * 32, 1)
 decode_attention_whole_kernel(const bf16* __restrict__ qkv, const bf16* __restrict__ kcache, const bf16* __restrict__ vcache,
                               const int* __restrict__ block_table, int max_blocks, const int* __restrict__ ctx_lens,
@@ -87,13 +89,31 @@ decode_attention_whole_kernel(const bf16* __restrict__ qkv, const bf16* __restri
     const int G = nh / nkv;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int g = lane >> 2, t = lane & 3;
+    const int* bt = block_table + (size_t)s * max_blocks;
+    const int b_first = lo / KB, b_last = p / KB;
+    float* sm_m = sm;
+    float* sm_l = sm + WARPS * 16;
+    float* sm_o = sm + 2 * WARPS * 16;
+    if constexpr (kColumns) {
+        static_assert(KB == 32 && !kMod, "the swapped form takes blocks of 32 keys and no options");
+        uint4 qb[DH / 32];
+        load_q32_columns<DH>(qb, g < G ? qkv + (size_t)tok * (nh + 2 * nkv) * DH + (size_t)(kvh * G + g) * DH : nullptr, t);
+        ColState<DH> st;
+        st.init();
+#pragma unroll 1
+        for (int b = b_first + warp; b <= b_last; b += WARPS) {
+            KFrag32<DH> kf;
+            VFrag32<DH> vf;
+            block_load32<DH>(kf, vf, kcache, vcache, bt, b * KB, p, kvh, nkv, page_size, num_pages, g, t);
+            compute32_columns<DH>(st, qb, kf, vf, b * KB, lo, p, scale, g);
+        }
+        put_state<DH>(st, sm_m, sm_l, sm_o, warp, G, g, t);
+    } else {
     unsigned qa[DH / 16][4];
     load_query_heads<DH, KB, kMod>(qa, qkv, tok, kvh, nh, nkv, g, t, mod);
     RowState<DH> st;
     st.init();
     const int lo2[2] = {lo, lo}, hi2[2] = {p, p};
-    const int* bt = block_table + (size_t)s * max_blocks;
-    const int b_first = lo / KB, b_last = p / KB;
     RowMod rm;
     if constexpr (kMod) {
         rm.softcap = mod.softcap;
@@ -114,26 +134,7 @@ decode_attention_whole_kernel(const bf16* __restrict__ qkv, const bf16* __restri
                 block_step<DH, KB, kMod>(st, qa, kcache, vcache, bt, key0, kvh, nkv, page_size, num_pages, lok, hik, scale, g, t, rm);
         }
     }
-    const float m0 = st.m[0], m1 = st.m[1];
-    const float l0 = quad_sum(st.l[0]), l1 = quad_sum(st.l[1]);
-    float* sm_m = sm;
-    float* sm_l = sm + WARPS * 16;
-    float* sm_o = sm + 2 * WARPS * 16;
-    if (t == 0) {
-        sm_m[warp * 16 + g] = m0; sm_m[warp * 16 + g + 8] = m1;
-        sm_l[warp * 16 + g] = l0; sm_l[warp * 16 + g + 8] = l1;
-    }
-#pragma unroll
-    for (int j = 0; j < DH / 8; ++j) {
-        const int col = j * 8 + 2 * t;
-        if (g < G) {
-            sm_o[((size_t)warp * G + g) * DH + col] = st.o[j][0];
-            sm_o[((size_t)warp * G + g) * DH + col + 1] = st.o[j][1];
-        }
-        if (g + 8 < G) {
-            sm_o[((size_t)warp * G + g + 8) * DH + col] = st.o[j][2];
-            sm_o[((size_t)warp * G + g + 8) * DH + col + 1] = st.o[j][3];
-        }
+    put_state<DH>(st, sm_m, sm_l, sm_o, warp, G, g, t);
     }
     __syncthreads();
     for (int e = threadIdx.x; e < G * DH; e += WARPS * 32) {
@@ -191,7 +192,7 @@ int ensure_workspace(size_t floats, float** buf, unsigned** counters) {
     return 0;
 }
 
-template <int DH, bool kMod>
+template <int DH, bool kMod, bool kColumns>
 int launch(const void* qkv, void* out, const void* kcache, const void* vcache, const int* block_table, int max_blocks,
            const int* ctx_lens, const int* old_lens, const int* q_start, int S, int nh, int nkv, int page_size, int num_pages, float scale,
            int window, int max_ctx_len, int expected, ScoreMod mod, cudaStream_t stream) {
@@ -215,17 +216,21 @@ int launch(const void* qkv, void* out, const void* kcache, const void* vcache, c
     const int want = (int)(pairs >= sms ? 1 : sms / pairs);                              // units per pair that fill the GPU once
     if (want == 1 && blocks > 1) {
         // one CTA per (sequence, kv head) fills the GPU: no split of the context
-        constexpr int W = 8, KB = KBS;
+        // (the swapped form leaves registers for twelve warps: half as many loads in flight again)
+        constexpr int W = kColumns ? 12 : 8, KB = KBS;
         const size_t wsmem = (2 * W * 16 + (size_t)W * G * DH) * sizeof(float);
         if (wsmem <= 200 * 1024) {
             static bool raised = false;
             if (!raised && wsmem > 48 * 1024) {
-                cudaError_t e = cudaFuncSetAttribute(decode_attention_whole_kernel<DH, W, KB, kMod>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+                cudaError_t e = cudaFuncSetAttribute(decode_attention_whole_kernel<DH, W, KB, kMod, kColumns>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
                 if (e != cudaSuccess) return li_fail("attention (decode): cannot raise shared memory: %s", cudaGetErrorString(e));
                 raised = true;
             }
-            li_launch_pdl(decode_attention_whole_kernel<DH, W, KB, kMod>, dim3(nkv, S), dim3(W * 32), wsmem, stream, (const bf16*)qkv, (const bf16*)kcache,
-                          (const bf16*)vcache, block_table, max_blocks, ctx_lens, q_start, (bf16*)out, nh, nkv, page_size, num_pages, scale, window, mod);
+            // Launched plainly: with CTAs that were there before the q|k|v product had finished a step of 64 sequences took longer
+            // (1.5B shape 2.78 against 2.53 ms, 61 sequences of the 7B shape 5.16 against 4.88 ms).
+            decode_attention_whole_kernel<DH, W, KB, kMod, kColumns><<<dim3(nkv, S), dim3(W * 32), wsmem, stream>>>(
+                (const bf16*)qkv, (const bf16*)kcache, (const bf16*)vcache, block_table, max_blocks, ctx_lens, q_start, (bf16*)out, nh, nkv, page_size,
+                num_pages, scale, window, mod);
             return li_check_launch("attention (decode, whole context)");
         }
     }
@@ -246,8 +251,8 @@ int launch(const void* qkv, void* out, const void* kcache, const void* vcache, c
     const size_t smem = smem_floats * sizeof(float);
     static bool attr_set = false;
     if (!attr_set && smem > 48 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(decode_attention_kernel<DH, KBS, false, kMod>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(decode_attention_kernel<DH, KBS, true, kMod>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+        cudaError_t e = cudaFuncSetAttribute(decode_attention_kernel<DH, KBS, false, kMod, kColumns>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(decode_attention_kernel<DH, KBS, true, kMod, kColumns>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
         if (e != cudaSuccess) return li_fail("attention (decode): cannot raise shared memory: %s", cudaGetErrorString(e));
         attr_set = true;
     }
@@ -255,11 +260,11 @@ int launch(const void* qkv, void* out, const void* kcache, const void* vcache, c
     LI_REQUIRE(S <= 65535 && nkv <= 65535, "attention (decode): batch %d or kv heads %d too large for one launch", S, nkv);
     dim3 grid(nsplit, nkv, S);
     if (cut)
-        li_launch_pdl(decode_attention_kernel<DH, KBS, true, kMod>, dim3(grid), dim3(kWarps * 32), smem, stream, (const bf16*)qkv, (const bf16*)kcache,
+        li_launch_pdl(decode_attention_kernel<DH, KBS, true, kMod, kColumns>, dim3(grid), dim3(kWarps * 32), smem, stream, (const bf16*)qkv, (const bf16*)kcache,
                       (const bf16*)vcache, block_table, max_blocks, ctx_lens, old_lens, q_start, part, counters, (bf16*)out, nh, nkv, page_size,
                       num_pages, scale, window, nsplit, want, mod);
     else
-        li_launch_pdl(decode_attention_kernel<DH, KBS, false, kMod>, dim3(grid), dim3(kWarps * 32), smem, stream, (const bf16*)qkv, (const bf16*)kcache,
+        li_launch_pdl(decode_attention_kernel<DH, KBS, false, kMod, kColumns>, dim3(grid), dim3(kWarps * 32), smem, stream, (const bf16*)qkv, (const bf16*)kcache,
                       (const bf16*)vcache, block_table, max_blocks, ctx_lens, old_lens, q_start, part, counters, (bf16*)out, nh, nkv, page_size,
                       num_pages, scale, window, nsplit, 0, mod);
     return li_check_launch("attention (decode)");
@@ -276,11 +281,21 @@ int li_attention_decode(const void* qkv, void* out, const void* kcache, const vo
                         const int* ctx_lens, const int* old_lens, const int* q_start, int S, int nh, int nkv, int dh, int page_size, int num_pages,
                         float scale, int window, int max_ctx_len, int expected, const AttentionOptions& opt, cudaStream_t stream) {
     const ScoreMod mod(opt, window);
+    // up to 8 heads a key/value head and none of the options: the heads as columns of the score tiles, half the products and
+    // exponentials (heads of 64 and 128; others take the rows)
+    if (!mod.any() && nh / nkv <= 8 && (dh == 128 || dh == 64)) {
 #define LI_CASE(D)                                                                                                             \
     case D:                                                                                                                    \
-        return mod.any() ? launch<D, true>(qkv, out, kcache, vcache, block_table, max_blocks, ctx_lens, old_lens, q_start, S, nh, nkv, page_size, \
+        return launch<D, false, true>(qkv, out, kcache, vcache, block_table, max_blocks, ctx_lens, old_lens, q_start, S, nh, nkv, page_size, \
+                                      num_pages, scale, window, max_ctx_len, expected, mod, stream);
+        switch (dh) { LI_CASE(64) LI_CASE(128) }
+#undef LI_CASE
+    }
+#define LI_CASE(D)                                                                                                             \
+    case D:                                                                                                                    \
+        return mod.any() ? launch<D, true, false>(qkv, out, kcache, vcache, block_table, max_blocks, ctx_lens, old_lens, q_start, S, nh, nkv, page_size, \
                                            num_pages, scale, window, max_ctx_len, expected, mod, stream)                           \
-                         : launch<D, false>(qkv, out, kcache, vcache, block_table, max_blocks, ctx_lens, old_lens, q_start, S, nh, nkv, page_size, \
+                         : launch<D, false, false>(qkv, out, kcache, vcache, block_table, max_blocks, ctx_lens, old_lens, q_start, S, nh, nkv, page_size, \
                                             num_pages, scale, window, max_ctx_len, expected, mod, stream);
     switch (dh) {
         LI_CASE(16) LI_CASE(32) LI_CASE(48) LI_CASE(64) LI_CASE(80) LI_CASE(96) LI_CASE(112) LI_CASE(128) LI_CASE(256)

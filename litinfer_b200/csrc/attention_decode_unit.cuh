@@ -88,7 +88,47 @@ __device__ __forceinline__ void block_load32(KFrag32<DH>& kf, VFrag32<DH>& vf, c
     load_v32<DH>(vf, vcache + ((size_t)vpage * nkv + kvh) * DH * page_size + vk % page_size, page_size, g);
 }
 
-template <int DH, int KB, bool kCut = false, bool kMod = false, typename Sync, typename Wait>
+// A warp's running result into the shared scratch of the merge: sm_m[w][16] | sm_l[w][16] | sm_o[w][G][DH].
+template <int DH>
+__device__ __forceinline__ void put_state(const RowState<DH>& st, float* sm_m, float* sm_l, float* sm_o, int warp, int G, int g, int t) {
+    const float l0 = quad_sum(st.l[0]), l1 = quad_sum(st.l[1]);
+    if (t == 0) {
+        sm_m[warp * 16 + g] = st.m[0]; sm_m[warp * 16 + g + 8] = st.m[1];
+        sm_l[warp * 16 + g] = l0; sm_l[warp * 16 + g + 8] = l1;
+    }
+#pragma unroll
+    for (int j = 0; j < DH / 8; ++j) {
+        const int col = j * 8 + 2 * t;
+        if (g < G) {
+            sm_o[((size_t)warp * G + g) * DH + col] = st.o[j][0];
+            sm_o[((size_t)warp * G + g) * DH + col + 1] = st.o[j][1];
+        }
+        if (g + 8 < G) {
+            sm_o[((size_t)warp * G + g + 8) * DH + col] = st.o[j][2];
+            sm_o[((size_t)warp * G + g + 8) * DH + col + 1] = st.o[j][3];
+        }
+    }
+}
+
+template <int DH>
+__device__ __forceinline__ void put_state(const ColState<DH>& st, float* sm_m, float* sm_l, float* sm_o, int warp, int G, int g, int t) {
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        const int head = 2 * t + h;
+        const float l = column_sum(st.l[h]);
+        if (g == 0) sm_m[warp * 16 + head] = st.m[h], sm_l[warp * 16 + head] = l;
+        if (head < G) {
+#pragma unroll
+            for (int i = 0; i < DH / 16; ++i) {
+                sm_o[((size_t)warp * G + head) * DH + 16 * i + g] = st.o[i][h];
+                sm_o[((size_t)warp * G + head) * DH + 16 * i + g + 8] = st.o[i][2 + h];
+            }
+        }
+    }
+}
+
+// kColumns: at most 8 heads a key/value head, as the columns of the score tiles (attention_mma.cuh)
+template <int DH, int KB, bool kCut = false, bool kMod = false, bool kColumns = false, typename Sync, typename Wait>
 __device__ __forceinline__ void decode_attention_unit(int split, int kvh, int s, int tid, const bf16* __restrict__ qkv, const bf16* __restrict__ kcache,
                                                       const bf16* __restrict__ vcache, const int* __restrict__ block_table, int max_blocks,
                                                       const int* __restrict__ ctx_lens, const int* __restrict__ old_lens,
@@ -134,12 +174,37 @@ __device__ __forceinline__ void decode_attention_unit(int split, int kvh, int s,
         if (early) block_load32<DH>(kf_early, vf_early, kcache, vcache, bt, my_key0, k_end - 1, kvh, nkv, page_size, num_pages, g, t);
     }
     wait_for_queries();
+    const int lo2[2] = {lo, lo}, hi2[2] = {k_end - 1, k_end - 1};
+    float* sm_m = sm;
+    float* sm_l = sm + kWarps * 16;
+    float* sm_o = sm + 2 * kWarps * 16;
+    if constexpr (kColumns) {
+        static_assert(KB == 32 && !kMod, "the swapped form takes blocks of 32 keys and no options");
+        uint4 qb[DH / 32];
+        load_q32_columns<DH>(qb, g < G ? qkv + (size_t)tok * (nh + 2 * nkv) * DH + (size_t)(kvh * G + g) * DH : nullptr, t);
+        ColState<DH> st;
+        st.init();
+        if (my_block) {
+            if (!early) block_load32<DH>(kf_early, vf_early, kcache, vcache, bt, my_key0, k_end - 1, kvh, nkv, page_size, num_pages, g, t);
+            compute32_columns<DH>(st, qb, kf_early, vf_early, my_key0, lo, k_end - 1, scale, g);
+        }
+        if constexpr (kCut) {
+#pragma unroll 1
+            for (int rd = 1; rd < rounds; ++rd) {
+                const int key0 = k_begin + (rd * kWarps + warp) * KB;
+                if (key0 < k_end && key0 + KB > lo) {            // warp-uniform
+                    block_load32<DH>(kf_early, vf_early, kcache, vcache, bt, key0, k_end - 1, kvh, nkv, page_size, num_pages, g, t);
+                    compute32_columns<DH>(st, qb, kf_early, vf_early, key0, lo, k_end - 1, scale, g);
+                }
+            }
+        }
+        put_state<DH>(st, sm_m, sm_l, sm_o, warp, G, g, t);
+    } else {
     // query fragments: rows g and g + 8 are heads kvh * G + g (+ 8)
     unsigned qa[DH / 16][4];
     load_query_heads<DH, KB, kMod>(qa, qkv, tok, kvh, nh, nkv, g, t, mod);
     RowState<DH> st;
     st.init();
-    const int lo2[2] = {lo, lo}, hi2[2] = {k_end - 1, k_end - 1};
     attn::RowMod rm;
     if constexpr (kMod) {
         rm.softcap = mod.softcap;
@@ -173,31 +238,9 @@ __device__ __forceinline__ void decode_attention_unit(int split, int kvh, int s,
                 block_step<DH, KB, kMod>(st, qa, kcache, vcache, bt, key0, kvh, nkv, page_size, num_pages, lok, hik, scale, g, t, rm);
         }
     }
-    const float m0 = st.m[0], m1 = st.m[1];
-    const float l0 = quad_sum(st.l[0]), l1 = quad_sum(st.l[1]);
-    auto& o = st.o;
-    constexpr int NT = DH / 8;
-
-    // merge the warps in fixed order: sm_m[w][16] | sm_l[w][16] | sm_o[w][G][DH]
-    float* sm_m = sm;
-    float* sm_l = sm + kWarps * 16;
-    float* sm_o = sm + 2 * kWarps * 16;
-    if (t == 0) {
-        sm_m[warp * 16 + g] = m0; sm_m[warp * 16 + g + 8] = m1;
-        sm_l[warp * 16 + g] = l0; sm_l[warp * 16 + g + 8] = l1;
+    put_state<DH>(st, sm_m, sm_l, sm_o, warp, G, g, t);
     }
-#pragma unroll
-    for (int j = 0; j < NT; ++j) {
-        const int col = j * 8 + 2 * t;
-        if (g < G) {
-            sm_o[((size_t)warp * G + g) * DH + col] = o[j][0];
-            sm_o[((size_t)warp * G + g) * DH + col + 1] = o[j][1];
-        }
-        if (g + 8 < G) {
-            sm_o[((size_t)warp * G + g + 8) * DH + col] = o[j][2];
-            sm_o[((size_t)warp * G + g + 8) * DH + col + 1] = o[j][3];
-        }
-    }
+    // merge the warps in fixed order
     sync();
     const bool alone = k_begin <= lo && k_end == ctx;      // the only unit of its sequence and key/value head: nothing to merge
     // partial layout per (sequence, head, split): DH floats of O, then m, l

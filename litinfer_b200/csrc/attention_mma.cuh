@@ -348,4 +348,104 @@ __device__ __forceinline__ void compute32(RowState<DH>& st, const unsigned (&qa)
     }
 }
 
+// ---- the same step for at most 8 query heads, with the operands' roles swapped ----
+//
+// With the heads as the 16 rows of a tile half of every product and of every exponential is for rows that do not exist (a
+// group of 5 to 8 heads).  Here the keys are the 16 rows and the heads the 8 columns: S^T = K Q^T and O^T += V^T P^T take 16
+// products each of a block of 32 keys instead of 32.  The fragments of keys and values are loaded as above; a score tile's
+// rows g and g + 8 are the keys 8 (g >> 1) + 2 q + (g & 1) of the groups q = 2 mt and 2 mt + 1, so that a group's 8 x 8 scores,
+// transposed within the warp (movmatrix), are the operand of the second product for the keys 8 t + 2 q + {0, 1}.
+
+template <int DH>
+struct ColState {                            // heads 2 t and 2 t + 1; o[i]: elements 16 i + g (0, 1) and 16 i + g + 8 (2, 3) of each
+    float m[2], l[2];
+    float o[DH / 16][4];
+    __device__ __forceinline__ void init() {
+        m[0] = m[1] = -INFINITY;
+        l[0] = l[1] = 0.0f;
+#pragma unroll
+        for (int i = 0; i < DH / 16; ++i) o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.0f;
+    }
+};
+
+__device__ __forceinline__ unsigned transpose8x8(unsigned v) {
+    unsigned r;
+    asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(r) : "r"(v));
+    return r;
+}
+
+// over the eight lanes that share t
+__device__ __forceinline__ float column_max(float v) {
+    v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, 4));
+    v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, 8));
+    return fmaxf(v, __shfl_xor_sync(0xffffffffu, v, 16));
+}
+__device__ __forceinline__ float column_sum(float v) {
+    v += __shfl_xor_sync(0xffffffffu, v, 4);
+    v += __shfl_xor_sync(0xffffffffu, v, 8);
+    return v + __shfl_xor_sync(0xffffffffu, v, 16);
+}
+
+// qb: the row of this thread's head g (null: no such head)
+template <int DH>
+__device__ __forceinline__ void load_q32_columns(uint4 (&qb)[DH / 32], const bf16* row, int t) {
+#pragma unroll
+    for (int f = 0; f < DH / 32; ++f) qb[f] = row ? ld16(row + f * 32 + t * 8) : make_uint4(0, 0, 0, 0);
+}
+
+template <int DH>
+__device__ __forceinline__ void compute32_columns(ColState<DH>& st, const uint4 (&qb)[DH / 32], const KFrag32<DH>& kf, const VFrag32<DH>& vf, int key0, int lo,
+                                                  int hi, float scale, int g) {
+    static_assert(DH % 32 == 0, "whole pieces of 32 elements");
+    float sc[2][4];
+#pragma unroll
+    for (int mt = 0; mt < 2; ++mt) {
+        float odd[4] = {0.0f, 0.0f, 0.0f, 0.0f};                 // two chains a tile
+        sc[mt][0] = sc[mt][1] = sc[mt][2] = sc[mt][3] = 0.0f;
+#pragma unroll
+        for (int f = 0; f < DH / 32; ++f) {
+            const uint4 a = kf.k[2 * mt][f], b = kf.k[2 * mt + 1][f];
+            mma_bf16(sc[mt], a.x, b.x, a.y, b.y, qb[f].x, qb[f].y);
+            mma_bf16(odd, a.z, b.z, a.w, b.w, qb[f].z, qb[f].w);
+        }
+#pragma unroll
+        for (int e = 0; e < 4; ++e) sc[mt][e] += odd[e];
+    }
+    float alpha[2];
+    const int mine = key0 + 8 * (g >> 1) + (g & 1);
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        float mx = -INFINITY;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            float& v = sc[q >> 1][2 * (q & 1) + h];
+            const int key = mine + 2 * q;
+            v = (key >= lo && key <= hi) ? v * scale : -INFINITY;
+            mx = fmaxf(mx, v);
+        }
+        const float mn = fmaxf(st.m[h], column_max(mx));
+        const float ms = (mn == -INFINITY) ? 0.0f : mn;
+        alpha[h] = expf(st.m[h] - ms);
+        float sum = 0.0f;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            float& v = sc[q >> 1][2 * (q & 1) + h];
+            v = expf(v - ms);
+            sum += v;
+        }
+        st.l[h] = st.l[h] * alpha[h] + sum;
+        st.m[h] = mn;
+    }
+    unsigned pb[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) pb[q] = transpose8x8(pack_bf16(sc[q >> 1][2 * (q & 1)], sc[q >> 1][2 * (q & 1) + 1]));
+#pragma unroll
+    for (int i = 0; i < DH / 16; ++i) {
+        const uint4 a = vf.v[2 * i], b = vf.v[2 * i + 1];
+        st.o[i][0] *= alpha[0]; st.o[i][1] *= alpha[1]; st.o[i][2] *= alpha[0]; st.o[i][3] *= alpha[1];
+        mma_bf16(st.o[i], a.x, b.x, a.y, b.y, pb[0], pb[1]);
+        mma_bf16(st.o[i], a.z, b.z, a.w, b.w, pb[2], pb[3]);
+    }
+}
+
 }  // namespace attn
