@@ -80,3 +80,30 @@ def test_product_with_a_long_k_on_either_side_of_the_persistent_rule(shape, epil
     assert torch.isfinite(out).all()
     # one rounding to bfloat16 of a float32 sum; the sums themselves are within a few 1e-6 of each other
     assert bool(((out.float() - ref).abs() <= 2.0 ** -8 * ref.abs() + 1e-3).all())
+
+
+@pytest.mark.parametrize("tokens", [1, 9, 16, 17, 33, 64])
+@pytest.mark.parametrize("cfg", [(28, 4, 128, 3136), (40, 8, 128, 4104)])
+def test_rotation_in_the_epilogue_of_the_streaming_tcgen05_product(cfg, tokens):
+    """q|k|v of few tokens with long rows: a tile a head, its splits of k merged within a cluster."""
+    T.test_linear_rope_kv_fused(torch.bfloat16, (*cfg, tokens))
+
+
+@pytest.mark.parametrize("shape", [(1536, 8960), (128, 8192), (200, 4096), (3584, 3584), (5120, 4160)])
+def test_splits_of_k_in_clusters_do_not_depend_on_the_batch(shape):
+    """Each number of tokens that shares a token tile (16, 32, 64) gives a token the same bits, whoever merges its splits."""
+    N, Kd = shape
+    g = torch.Generator(device="cuda").manual_seed(N)
+    a = torch.randn((64, Kd), generator=g, device="cuda").to(torch.bfloat16)
+    w = (torch.randn((N, Kd), generator=g, device="cuda") * Kd ** -0.5).to(torch.bfloat16)
+    bias = torch.randn(N, generator=g, device="cuda")
+    ref = a.float() @ w.float().T + bias
+    for tile, counts in ((16, (1, 2, 5, 16)), (32, (17, 31, 32)), (64, (33, 50, 64))):
+        whole = None
+        for m in reversed(counts):
+            out = torch.full((m, N), float("nan"), device="cuda")
+            K().linear_with("gemv_tcgen05", a[:m].contiguous(), w, bias, out)
+            assert float((out - ref[:m]).abs().max()) <= 1e-4          # float32 sums of Kd terms of size Kd ** -0.5
+            if whole is not None:
+                assert torch.equal(out, whole[:m]), (tile, m)
+            whole = out if whole is None else whole
