@@ -182,8 +182,9 @@ prefill_attention_tc_kernel(const bf16* __restrict__ qkv, long long row_elems, c
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     // Tensor memory is taken only once the kernel before this one has finished: a CTA that waits for that kernel must not
-    // hold what a CTA of it may still ask for (gemm_tcgen05.cu has the story).
-    pdl_launch_dependents();
+    // hold what a CTA of it may still ask for (gemm_tcgen05.cu has the story).  And the kernel behind this one is let go only
+    // once this CTA holds it: the streaming product (gemv_tcgen05.cu) takes its columns before it waits, and with heads of 64
+    // its CTA has room beside this one.
     pdl_wait();
     if (warp == 1) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&sm.tmem_base)), "r"(kTmemCols) : "memory");
@@ -191,6 +192,7 @@ prefill_attention_tc_kernel(const bf16* __restrict__ qkv, long long row_elems, c
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
+    pdl_launch_dependents();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     // S of tile j at tmem_s + 128 (j & 1), and P of tile j over its first 64 columns (two bfloat16 a column)
     const unsigned tmem_s = sm.tmem_base, tmem_pv = sm.tmem_base + 256, tmem_q = sm.tmem_base + 384;

@@ -218,7 +218,8 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     // Tensor memory is taken only once the kernel before this one has finished (warp 1, below): a CTA that waits for
     // that kernel must not hold what a CTA of it may still ask for.  With the accumulators taken first and every launch a
     // dependent one, steps of thousands of tokens of a 7B-shaped model stopped in tcgen05.alloc about two runs in five.
-    // The warps that read the accumulator meet warp 1 at a named barrier once it has the address.
+    // The warps that read the accumulator meet warp 1 at a named barrier once it has the address.  The kernel behind this one
+    // is let go by that warp, once it has the columns: gemv_tcgen05.cu takes its own before it waits.
     constexpr int kAllocMeet = 32 + (threads_of<kRope>() - 64);
     auto take_tensor_memory = [&]() {
         pdl_wait();
@@ -231,6 +232,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                          : "memory");
             asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
         }
+        pdl_launch_dependents();
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     };
     auto meet_tensor_memory = [&]() {
@@ -240,7 +242,6 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     };
     // programmatic dependent launch: everything up to here overlapped the end of the kernel before this one; what reads
     // its results (the producer) or writes over memory it may still read (the epilogue) waits for it
-    pdl_launch_dependents();
 
     if (warp == 0) {
         if (lane == 0) {

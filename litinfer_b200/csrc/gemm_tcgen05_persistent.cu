@@ -71,7 +71,7 @@ gemm_tcgen05_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const 
     }
     // Tensor memory is taken only once the kernel before this one has finished: a CTA that waits for that kernel must not
     // hold what a CTA of it may still ask for (gemm_tcgen05.cu has the story).  Nothing here could start before that anyway.
-    pdl_launch_dependents();
+    // The kernel behind this one is let go once this CTA holds its columns.
     pdl_wait();
     if (warp == 1) {
         asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&sm.tmem_base)), "r"(kCols) : "memory");
@@ -79,6 +79,7 @@ gemm_tcgen05_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const 
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
+    pdl_launch_dependents();
     cluster_sync_all();                               // the other CTA's barriers are set up before anything arrives on them
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const unsigned tmem_acc = sm.tmem_base;
