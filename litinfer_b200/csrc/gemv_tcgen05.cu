@@ -110,8 +110,12 @@ __device__ __forceinline__ float peer_load(unsigned addr) {
 enum { kEpiNone = 0, kEpiSwiglu = 1, kEpiAddScaled = 2, kEpiGluClamped = 3, kEpiGeglu = 4, kEpiRope = 5 };     // (3 and 4: SwiGLU's layout, another activation)
 
 // kSplit: k is split over the CTAs of clusters of `csize` (the grid's y: splits, a cluster's consecutive).
+// The sum into the residual stream is held to two CTAs a multiprocessor: without the bound its 33 to 64 tokens took 255
+// registers, one CTA a multiprocessor, and clusters of five, six and eight, of which the GPU then holds 26, 22 and 15, no longer
+// ran all at once (64 tokens, N 3584, K 8960, 28 clusters of five: 40.5 us, with the bound 22.3; N 2048, K 8960 35.9 and 20.1).
+// The other forms stay below that number by themselves.
 template <int BT, typename Tout, int kEpi, bool kSplit>
-__global__ void __launch_bounds__(kThreads)
+__global__ void __launch_bounds__(kThreads, kEpi == kEpiAddScaled && BT >= 32 ? 2 : 0)
 gemv_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
                     const float* __restrict__ bias, Tout* __restrict__ out, float* __restrict__ partial,
                     unsigned* __restrict__ counters, int M, int N, int K, int ksplit, int csize, int* __restrict__ error_flag, const RowScale rs,
@@ -213,13 +217,17 @@ gemv_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
         // the tokens this CTA finishes: all of them, or every csize-th of a cluster's
         const int rank = kSplit ? split % csize : 0, step = kSplit ? csize : 1;
         float xold[kAdd ? kMine : 1];
-        if constexpr (kAdd) {
+        auto load_old = [&]() {
+            if constexpr (kAdd) {
 #pragma unroll
-            for (int i = 0; i < kMine; ++i) {
-                const int j = rank + i * step;
-                xold[i] = (j < M && row < N) ? __ldcg(add.x32 + (size_t)j * N + row) : 0.0f;
+                for (int i = 0; i < kMine; ++i) {
+                    const int j = rank + i * step;
+                    xold[i] = (j < M && row < N) ? __ldcg(add.x32 + (size_t)j * N + row) : 0.0f;
+                }
             }
-        }
+        };
+        // (32 tokens with a split: asked for when the partial tile has left its registers, else some of them spill)
+        if constexpr (!kSplit || BT != 32) load_old();
         const bool ok = mbar_wait(&sm.accum, 0);
         if (!ok && lane == 0) atomicExch(error_flag, 33);
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -232,6 +240,7 @@ gemv_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
 #pragma unroll
             for (int j = 0; j < BT; ++j)
                 if (j < M) mine[j * BR] = v[j];
+            if constexpr (BT == 32) load_old();
             cluster_arrive_wait();
             float t[kMine];
 #pragma unroll
