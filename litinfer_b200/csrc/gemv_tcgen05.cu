@@ -13,12 +13,13 @@
 // CTAs of a tile form clusters of up to eight: each leaves its float partial tile
 // in its shared memory, and CTA r of a cluster takes the tokens r, r + size, ...,
 // adds their sums in split order through distributed shared memory and does their
-// epilogue.  More than eight splits: clusters of four, whose sums meet in a
-// workspace where the last one to arrive (a counter per tile and place in the
-// cluster) adds them in order.  The number of splits depends on N, K and the token
-// tile only, so a token's result does not depend on the batch it is in.  (One CTA
-// that read every split's partial tile from the workspace took several round trips
-// for itself: 64 tokens, eight splits, 262 KB.)
+// epilogue.  More than eight splits (up to 16 tokens): clusters of four, whose sums
+// meet in a workspace where the last one to arrive (a counter per tile and place in
+// the cluster) adds them in order.  The splits are a function of N, K and the token
+// tile (up to 16, 32 or 64 tokens): within a tile a token's result does not depend
+// on how many others there are; from one tile to the next the order of its sums may
+// change.  (One CTA that read every split's partial tile from the workspace took
+// several round trips for itself: 64 tokens, eight splits, 262 KB.)
 // Epilogue: bias, or the SwiGLU of gate and up rows interleaved in groups of 8
 // (up * gate / (1 + exp(-gate)), src/ops/swiglu/op.cpp:17-23).
 //
@@ -423,11 +424,15 @@ int choose_ksplit(int N, int K, int bt) {
         if (ks > by_work) ks = by_work;
     }
     while (ks > 1 && (size_t)ks * tiles * 64 * BR > kWorkspaceFloats) --ks;      // the partial sums fit the workspace: sized for 64 tokens whatever M is
-    // many tokens: one cluster a tile (64 tokens, N 1536, K 8960: 21.8 us with three clusters of four, whose sums meet in the workspace)
-    if (bt == 64 && ks > 8) ks = 8;
+    // more than 16 tokens: one cluster a tile.  Clusters of four whose sums meet in the workspace write and read every CTA's share
+    // of the tokens once more (64 tokens, N 1536, K 8960: 21.8 us with three of them, 16.4 with one cluster of eight; 32 tokens
+    // 16.2 and 12.5, N 512, K 4096 19.7 and 8.2; up to 16 tokens, N 1536, K 18944 15.4 and 16.0)
+    if (bt >= 32 && ks > 8) ks = 8;
     if (ks > 8) ks -= ks % 4;                                         // clusters of four
     return ks;
 }
+int cluster_of(int ksplit) { return ksplit <= 8 ? ksplit : 4; }
+int token_tile(int M) { return M <= 16 ? 16 : M <= 32 ? 32 : 64; }
 
 template <int BT, typename Tout, int kEpi>
 int launch(const void* a, const void* w, const float* bias, void* out, int M, int N, int K, cudaStream_t stream, const RowScale& rs,
@@ -459,7 +464,7 @@ int launch(const void* a, const void* w, const float* bias, void* out, int M, in
         li_launch_pdl(gemv_tcgen05_kernel<BT, Tout, kEpi, false>, dim3(tiles, 1), dim3(kThreads), smem, stream, map_w, map_x, bias, (Tout*)out,
                       ws->partial, ws->counters, M, N, K, 1, 1, err_dev, rs, add, rope);
     } else {
-        const int csize = ksplit <= 8 ? ksplit : 4;
+        const int csize = cluster_of(ksplit);
         LI_REQUIRE(tiles * csize <= kMaxTiles, "linear (tcgen05 gemv): N=%d has too many tiles for a split of k", N);
         li_launch_pdl(gemv_tcgen05_kernel<BT, Tout, kEpi, true>, dim3(tiles, ksplit), dim3(kThreads), smem, stream, dim3(1, csize, 1), map_w, map_x, bias,
                       (Tout*)out, ws->partial, ws->counters, M, N, K, ksplit, csize, err_dev, rs, add, rope);
@@ -477,8 +482,17 @@ int launch_bt(const void* a, const void* w, const float* bias, void* out, int M,
 
 }  // namespace
 
-// 0: splits of k by shape; n > 0: n splits always.  For measurements.
+// 0: splits of k by shape; n > 0: n splits, as far as there are k-blocks, room in the workspace and whole clusters for them
+// (li_gemv_tcgen05_plan says how many it became).  For measurements.
 LI_EXPORT void li_gemv_tcgen05_force_ksplit(int n) { g_forced_ksplit = n; }
+
+// How a product of M <= 64 rows is cut: the splits of k, and how many of them form a cluster.  For tests.
+LI_EXPORT int li_gemv_tcgen05_plan(int M, int N, int K, int* splits, int* cluster) {
+    LI_REQUIRE(M >= 1 && M <= 64 && N >= 1 && K >= 8 && splits && cluster, "linear (tcgen05 gemv): no plan for M=%d N=%d K=%d", M, N, K);
+    *splits = choose_ksplit(N, K, token_tile(M));
+    *cluster = cluster_of(*splits);
+    return 0;
+}
 
 bool li_gemv_tcgen05_accepts(const void* a, const void* w, int M, int N, int K) {
     return M >= 1 && M <= 64 && N >= 1 && K >= 8 && K % 8 == 0 && ((uintptr_t)a % 16 == 0) && ((uintptr_t)w % 16 == 0);

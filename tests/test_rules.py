@@ -1,0 +1,31 @@
+"""The rules by which a call is given to one kernel or cut in one way, as far as the sizes decide."""
+
+from __future__ import annotations
+
+import ctypes
+
+import pytest
+
+
+def library():
+    from litinfer_b200 import kernels
+    return kernels.library()
+
+
+def plan(M, N, K):
+    splits, cluster = ctypes.c_int(), ctypes.c_int()
+    assert library().li_gemv_tcgen05_plan(M, N, K, ctypes.byref(splits), ctypes.byref(cluster)) == 0
+    return splits.value, cluster.value
+
+
+@pytest.mark.parametrize("N", [128, 512, 1536, 2048, 3584, 8192, 9472, 12288])
+@pytest.mark.parametrize("K", [64, 4096, 8960, 18944])
+def test_splits_of_the_streaming_product(N, K):
+    """The token tile decides, not the tokens; one cluster a tile from 17 tokens on; whole clusters."""
+    for counts in ((1, 7, 16), (17, 25, 32), (33, 64)):
+        plans = {plan(M, N, K) for M in counts}
+        assert len(plans) == 1
+        splits, cluster = plans.pop()
+        assert 1 <= splits <= max(1, K // 64) and splits % cluster == 0 and cluster <= 8
+        if counts[0] > 16:
+            assert splits == cluster
