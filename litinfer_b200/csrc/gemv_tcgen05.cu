@@ -29,6 +29,8 @@
 #include "row_scale.cuh"
 #include "tcgen05.cuh"
 
+#include <atomic>
+
 namespace {
 
 using namespace tc;
@@ -39,11 +41,15 @@ constexpr int kTargetCtas = 148;
 constexpr size_t kWorkspaceFloats = 4u << 20;
 constexpr int kMaxTiles = 1 << 16;
 
+// Stages: six (deep), or as many as two CTAs a multiprocessor leave room for.  Two are better where the CTAs come in several waves,
+// since the next tile streams in while the other's epilogue runs (64 tokens, N 37888, K 3584: 61 -> 49 us).  Where every CTA of
+// the launch has a multiprocessor to itself, four stages only keep less in flight (N 12288, K 18944: 102 us, with six 90).
+constexpr int kDeep = 6;
 template <int BT>
+constexpr int kShallow = BT <= 16 ? 6 : BT <= 32 ? 5 : 4;
+
+template <int BT, int kStages>
 struct __align__(1024) Smem {
-    // as many stages as two CTAs a multiprocessor leave room for: the next tile, or the next kernel's first one, streams in
-    // while the other's epilogue runs (64 tokens with six stages had room for one: N 37888, K 3584 61 -> 49 us)
-    static constexpr int kStages = BT <= 16 ? 6 : BT <= 32 ? 5 : 4;
     unsigned char w[kStages][BR * BK * 2];
     unsigned char x[kStages][BT * BK * 2];
     unsigned long long full[kStages];
@@ -115,7 +121,7 @@ enum { kEpiNone = 0, kEpiSwiglu = 1, kEpiAddScaled = 2, kEpiGluClamped = 3, kEpi
 // registers, one CTA a multiprocessor, and clusters of five, six and eight, of which the GPU then holds 26, 22 and 15, no longer
 // ran all at once (64 tokens, N 3584, K 8960, 28 clusters of five: 40.5 us, with the bound 22.3; N 2048, K 8960 35.9 and 20.1).
 // The other forms stay below that number by themselves.
-template <int BT, typename Tout, int kEpi, bool kSplit>
+template <int BT, typename Tout, int kEpi, bool kSplit, int kStages>
 __global__ void __launch_bounds__(kThreads, kEpi == kEpiAddScaled && BT >= 32 ? 2 : 0)
 gemv_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
                     const float* __restrict__ bias, Tout* __restrict__ out, float* __restrict__ partial,
@@ -124,7 +130,7 @@ gemv_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
     constexpr int kSwiglu = kEpi == kEpiSwiglu ? LI_EPILOGUE_SWIGLU : kEpi == kEpiGluClamped ? LI_EPILOGUE_GLU_CLAMPED : kEpi == kEpiGeglu ? LI_EPILOGUE_GEGLU : 0;
     constexpr bool kAdd = kEpi == kEpiAddScaled;
     extern __shared__ unsigned char smem_raw[];
-    Smem<BT>& sm = *reinterpret_cast<Smem<BT>*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+    Smem<BT, kStages>& sm = *reinterpret_cast<Smem<BT, kStages>*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int tile = blockIdx.x, split = blockIdx.y;
     const int n0 = tile * BR;
@@ -133,7 +139,6 @@ gemv_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
     const int nkb = kb1 - kb0;
     constexpr unsigned kStageBytes = BR * BK * 2 + BT * BK * 2;
     constexpr unsigned kCols = BT < 32 ? 32 : BT;
-    constexpr int kStages = Smem<BT>::kStages;
     constexpr int kMine = kSplit ? BT / 2 : BT;            // tokens a CTA finishes at most (a cluster has at least two)
 
     if (threadIdx.x == 0) {
@@ -434,6 +439,79 @@ int choose_ksplit(int N, int K, int bt) {
 int cluster_of(int ksplit) { return ksplit <= 8 ? ksplit : 4; }
 int token_tile(int M) { return M <= 16 ? 16 : M <= 32 ? 32 : 64; }
 
+// How many clusters of `csize` CTAs of a kernel the current device holds at once (asked once a size and device; a size that is asked
+// by two threads at the same time is asked twice).
+template <int BT, typename Tout, int kEpi, int kStages>
+int clusters_at_once(int csize) {
+    static std::atomic<int> known[16][9];
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 16) return 0;
+    int n = known[dev][csize].load(std::memory_order_relaxed);
+    if (n == 0) {
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(1, csize);
+        cfg.blockDim = dim3(kThreads);
+        cfg.dynamicSmemBytes = sizeof(Smem<BT, kStages>) + 1024;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = attr[0].val.clusterDim.z = 1;
+        attr[0].val.clusterDim.y = csize;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        if (cudaOccupancyMaxActiveClusters(&n, gemv_tcgen05_kernel<BT, Tout, kEpi, true, kStages>, &cfg) != cudaSuccess) {
+            cudaGetLastError();
+            n = 0;
+        }
+        known[dev][csize].store(n, std::memory_order_relaxed);
+    }
+    return n;
+}
+
+template <int BT, typename Tout, int kEpi, int kStages>
+int raise_shared() {
+    static bool raised = false;
+    if (raised) return 0;
+    const size_t smem = sizeof(Smem<BT, kStages>) + 1024;
+    cudaError_t e = cudaFuncSetAttribute(gemv_tcgen05_kernel<BT, Tout, kEpi, false, kStages>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(gemv_tcgen05_kernel<BT, Tout, kEpi, true, kStages>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return li_fail("linear (tcgen05 gemv): cannot raise shared memory to %zu: %s", smem, cudaGetErrorString(e));
+    raised = true;
+    return 0;
+}
+
+// Deep where the launch is one wave of CTAs with a multiprocessor each: without a split as many tiles as there are
+// multiprocessors at most, with one as many clusters as the device holds of that kernel at once.  (Clusters that do not all
+// fit must come two CTAs a multiprocessor: 64 tokens, N 3584, K 8960, 28 clusters of five: 19.1 us, deep 32.2.)
+template <int BT, typename Tout, int kEpi>
+int choose_deep(int tiles, int ksplit, bool* deep) {
+    *deep = false;
+    if (kShallow<BT> == kDeep) return 0;
+    if (ksplit == 1) {
+        *deep = tiles <= kTargetCtas;
+        return 0;
+    }
+    if (int rc = raise_shared<BT, Tout, kEpi, kDeep>()) return rc;
+    *deep = (long long)tiles * ksplit <= (long long)clusters_at_once<BT, Tout, kEpi, kDeep>(cluster_of(ksplit)) * cluster_of(ksplit);
+    return 0;
+}
+
+template <int BT, typename Tout, int kEpi, int kStages>
+int launch_stages(const CUtensorMap& map_w, const CUtensorMap& map_x, const float* bias, void* out, Workspace* ws, int M, int N, int K, int tiles, int ksplit,
+                  int* err_dev, const RowScale& rs, const AddScaled& add, const RopeArgs& rope, cudaStream_t stream) {
+    if (int rc = raise_shared<BT, Tout, kEpi, kStages>()) return rc;
+    const size_t smem = sizeof(Smem<BT, kStages>) + 1024;
+    if (ksplit == 1) {
+        li_launch_pdl(gemv_tcgen05_kernel<BT, Tout, kEpi, false, kStages>, dim3(tiles, 1), dim3(kThreads), smem, stream, map_w, map_x, bias, (Tout*)out,
+                      ws->partial, ws->counters, M, N, K, 1, 1, err_dev, rs, add, rope);
+    } else {
+        const int csize = cluster_of(ksplit);
+        LI_REQUIRE(tiles * csize <= kMaxTiles, "linear (tcgen05 gemv): N=%d has too many tiles for a split of k", N);
+        li_launch_pdl(gemv_tcgen05_kernel<BT, Tout, kEpi, true, kStages>, dim3(tiles, ksplit), dim3(kThreads), smem, stream, dim3(1, csize, 1), map_w, map_x, bias,
+                      (Tout*)out, ws->partial, ws->counters, M, N, K, ksplit, csize, err_dev, rs, add, rope);
+    }
+    return li_check_launch("linear (tcgen05 gemv)");
+}
+
 template <int BT, typename Tout, int kEpi>
 int launch(const void* a, const void* w, const float* bias, void* out, int M, int N, int K, cudaStream_t stream, const RowScale& rs,
            const AddScaled& add, const RopeArgs& rope) {
@@ -452,24 +530,10 @@ int launch(const void* a, const void* w, const float* bias, void* out, int M, in
     CUtensorMap map_w, map_x;
     if (int rc = make_map(&map_w, w, N, K, BR)) return rc;
     if (int rc = make_map(&map_x, a, M, K, BT)) return rc;
-    const size_t smem = sizeof(Smem<BT>) + 1024;
-    static bool raised = false;
-    if (!raised) {
-        cudaError_t e = cudaFuncSetAttribute(gemv_tcgen05_kernel<BT, Tout, kEpi, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(gemv_tcgen05_kernel<BT, Tout, kEpi, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return li_fail("linear (tcgen05 gemv): cannot raise shared memory to %zu: %s", smem, cudaGetErrorString(e));
-        raised = true;
-    }
-    if (ksplit == 1) {
-        li_launch_pdl(gemv_tcgen05_kernel<BT, Tout, kEpi, false>, dim3(tiles, 1), dim3(kThreads), smem, stream, map_w, map_x, bias, (Tout*)out,
-                      ws->partial, ws->counters, M, N, K, 1, 1, err_dev, rs, add, rope);
-    } else {
-        const int csize = cluster_of(ksplit);
-        LI_REQUIRE(tiles * csize <= kMaxTiles, "linear (tcgen05 gemv): N=%d has too many tiles for a split of k", N);
-        li_launch_pdl(gemv_tcgen05_kernel<BT, Tout, kEpi, true>, dim3(tiles, ksplit), dim3(kThreads), smem, stream, dim3(1, csize, 1), map_w, map_x, bias,
-                      (Tout*)out, ws->partial, ws->counters, M, N, K, ksplit, csize, err_dev, rs, add, rope);
-    }
-    return li_check_launch("linear (tcgen05 gemv)");
+    bool deep = false;
+    if (int rc = choose_deep<BT, Tout, kEpi>(tiles, ksplit, &deep)) return rc;
+    return deep ? launch_stages<BT, Tout, kEpi, kDeep>(map_w, map_x, bias, out, ws, M, N, K, tiles, ksplit, err_dev, rs, add, rope, stream)
+                : launch_stages<BT, Tout, kEpi, kShallow<BT>>(map_w, map_x, bias, out, ws, M, N, K, tiles, ksplit, err_dev, rs, add, rope, stream);
 }
 
 template <typename Tout, int kEpi>
@@ -486,11 +550,20 @@ int launch_bt(const void* a, const void* w, const float* bias, void* out, int M,
 // (li_gemv_tcgen05_plan says how many it became).  For measurements.
 LI_EXPORT void li_gemv_tcgen05_force_ksplit(int n) { g_forced_ksplit = n; }
 
-// How a product of M <= 64 rows is cut: the splits of k, and how many of them form a cluster.  For tests.
-LI_EXPORT int li_gemv_tcgen05_plan(int M, int N, int K, int* splits, int* cluster) {
+// How a product of M <= 64 rows is cut: the splits of k, and how many of them form a cluster; with `deep` (needs a device)
+// whether its plain form takes the deep pipeline.  For tests.
+LI_EXPORT int li_gemv_tcgen05_plan(int M, int N, int K, int* splits, int* cluster, int* deep) {
     LI_REQUIRE(M >= 1 && M <= 64 && N >= 1 && K >= 8 && splits && cluster, "linear (tcgen05 gemv): no plan for M=%d N=%d K=%d", M, N, K);
     *splits = choose_ksplit(N, K, token_tile(M));
     *cluster = cluster_of(*splits);
+    if (deep) {
+        bool d = false;
+        const int tiles = ceil_div(N, BR);
+        if (int rc = token_tile(M) == 16 ? choose_deep<16, bf16, kEpiNone>(tiles, *splits, &d)
+                     : token_tile(M) == 32 ? choose_deep<32, bf16, kEpiNone>(tiles, *splits, &d) : choose_deep<64, bf16, kEpiNone>(tiles, *splits, &d))
+            return rc;
+        *deep = d;
+    }
     return 0;
 }
 

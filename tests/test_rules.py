@@ -12,9 +12,9 @@ def library():
     return kernels.library()
 
 
-def plan(M, N, K):
+def plan(M, N, K, deep=None):
     splits, cluster = ctypes.c_int(), ctypes.c_int()
-    assert library().li_gemv_tcgen05_plan(M, N, K, ctypes.byref(splits), ctypes.byref(cluster)) == 0
+    assert library().li_gemv_tcgen05_plan(M, N, K, ctypes.byref(splits), ctypes.byref(cluster), None if deep is None else ctypes.byref(deep)) == 0
     return splits.value, cluster.value
 
 
@@ -29,3 +29,22 @@ def test_splits_of_the_streaming_product(N, K):
         assert 1 <= splits <= max(1, K // 64) and splits % cluster == 0 and cluster <= 8
         if counts[0] > 16:
             assert splits == cluster
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("M", [32, 64])
+def test_pipeline_depth_of_the_streaming_product(M):
+    """Six stages where every CTA has a multiprocessor to itself, fewer where the CTAs come in waves or the clusters do not all fit."""
+    import torch
+
+    torch.zeros(1, device="cuda")
+
+    def deep(N, K=8960):
+        d = ctypes.c_int()
+        plan(M, N, K, d)
+        return d.value
+
+    assert deep(128 * 148, 3584) == 1 and deep(128 * 149, 3584) == 0
+    assert deep(1536) == 1 and deep(5120) == 1 and deep(8192) == 1
+    # 16 clusters of eight: a B200 holds 15 of them with a multiprocessor a CTA
+    assert plan(M, 2048, 8960) == (8, 8) and deep(2048) == 0
