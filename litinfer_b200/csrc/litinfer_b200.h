@@ -435,6 +435,12 @@ int li_argmax(const float* logits, int* out, int R, int V, cudaStream_t stream);
  * max with a counter-based generator, independent of the batch. */
 int li_sample(const float* logits, const int* params, int* out, int R, int V, cudaStream_t stream);
 
+/* The same; small_top_k 0 says that no row has a top_k of 2 to 256. */
+int li_sample_rows(const float* logits, const int* params, int* out, int R, int V, int small_top_k, cudaStream_t stream);
+
+/* Tests: 1 leaves -1 in the rows that the pass for a small top_k does not settle by itself (0: they are drawn another way). */
+void li_sample_leave_rows(int on);
+
 /* ---- fill_random.cu ---- */
 /* out[i] = mean + std * n(key, i), n standard normal from a counter-based generator (a pure function of key and i). */
 int li_fill_normal(void* out, int dtype, long long n, unsigned long long key, float mean, float std, cudaStream_t stream);

@@ -23,10 +23,10 @@
 // Large vocabularies with a small top_k (sample_topk_kernel, the usual options): a cluster of blocks a row, one pass.  Each
 // thread keeps the maximum of its elements; the k-th largest of a block's thread maxima is a bound below the row's
 // k-th largest value, and only the few threads whose maximum reaches it are looked through again, by their whole warp.
-// The candidates, the sums over them (the same order, so the same bits) and the draw are those of the general kernel,
-// which takes whatever this one leaves (NaN, too many equal values, other options).  64 rows of 151,936, top-k 50 and
-// top-p 0.8: 20 us (two blocks a row); six passes by one block a row and 32 block-wide sums for the second threshold took
-// 136 us.
+// The candidates, the sums over them (the same order, so the same bits) and the draw are those of the general way,
+// by which the cluster's first block does whatever row this leaves (NaN, too many equal values, other options).  64 rows
+// of 151,936, top-k 50 and top-p 0.8: 20 us (two blocks a row); six passes by one block a row and 32 block-wide sums for
+// the second threshold took 136 us.
 #include "common.cuh"
 
 #include <cooperative_groups.h>
@@ -364,6 +364,114 @@ __device__ unsigned block_exclusive_scan(unsigned v, SelectShared& sh, unsigned*
     return r;
 }
 
+struct GeneralShared {
+    Best scratch[32];
+    float fscratch[32];
+    SelectShared select;
+};
+
+// A row by one block, whatever its options.  chunked_plain: rows with temperature alone are drawn by
+// sample_temperature_chunks_kernel, launched behind; here they only get the first maximum as a stand-in (which stays if the
+// row has nothing finite).
+__device__ __noinline__ void sample_row(const float* __restrict__ row, const int* __restrict__ pr, int* __restrict__ out, int V, int chunked_plain, GeneralShared& gs) {
+    Best* scratch = gs.scratch;
+    float* fscratch = gs.fscratch;
+    SelectShared& sh = gs.select;
+    const float temperature = __int_as_float(pr[0]);
+    const int top_k = pr[1];
+    const float top_p = __int_as_float(pr[2]);
+    const unsigned long long seed = (unsigned long long)(unsigned)pr[3] | ((unsigned long long)(unsigned)pr[4] << 32);
+    const unsigned long long index = (unsigned long long)(long long)pr[5];
+
+    const bool use_k = top_k > 0 && top_k < V, use_p = top_p > 0.0f && top_p < 1.0f;
+    if (chunked_plain && temperature > 0.0f && top_k != 1 && !use_k && !use_p) {
+        if (threadIdx.x == 0) *out = 0;                // stands only if the row has nothing finite (what the first maximum would give)
+        return;
+    }
+    const Best top = row_argmax(row, V, scratch);
+    if (temperature <= 0.0f || top_k == 1) {
+        if (threadIdx.x == 0) *out = top.i;
+        return;
+    }
+    if (V <= kCand || !(use_k || use_p) || (use_k && top_k > kCand)) {
+        sample_row_by_bisection(row, V, temperature, top_k, top_p, seed, index, top, out, scratch, fscratch);
+        return;
+    }
+    const float zmax = top.v / temperature;
+    // the k-th largest key (top-k), or the kCand-th largest (top-p alone)
+    if (threadIdx.x == 0) {
+        sh.prefix = 0;
+        sh.need = use_k ? (unsigned)top_k : (unsigned)kCand;
+    }
+    __syncthreads();
+    float zsum = 0.0f;                                   // over the whole row, for top-p alone: sum of exp(z - zmax) in a fixed order
+    select_round(row, V, temperature, 0u, 21, 11, sh, [&](int, float z, unsigned) { zsum += expf(z - zmax); });
+    select_round(row, V, temperature, 0xFFE00000u, 10, 11, sh, [](int, float, unsigned) {});
+    select_round(row, V, temperature, 0xFFFFFC00u, 0, 10, sh, [](int, float, unsigned) {});
+    const unsigned kth = sh.prefix;
+    // candidates: keys >= the k-th largest (top-k: equal values stay together), keys > the kCand-th largest (top-p alone)
+    const unsigned low = use_k ? kth : kth + 1u;          // kth < 0xFFFFFFFF: it is the key of a finite or infinite float, never all ones
+    unsigned mine = 0;
+    for_each_element(row, V, [&](int, float x) { mine += sortable(x / temperature) >= low ? 1u : 0u; });
+    unsigned total = 0;
+    unsigned at = block_exclusive_scan(mine, sh, &total);
+    if (total > (unsigned)kCand || total == 0) {          // more equal values than fit, or nothing finite: the slow way decides
+        sample_row_by_bisection(row, V, temperature, top_k, top_p, seed, index, top, out, scratch, fscratch);
+        return;
+    }
+    for_each_element(row, V, [&](int i, float x) {
+        const unsigned key = sortable(x / temperature);
+        if (key >= low) {
+            sh.ckey[at] = key;
+            sh.cidx[at] = i;
+            ++at;
+        }
+    });
+    __syncthreads();
+    const int C = (int)total;
+    unsigned keep_from = low;
+    if (use_p) {
+        float zc = 0.0f;
+        for (int j = threadIdx.x; j < C; j += blockDim.x) zc += expf(unsortable(sh.ckey[j]) - zmax);
+        zc = block_sum(zc, fscratch);
+        float target;
+        if (use_k) {
+            target = top_p * zc;                          // the mass after top-k
+        } else {
+            const float zall = block_sum(zsum, fscratch);
+            target = top_p * zall;
+            if (!(zc >= target)) {                        // the gathered tokens hold less than top_p of the mass: the cut is below them
+                sample_row_by_bisection(row, V, temperature, top_k, top_p, seed, index, top, out, scratch, fscratch);
+                return;
+            }
+        }
+        unsigned lo = low, hi = 0xFFFFFFFFu;
+        while (lo < hi) {
+            const unsigned mid = lo + ((hi - lo) >> 1);
+            float mass = 0.0f;
+            for (int j = threadIdx.x; j < C; j += blockDim.x) {
+                const unsigned key = sh.ckey[j];
+                if (key > mid) mass += expf(unsortable(key) - zmax);
+            }
+            mass = block_sum(mass, fscratch);
+            if (mass < target) hi = mid; else lo = mid + 1;
+        }
+        if (lo > keep_from) keep_from = lo;
+    }
+    const unsigned long long key = splitmix64(seed ^ splitmix64(index));
+    Best b{-INFINITY, 0x7fffffff};
+    for (int j = threadIdx.x; j < C; j += blockDim.x) {
+        const unsigned kj = sh.ckey[j];
+        if (kj >= keep_from) {
+            const int i = sh.cidx[j];
+            const float v = unsortable(kj) + gumbel(key, i);
+            if (v > b.v || (v == b.v && i < b.i)) b = Best{v, i};
+        }
+    }
+    b = block_best(b, scratch);
+    if (threadIdx.x == 0) *out = (b.i == 0x7fffffff) ? top.i : b.i;
+}
+
 // The rows that sample_topk_kernel looks at (a vocabulary that leaves every thread of its blocks something).
 constexpr int kFastK = 256, kFastCand = 1024, kFastVocab = 16384;
 __device__ __forceinline__ bool fast_options(float temperature, int top_k, int V) {
@@ -381,11 +489,20 @@ struct FastShared {
     Best scratch[32];
 };
 
-// out[r] = the row's token, or -1: sample_kernel, launched behind this one, takes the row.
+// A row by the cluster's blocks in one pass if its options are such and the pass settles it, else by the first block alone
+// (sample_row), in the same launch.  A caller that knows of no such row does not launch it (li_sample_rows): its blocks
+// are in the way of the kernels around them (8 rows of 151,936 with temperature alone: 12.6 us without, 18.2 with).
+// leave: rows that the pass does not settle get -1 instead.
 template <bool kVec>
-__global__ void __launch_bounds__(kThreads) sample_topk_kernel(const float* __restrict__ logits, const int* __restrict__ params, int* __restrict__ out, int V) {
+__global__ void __launch_bounds__(kThreads) sample_topk_kernel(const float* __restrict__ logits, const int* __restrict__ params, int* __restrict__ out, int V,
+                                                               int chunked_plain, int leave) {
     namespace cg = cooperative_groups;
-    __shared__ FastShared sh;
+    __shared__ union Shared {
+        FastShared fast;
+        GeneralShared general;
+        __device__ Shared() {}
+    } shared;
+    FastShared& sh = shared.fast;
     cg::cluster_group cluster = cg::this_cluster();
     pdl_launch_dependents();
     pdl_wait();
@@ -395,11 +512,19 @@ __global__ void __launch_bounds__(kThreads) sample_topk_kernel(const float* __re
     const float temperature = __int_as_float(pr[0]);
     const int top_k = pr[1];
     const float top_p = __int_as_float(pr[2]);
+    const float* row = logits + (size_t)r * V;
+    auto otherwise = [&]() {                              // (called by the whole first block, once no other block looks at its memory)
+        if (leave) {
+            if (tid == 0) out[r] = -1;
+            return;
+        }
+        __syncthreads();
+        sample_row(row, pr, out + r, V, chunked_plain, shared.general);
+    };
     if (!fast_options(temperature, top_k, V)) {           // (the whole cluster agrees)
-        if (rank == 0 && tid == 0) out[r] = -1;
+        if (rank == 0) otherwise();
         return;
     }
-    const float* row = logits + (size_t)r * V;
     const int per = ((V + blocks - 1) / blocks + 3) & ~3;
     const int lo = min(V, rank * per), hi = min(V, lo + per);
     // a thread's elements: four in a row at 4 (tid + 1024 j)
@@ -476,7 +601,7 @@ __global__ void __launch_bounds__(kThreads) sample_topk_kernel(const float* __re
     if (rank != 0) return;
     const int n = (int)sh.count;
     if (give_up || n > kFastCand || n < top_k) {          // (uniform)
-        if (tid == 0) out[r] = -1;
+        otherwise();
         return;
     }
     const unsigned key = tid < n ? sortable(sh.x[tid] / temperature) : 0u;
@@ -534,118 +659,26 @@ __global__ void __launch_bounds__(kThreads) sample_topk_kernel(const float* __re
         if (v > best.v) best = Best{v, sh.oidx[tid]};
     }
     best = block_best(best, sh.scratch);
-    if (tid == 0) out[r] = best.i == 0x7fffffff ? -1 : best.i;
+    if (tid == 0) sh.count = best.i == 0x7fffffff;
+    __syncthreads();
+    if (sh.count) otherwise();                            // no candidate has a number
+    else if (tid == 0) out[r] = best.i;
 }
 
-// chunked_plain: rows with temperature alone are drawn by sample_temperature_chunks_kernel, launched after this kernel; here
-// they only get the first maximum as a stand-in (which stays if the row has nothing finite).
 __global__ void __launch_bounds__(kThreads) sample_kernel(const float* __restrict__ logits, const int* __restrict__ params,
-                                                          int* __restrict__ out, int V, int chunked_plain, int fast) {
-    __shared__ Best scratch[32];
-    __shared__ float fscratch[32];
-    __shared__ SelectShared sh;
+                                                          int* __restrict__ out, int V, int chunked_plain) {
+    __shared__ GeneralShared sh;
     pdl_launch_dependents();
     pdl_wait();
-    const int r = blockIdx.x;
-    const float* row = logits + (size_t)r * V;
-    const int* pr = params + r * 6;
-    const float temperature = __int_as_float(pr[0]);
-    const int top_k = pr[1];
-    const float top_p = __int_as_float(pr[2]);
-    const unsigned long long seed = (unsigned long long)(unsigned)pr[3] | ((unsigned long long)(unsigned)pr[4] << 32);
-    const unsigned long long index = (unsigned long long)(long long)pr[5];
-
-    const bool use_k = top_k > 0 && top_k < V, use_p = top_p > 0.0f && top_p < 1.0f;
-    if (fast && fast_options(temperature, top_k, V) && out[r] >= 0) return;
-    if (chunked_plain && temperature > 0.0f && top_k != 1 && !use_k && !use_p) {
-        if (threadIdx.x == 0) out[r] = 0;                // stands only if the row has nothing finite (what the first maximum would give)
-        return;
-    }
-    const Best top = row_argmax(row, V, scratch);
-    if (temperature <= 0.0f || top_k == 1) {
-        if (threadIdx.x == 0) out[r] = top.i;
-        return;
-    }
-    if (V <= kCand || !(use_k || use_p) || (use_k && top_k > kCand)) {
-        sample_row_by_bisection(row, V, temperature, top_k, top_p, seed, index, top, out + r, scratch, fscratch);
-        return;
-    }
-    const float zmax = top.v / temperature;
-    // the k-th largest key (top-k), or the kCand-th largest (top-p alone)
-    if (threadIdx.x == 0) {
-        sh.prefix = 0;
-        sh.need = use_k ? (unsigned)top_k : (unsigned)kCand;
-    }
-    __syncthreads();
-    float zsum = 0.0f;                                   // over the whole row, for top-p alone: sum of exp(z - zmax) in a fixed order
-    select_round(row, V, temperature, 0u, 21, 11, sh, [&](int, float z, unsigned) { zsum += expf(z - zmax); });
-    select_round(row, V, temperature, 0xFFE00000u, 10, 11, sh, [](int, float, unsigned) {});
-    select_round(row, V, temperature, 0xFFFFFC00u, 0, 10, sh, [](int, float, unsigned) {});
-    const unsigned kth = sh.prefix;
-    // candidates: keys >= the k-th largest (top-k: equal values stay together), keys > the kCand-th largest (top-p alone)
-    const unsigned low = use_k ? kth : kth + 1u;          // kth < 0xFFFFFFFF: it is the key of a finite or infinite float, never all ones
-    unsigned mine = 0;
-    for_each_element(row, V, [&](int, float x) { mine += sortable(x / temperature) >= low ? 1u : 0u; });
-    unsigned total = 0;
-    unsigned at = block_exclusive_scan(mine, sh, &total);
-    if (total > (unsigned)kCand || total == 0) {          // more equal values than fit, or nothing finite: the slow way decides
-        sample_row_by_bisection(row, V, temperature, top_k, top_p, seed, index, top, out + r, scratch, fscratch);
-        return;
-    }
-    for_each_element(row, V, [&](int i, float x) {
-        const unsigned key = sortable(x / temperature);
-        if (key >= low) {
-            sh.ckey[at] = key;
-            sh.cidx[at] = i;
-            ++at;
-        }
-    });
-    __syncthreads();
-    const int C = (int)total;
-    unsigned keep_from = low;
-    if (use_p) {
-        float zc = 0.0f;
-        for (int j = threadIdx.x; j < C; j += blockDim.x) zc += expf(unsortable(sh.ckey[j]) - zmax);
-        zc = block_sum(zc, fscratch);
-        float target;
-        if (use_k) {
-            target = top_p * zc;                          // the mass after top-k
-        } else {
-            const float zall = block_sum(zsum, fscratch);
-            target = top_p * zall;
-            if (!(zc >= target)) {                        // the gathered tokens hold less than top_p of the mass: the cut is below them
-                sample_row_by_bisection(row, V, temperature, top_k, top_p, seed, index, top, out + r, scratch, fscratch);
-                return;
-            }
-        }
-        unsigned lo = low, hi = 0xFFFFFFFFu;
-        while (lo < hi) {
-            const unsigned mid = lo + ((hi - lo) >> 1);
-            float mass = 0.0f;
-            for (int j = threadIdx.x; j < C; j += blockDim.x) {
-                const unsigned key = sh.ckey[j];
-                if (key > mid) mass += expf(unsortable(key) - zmax);
-            }
-            mass = block_sum(mass, fscratch);
-            if (mass < target) hi = mid; else lo = mid + 1;
-        }
-        if (lo > keep_from) keep_from = lo;
-    }
-    const unsigned long long key = splitmix64(seed ^ splitmix64(index));
-    Best b{-INFINITY, 0x7fffffff};
-    for (int j = threadIdx.x; j < C; j += blockDim.x) {
-        const unsigned kj = sh.ckey[j];
-        if (kj >= keep_from) {
-            const int i = sh.cidx[j];
-            const float v = unsortable(kj) + gumbel(key, i);
-            if (v > b.v || (v == b.v && i < b.i)) b = Best{v, i};
-        }
-    }
-    b = block_best(b, scratch);
-    if (threadIdx.x == 0) out[r] = (b.i == 0x7fffffff) ? top.i : b.i;
+    sample_row(logits + (size_t)blockIdx.x * V, params + blockIdx.x * 6, out + blockIdx.x, V, chunked_plain, sh);
 }
 
+int g_leave = 0;
+
 }  // namespace
+
+// 1: rows that the one pass of sample_topk_kernel does not settle get -1.  For tests.
+LI_EXPORT void li_sample_leave_rows(int on) { g_leave = on; }
 
 LI_EXPORT int li_argmax(const float* logits, int* out, int R, int V, cudaStream_t stream) {
     LI_REQUIRE(R >= 0 && V > 0, "argmax: bad sizes R=%d V=%d", R, V);
@@ -658,27 +691,32 @@ LI_EXPORT int li_argmax(const float* logits, int* out, int R, int V, cudaStream_
     return li_check_launch("argmax");
 }
 
-LI_EXPORT int li_sample(const float* logits, const int* params, int* out, int R, int V, cudaStream_t stream) {
+// small_top_k: whether some row may have a top_k of 2 to 256 (else its kernel is not launched).
+LI_EXPORT int li_sample_rows(const float* logits, const int* params, int* out, int R, int V, int small_top_k, cudaStream_t stream) {
     LI_REQUIRE(R >= 0 && V > 0, "sample: bad sizes R=%d V=%d", R, V);
     LI_REQUIRE(V < (1 << 24), "sample: vocabulary %d is too large", V);
     if (R == 0) return 0;
     // few rows of a large vocabulary: rows with temperature alone are drawn over many CTAs by a second kernel
     const int chunked_plain = (R <= 64 && R <= kChunkRows && V >= 16384) ? 1 : 0;
-    // rows with a small top-k: two to eight blocks a row, as many as fill the GPU once (from 65 rows on one block a row does)
-    const int fast = (R <= 64 && V >= kFastVocab) ? 1 : 0;
-    if (fast) {
-        const int blocks = R > 32 ? 2 : R > 16 ? 4 : 8;
+    // rows with a small top-k: two to eight blocks a row, as many as there is room for at once, a block a multiprocessor (15 clusters
+    // of eight, 33 of four, 74 of two; 16 rows in clusters of eight: 24 us, of four 15)
+    if (R <= 64 && V >= kFastVocab && small_top_k) {
+        const int blocks = R > 32 ? 2 : R > 15 ? 4 : 8;
         if (V % 4 == 0 && (uintptr_t)logits % 16 == 0)
-            li_launch_pdl(sample_topk_kernel<true>, dim3(blocks, R), dim3(kThreads), 0, stream, dim3(blocks, 1, 1), logits, params, out, V);
+            li_launch_pdl(sample_topk_kernel<true>, dim3(blocks, R), dim3(kThreads), 0, stream, dim3(blocks, 1, 1), logits, params, out, V, chunked_plain, g_leave);
         else
-            li_launch_pdl(sample_topk_kernel<false>, dim3(blocks, R), dim3(kThreads), 0, stream, dim3(blocks, 1, 1), logits, params, out, V);
-        if (int rc = li_check_launch("sample (top-k)")) return rc;
+            li_launch_pdl(sample_topk_kernel<false>, dim3(blocks, R), dim3(kThreads), 0, stream, dim3(blocks, 1, 1), logits, params, out, V, chunked_plain, g_leave);
+    } else {
+        li_launch_pdl(sample_kernel, dim3(R), dim3(kThreads), 0, stream, logits, params, out, V, chunked_plain);
     }
-    li_launch_pdl(sample_kernel, dim3(R), dim3(kThreads), 0, stream, logits, params, out, V, chunked_plain, fast);
     if (int rc = li_check_launch("sample")) return rc;
     if (chunked_plain) {
         li_launch_pdl(sample_temperature_chunks_kernel, dim3(kDrawChunks, R), dim3(256), 0, stream, logits, params, out, V);
         return li_check_launch("sample (temperature, chunks)");
     }
     return 0;
+}
+
+LI_EXPORT int li_sample(const float* logits, const int* params, int* out, int R, int V, cudaStream_t stream) {
+    return li_sample_rows(logits, params, out, R, V, 1, stream);
 }
