@@ -472,10 +472,16 @@ __device__ __noinline__ void sample_row(const float* __restrict__ row, const int
     if (threadIdx.x == 0) *out = (b.i == 0x7fffffff) ? top.i : b.i;
 }
 
-// The rows that sample_topk_kernel looks at (a vocabulary that leaves every thread of its blocks something).
+// The rows that sample_topk_kernel looks at: a vocabulary that leaves most threads of its blocks something, and a top_k whose
+// candidates are few.  A block's bound, the top_k-th largest of its threads' maxima, is reached by a little more than top_k
+// of its elements, and the largest of the blocks' bounds by as many of every other block's: about blocks x top_k
+// candidates, of which there is room for 1,024.  Each is ranked against all: beyond an element in forty of the row the general
+// way is as fast, and a large top_k of a small vocabulary is not worth its cut at top_p.  Measured, general way / this one,
+// us: 16,384 x 8 rows, top_k 50, top_p 0.8 35.2 / 27.7, top_k 128 21.8 / 65; 32,000 x 33 rows, top_k 256, top_p 0.9 49 / 59;
+// 151,936 x 8 rows, top_k 128 121 / 65, top_k 256 (2,300 candidates, so both ways one after the other) 134 / 150.
 constexpr int kFastK = 256, kFastCand = 1024, kFastVocab = 16384;
-__device__ __forceinline__ bool fast_options(float temperature, int top_k, int V) {
-    return temperature > 0.0f && top_k > 1 && top_k <= kFastK && V >= kFastVocab;
+__device__ __forceinline__ bool fast_options(float temperature, int top_k, int V, int blocks) {
+    return temperature > 0.0f && top_k > 1 && top_k <= kFastK && V >= kFastVocab && top_k <= V / 160 && blocks * top_k <= min(V / 40, kFastCand);
 }
 
 struct FastShared {
@@ -521,7 +527,7 @@ __global__ void __launch_bounds__(kThreads) sample_topk_kernel(const float* __re
         __syncthreads();
         sample_row(row, pr, out + r, V, chunked_plain, shared.general);
     };
-    if (!fast_options(temperature, top_k, V)) {           // (the whole cluster agrees)
+    if (!fast_options(temperature, top_k, V, blocks)) {           // (the whole cluster agrees)
         if (rank == 0) otherwise();
         return;
     }

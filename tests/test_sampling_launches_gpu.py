@@ -48,6 +48,28 @@ def test_the_sampler_says_which_options_its_rows_have(monkeypatch):
     assert said == [False, True, True, False]
 
 
+@pytest.mark.parametrize("V", [16384, 16387, 32000, 151936])
+@pytest.mark.parametrize("R", [1, 15, 16, 32, 33, 64])
+def test_ordinary_rows_are_settled_in_one_pass(R, V):
+    """Where the candidates of a row are few: eight blocks a row up to 15 rows, four up to 32, then two."""
+    g = torch.Generator(device="cuda").manual_seed(V + R)
+    x = torch.randn((R, V), generator=g, device="cuda") * 2.5
+    blocks = 8 if R <= 15 else 4 if R <= 32 else 2
+    most = min(256, V // 160, min(V // 40, 1024) // blocks)                # the largest top_k that is taken
+    ks = [50 if most >= 50 else 20, min(most, 800 // blocks), 20, 2, most + 1]
+    p = params([(0.8, ks[i % 5], (0.8, 1.0)[i % 2], 100 + i, i) for i in range(R)])
+    got, all_rows = torch.full((R,), -7, dtype=torch.int32, device="cuda"), torch.empty(R, dtype=torch.int32, device="cuda")
+    K().sample(x, p, all_rows)
+    K().library().li_sample_leave_rows(1)
+    try:
+        K().sample(x, p, got)
+        torch.cuda.synchronize()
+    finally:
+        K().library().li_sample_leave_rows(0)
+    assert min(all_rows.tolist()) >= 0
+    assert got.tolist() == [-1 if i % 5 == 4 else t for i, t in enumerate(all_rows.tolist())]
+
+
 def test_rows_that_the_pass_leaves():
     """Other options, rows with no number, and more equal values than there is room for."""
     x = torch.randn((6, 30000), device="cuda")
