@@ -200,14 +200,19 @@ int launch(const void* a, const void* w, const float* bias, void* out, int M, in
 
 }  // namespace
 
-// Worth it when a pair of multiprocessors gets more than one tile, whatever k is (measured against 256 x 256 tiles of one CTA
-// each: gate|up of K 1536 and 512 rows, 140 tiles: 29 us against 33 us; 2,048 rows: 94 us against 138 us; K 5120, N 27648:
-// 640 rows 149 against 184 us, 2,048 rows 385 against 428 us; K 13824, N 5120, 2,048 rows 224 against 300 us).
+// Worth it when a pair of multiprocessors gets more than one tile (measured against 256 x 256 tiles of one CTA each: gate|up of
+// K 1536 and 512 rows, 140 tiles: 29 us against 33 us; 2,048 rows: 94 us against 138 us; K 5120, N 27648: 640 rows 149 against
+// 184 us, 2,048 rows 385 against 428 us; K 13824, N 5120, 2,048 rows 224 against 300 us), except where the single CTAs fill one
+// wave (up to 148 tiles: a pair then takes two of its tiles in the time a CTA takes one of its own) and k is so long that the
+// epilogue hardly counts: 2,048 rows, N 4096, 128 tiles, K 4160 66.6 against 68.6 us, K 8192 111.0 against 107.8, K 13824 183.0
+// against 175.9; 150 tiles, K 13824 228 against 300.
 bool li_tcgen05_persistent_wanted(int M, int N, int K) {
     const long long total = (long long)((ceil_div(M, kRows) + 1) / 2) * ceil_div(N, BN);
-    (void)K;
-    return total >= 120;
+    return total >= 120 && (total > 148 || ceil_div(K, BK) < 128);
 }
+
+// The same, for tests of the rule.
+LI_EXPORT int li_tcgen05_takes_persistent(int M, int N, int K) { return li_tcgen05_persistent_wanted(M, N, K) ? 1 : 0; }
 
 int li_linear_tcgen05_persistent(const void* a, const void* w, const float* bias, void* out, int dtype_out, int M, int N, int K, int epilogue,
                                  cudaStream_t stream) {

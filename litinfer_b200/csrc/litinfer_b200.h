@@ -256,6 +256,10 @@ void li_tcgen05_force_tile(int tile);
 /* Tests and measurements: force the splits of k of the tcgen05 product (0: by shape). */
 void li_tcgen05_force_ksplit(int n);
 
+/* ---- gemm_tcgen05_persistent.cu ---- */
+/* Tests: 1 if a tcgen05 product of these sizes goes to the persistent kernel. */
+int li_tcgen05_takes_persistent(int M, int N, int K);
+
 /* ---- gemv_bf16.cu ---- */
 /* The weight-streaming product for callers that may not allocate (see no_alloc.h). */
 int li_linear_gemv_static(const void* a, const void* w, const float* bias, void* out, int dtype_out, int M, int N, int

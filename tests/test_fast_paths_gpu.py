@@ -63,7 +63,9 @@ def test_rotation_in_the_epilogue_of_wide_long_steps(cfg):
     T.test_linear_rope_kv_fused(torch.bfloat16, cfg)
 
 
-@pytest.mark.parametrize("shape", [(640, 15360, 4224), (520, 13000, 4168), (769, 12800, 5120)])
+# (tiles of 256 x 256: 180, 153 and 200, then 119, 120 with less than 8,192 columns of k and with more, 150)
+@pytest.mark.parametrize("shape", [(640, 15360, 4224), (520, 13000, 4168), (769, 12800, 5120), (1792, 4352, 4168), (2048, 3840, 4168), (2048, 3840, 8200),
+                                   (2560, 3840, 8200)])
 @pytest.mark.parametrize("epilogue", [None, "swiglu"])
 def test_product_with_a_long_k_on_either_side_of_the_persistent_rule(shape, epilogue):
     M, N, Kd = shape

@@ -48,3 +48,11 @@ def test_pipeline_depth_of_the_streaming_product(M):
     assert deep(1536) == 1 and deep(5120) == 1 and deep(8192) == 1
     # 16 clusters of eight: a B200 holds 15 of them with a multiprocessor a CTA
     assert plan(M, 2048, 8960) == (8, 8) and deep(2048) == 0
+
+
+@pytest.mark.parametrize("tiles,M,N", [(119, 1792, 4352), (120, 2048, 3840), (128, 900, 8192), (144, 2304, 4096), (148, 1024, 9472), (150, 2560, 3840), (256, 2048, 8192)])
+def test_which_products_the_persistent_kernel_takes(tiles, M, N):
+    """From 120 tiles of 256 x 256 on; up to 148, which single CTAs do in one wave, only with less than 8,192 columns of k."""
+    assert -(-M // 256) * -(-N // 256) == tiles
+    for K in (1536, 4160, 8128, 8192, 13824):
+        assert library().li_tcgen05_takes_persistent(M, N, K) == (tiles >= 120 and (tiles > 148 or K < 8129))
