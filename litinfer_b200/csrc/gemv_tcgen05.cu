@@ -587,7 +587,7 @@ int li_linear_gemv_tcgen05(const void* a, const void* w, const float* bias, void
 }
 
 // The fused q|k|v projection with rotary encoding and cache write in its epilogue: heads of 128 (rotated whole or not at all),
-// a tile a head.  Against the register-fed kernel's (li_linear_gemv_rope) where its rows are long: linear.cu says from where.
+// a tile a head.  Against the register-fed kernel's (li_linear_gemv_rope) where its rows are long: rope.cu says from where.
 bool li_gemv_tcgen05_rope_accepts(const void* a, const void* w, int M, int N, int K, int nh, int nkv, int dh, int rotary_dim) {
     return li_gemv_tcgen05_accepts(a, w, M, N, K) && dh == BR && (rotary_dim == dh || rotary_dim == 0) && N == (nh + 2 * nkv) * dh;
 }

@@ -32,7 +32,7 @@ bool li_gemv_tcgen05_accepts(const void* a, const void* w, int M, int N, int K);
 // Whether a product of few rows goes to the tcgen05 kernel with swapped operands rather than to the register-fed one
 // (register-fed / tcgen05, us, 1 and 64 rows: 3584 x 3584 9.4 / 8.1 and 20.8 / 12.6; 4608 x 3584 10.3 / 9.6 and 21.4 / 13.8; but
 // 1536 x 3584 4.5 / 7.2 and 10.4 / 12.2, 1536 x 1536 2.9 / 6.2 and 5.8 / 10.6: few short tiles leave a split too little to do).
-bool li_few_rows_take_tcgen05(int N, int K) {
+static bool few_rows_take_tcgen05(int N, int K) {
     const int tiles = (N + 127) / 128, nkb = (K + 63) / 64;
     if (tiles >= 96) return true;                              // fills the GPU without a split of k
     if (nkb >= 64) return true;                                // a split of k leaves every CTA enough to stream (measured: down projection)
@@ -49,7 +49,7 @@ namespace {
 int few_rows_kernel(const void* a, const void* w, const void* out, int M, int N, int K) {
     const bool aligned = ((uintptr_t)a % 16 == 0) && ((uintptr_t)w % 16 == 0) && ((uintptr_t)out % 16 == 0);
     if (!aligned || M > 64) return 0;
-    if (li_few_rows_take_tcgen05(N, K) && li_gemv_tcgen05_accepts(a, w, M, N, K)) return 3;
+    if (few_rows_take_tcgen05(N, K) && li_gemv_tcgen05_accepts(a, w, M, N, K)) return 3;
     if (li_gemv_bf16_accepts(M, N, K)) return 1;
     return 0;
 }

@@ -304,6 +304,9 @@ int li_linear_with(int which, const void* a, const void* w, const float* bias, v
 /* out[t, j] = (cos, sin)(positions[t] / denom[j]). */
 int li_rope_table(const int* positions, const float* denom, int half, float* out, int T, cudaStream_t stream);
 
+/* Tests: 1 if q|k|v [N, K] of T <= 64 tokens with heads of 128 goes to the tcgen05 kernel. */
+int li_rope_takes_tcgen05(int T, int N, int K);
+
 /* Rotate q in place, rotate k and store it, store v (transposed) at slot_mapping[t] of the paged caches. */
 int li_rope_kv_write(void* qkv, int dtype, const int* positions, const float* denom, int rotary_dim, const int*
     slot_mapping, void* kcache, void* vcache, int T, int nh, int nkv, int dh, int page_size, int num_pages, int write,

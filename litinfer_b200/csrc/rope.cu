@@ -267,7 +267,21 @@ bool li_gemv_rope_accepts(const void* a, const void* w, int M, int N, int K, int
 bool li_gemv_tcgen05_rope_accepts(const void* a, const void* w, int M, int N, int K, int nh, int nkv, int dh, int rotary_dim);
 int li_linear_gemv_tcgen05_rope(const void* a, const void* w, const float* bias, void* out, int M, int N, int K, const RopeArgs& rope, const RowScale& rs,
                                 cudaStream_t stream);
-bool li_few_rows_take_tcgen05(int N, int K);
+
+// Whether q|k|v of T <= 64 tokens with heads of 128 goes to the tcgen05 kernel rather than to the register-fed one, which is
+// never split along k here.  With few tiles the merge of the tcgen05 kernel's splits outweighs them however long the rows are:
+// register-fed / tcgen05, us, 8 tokens: 20 tiles of 128 rows, K 4096 9.9 / 8.7, 24 tiles, K 3072 9.1 / 8.3, but 18 tiles, K 4096
+// 5.6 / 8.2, 6 tiles, K 4096 4.5 / 8.8.  With more than 32 tokens the tcgen05 kernel wins from 8,192 columns of k on whatever the
+// tiles (33 tokens, 10 tiles 18.0 / 16.1, with 32 tokens 14.0 / 16.2).
+static bool few_tokens_rope_on_tcgen05(int T, int N, int K) {
+    const int tiles = (N + 127) / 128, nkb = (K + 63) / 64;
+    if (T > 32 && nkb >= 128) return true;
+    return tiles >= 96 || (nkb >= 64 && tiles >= 20) || (nkb >= 48 && tiles >= 24);
+}
+
+// The same, for tests of the rule.
+LI_EXPORT int li_rope_takes_tcgen05(int T, int N, int K) { return few_tokens_rope_on_tcgen05(T, N, K) ? 1 : 0; }
+
 bool li_tcgen05_rope_wanted(const void* a, const void* w, const void* out, int M, int N, int K);
 int li_linear_tcgen05_rope(const void* a, const void* w, const float* bias, void* out, int M, int N, int K, const RopeEpilogue& rope,
                            cudaStream_t stream);
@@ -311,7 +325,7 @@ LI_EXPORT int li_linear_rope_kv(const void* a, const void* w, const float* bias,
         rs.width = (float)width;
         rs.eps = eps;
     }
-    if (allow_fused && dtype == LI_BF16 && li_few_rows_take_tcgen05(N, K) && li_gemv_tcgen05_rope_accepts(a, w, T, N, K, nh, nkv, dh, rotary_dim)) {
+    if (allow_fused && dtype == LI_BF16 && few_tokens_rope_on_tcgen05(T, N, K) && li_gemv_tcgen05_rope_accepts(a, w, T, N, K, nh, nkv, dh, rotary_dim)) {
         const RopeArgs ra{positions, rotary_dim ? denom : nullptr, slot_mapping, (bf16*)kcache, (bf16*)vcache, nh, nkv, dh, page_size, num_pages, write,
                           (bf16*)extra_out, extra};
         return li_linear_gemv_tcgen05_rope(a, w, bias, qkv, T, N, K, ra, rs, stream);

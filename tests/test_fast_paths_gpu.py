@@ -85,7 +85,8 @@ def test_product_with_a_long_k_on_either_side_of_the_persistent_rule(shape, epil
 
 
 @pytest.mark.parametrize("tokens", [1, 9, 16, 17, 33, 64])
-@pytest.mark.parametrize("cfg", [(28, 4, 128, 3136), (40, 8, 128, 4104)])
+# (few heads: on the register-fed kernel but for more than 32 tokens with rows of 8,192)
+@pytest.mark.parametrize("cfg", [(28, 4, 128, 3136), (40, 8, 128, 4104), (16, 2, 128, 4096), (4, 1, 128, 4104), (4, 1, 128, 8200)])
 def test_rotation_in_the_epilogue_of_the_streaming_tcgen05_product(cfg, tokens):
     """q|k|v of few tokens with long rows: a tile a head, its splits of k merged within a cluster."""
     T.test_linear_rope_kv_fused(torch.bfloat16, (*cfg, tokens))

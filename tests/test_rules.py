@@ -56,3 +56,13 @@ def test_which_products_the_persistent_kernel_takes(tiles, M, N):
     assert -(-M // 256) * -(-N // 256) == tiles
     for K in (1536, 4160, 8128, 8192, 13824):
         assert library().li_tcgen05_takes_persistent(M, N, K) == (tiles >= 120 and (tiles > 148 or K < 8129))
+
+
+@pytest.mark.parametrize("heads,K,taken", [(6, 4096, 0), (18, 4096, 0), (10, 8128, 0), (20, 4096, 1), (20, 4032, 0), (24, 3072, 1), (24, 3008, 0), (23, 3072, 0), (36, 3584, 1),
+                                           (96, 256, 1), (95, 256, 0)])
+def test_which_q_k_v_of_few_tokens_the_tcgen05_kernel_takes(heads, K, taken):
+    """Few heads stay on the register-fed kernel however long their rows are (more than 32 tokens: up to 8,192 columns)."""
+    for T in (1, 32, 33, 64):
+        assert library().li_rope_takes_tcgen05(T, heads * 128, K) == taken
+    assert library().li_rope_takes_tcgen05(33, heads * 128, 8192) == 1
+    assert library().li_rope_takes_tcgen05(32, heads * 128, 8192) == (heads >= 20)
