@@ -8,7 +8,7 @@
 // (16-byte copies, rows 16 bytes further apart than they are long), a lane a key for the scores, a lane every 32nd element
 // for the values.  The units' results (maximum, denominator, weighted values) are merged in ascending order with a running
 // maximum, so that a token's output does not depend on how many warps or blocks shared its units out: a block of four
-// warps alone where there are many tokens, a cluster of eight blocks a token where there are few.  A round's merge takes
+// warps alone where there are many tokens, a cluster of up to eight blocks a token where there are few.  A round's merge takes
 // its factors for all units at once (a lane a unit, the running maximum by a scan), then one multiply-add a unit and output.
 // Scores, exponentials (full precision), sums and weighted values are float.
 //
@@ -251,6 +251,17 @@ attention_f32_kernel(const float* __restrict__ qkv, float* __restrict__ out, con
     }
 }
 
+// Blocks of a cluster that share a token's units and the outputs of its merge (1, 2, 4 or 8), for `pairs` (token, key/value head,
+// part of its heads): as many as one wave of blocks has room for, however short the contexts are (a token of 12 heads on 2 at
+// 8 keys, one unit: 9.1 us with eight, whose warps share the merge, 12.6 with one).  (Eight below 128 pairs, one from there on: a
+// prompt of 16 tokens of 28 heads on 4 took four waves of clusters, 44.4 us against 21.4 of the general kernel.)
+int attention_f32_cluster(long long pairs, int dh) {
+    const long long room = 148LL * (dh > 64 ? 1 : 2);                        // blocks at once, by shared memory and registers
+    int c = 8;
+    while (c > 1 && pairs * c > room) c /= 2;
+    return c;
+}
+
 // heads a block: a key/value head's group in equal parts of at most eight
 int heads_of(int nh, int nkv) {
     const int G = nh / nkv;
@@ -262,9 +273,7 @@ int launch(const void* qkv, void* out, const void* kcache, const void* vcache, c
            const int* positions, int T, int nh, int nkv, int dh, int page_size, int num_pages, float scale, int window, const AttentionOptions& opt,
            cudaStream_t stream) {
     const int groups = ceil_div(nh / nkv, NH);
-    // one block of four warps a (token, key/value head) from about one such block a multiprocessor on; below that a cluster of
-    // eight blocks shares a token's units (a launch does not know how long the contexts are: short ones leave blocks idle)
-    const int csize = (long long)T * nkv * groups >= 128 ? 1 : 8;
+    const int csize = attention_f32_cluster((long long)T * nkv * groups, dh);
     static bool raised = false;
     if (!raised) {
         cudaError_t e = cudaFuncSetAttribute(attention_f32_kernel<NH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(shared_floats(kMaxDim) * sizeof(float)));
@@ -292,6 +301,11 @@ int launch(const void* qkv, void* out, const void* kcache, const void* vcache, c
 bool li_attention_f32_accepts(const void* qkv, const void* kcache, const void* vcache, int nh, int nkv, int dh, int page_size, const AttentionOptions& opt) {
     return opt.maps == 1 && dh % 4 == 0 && dh <= kMaxDim && page_size % 16 == 0 && nkv * ceil_div(nh / nkv, heads_of(nh, nkv)) <= 65535 &&
            (uintptr_t)kcache % 16 == 0 && (uintptr_t)vcache % 16 == 0 && (uintptr_t)qkv % 4 == 0;
+}
+
+// For tests of the rule.
+LI_EXPORT int li_attention_f32_blocks(int T, int nh, int nkv, int dh) {
+    return attention_f32_cluster((long long)T * nkv * ceil_div(nh / nkv, heads_of(nh, nkv)), dh);
 }
 
 int li_attention_f32(const void* qkv, void* out, const void* kcache, const void* vcache, const int* block_table, int max_blocks, const int* seq_of_token,

@@ -256,6 +256,10 @@ void li_tcgen05_force_tile(int tile);
 /* Tests and measurements: force the splits of k of the tcgen05 product (0: by shape). */
 void li_tcgen05_force_ksplit(int n);
 
+/* ---- attention_f32.cu ---- */
+/* Tests: how many blocks share a token's keys in the float32 attention of a step of T tokens. */
+int li_attention_f32_blocks(int T, int nh, int nkv, int dh);
+
 /* ---- gemm_tcgen05_persistent.cu ---- */
 /* Tests: 1 if a tcgen05 product of these sizes goes to the persistent kernel. */
 int li_tcgen05_takes_persistent(int M, int N, int K);

@@ -122,3 +122,23 @@ def test_attention_does_not_depend_on_the_batch():
     whole = run(0, 100)
     for lo, hi in ((0, 1), (57, 60), (99, 100)):
         assert torch.equal(run(lo, hi), whole[lo:hi])
+
+
+@pytest.mark.parametrize("longest", [700, 2500])
+def test_attention_in_clusters_of_every_size(longest):
+    """One block to eight a token, by how many tokens there are: the same bits."""
+    nh, nkv, dh, page = 12, 2, 128, 16
+    c = on_device(make_attention_case([100], [longest], nh, nkv, dh, page, torch.float32, seed=9))
+
+    def run(n):
+        out = torch.empty((n, nh * dh), device="cuda")
+        K().paged_attention(c["qkv"][:n].contiguous(), out, c["k_cache"], c["v_cache"], c["block_table"], torch.tensor([0, n], dtype=torch.int32, device="cuda"),
+                            c["ctx_lens"], c["seq_of_token"][:n].contiguous(), c["positions"][:n].contiguous(), nh, nkv, dh, dh ** -0.5, None, n, longest,
+                            implementation="float32")
+        return out
+
+    whole, seen = run(100), set()
+    for n in (1, 9, 18, 37, 70):
+        seen.add(K().library().li_attention_f32_blocks(n, nh, nkv, dh))
+        assert torch.equal(run(n), whole[:n])
+    assert {2, 4, 8} <= seen

@@ -66,3 +66,13 @@ def test_which_q_k_v_of_few_tokens_the_tcgen05_kernel_takes(heads, K, taken):
         assert library().li_rope_takes_tcgen05(T, heads * 128, K) == taken
     assert library().li_rope_takes_tcgen05(33, heads * 128, 8192) == 1
     assert library().li_rope_takes_tcgen05(32, heads * 128, 8192) == (heads >= 20)
+
+
+def test_blocks_that_share_a_token_in_float32_attention():
+    """As many as one wave has room for: 148 with heads of more than 64 elements, 296 with smaller ones."""
+    def blocks(T, nh, nkv, dh):
+        return library().li_attention_f32_blocks(T, nh, nkv, dh)
+
+    assert [blocks(T, 12, 2, 128) for T in (1, 9, 10, 18, 19, 37, 38, 2048)] == [8, 8, 4, 4, 2, 2, 1, 1]
+    assert [blocks(T, 32, 1, 64) for T in (9, 10, 18, 19, 37, 38)] == [8, 4, 4, 2, 2, 1]          # 32 heads: four parts
+    assert blocks(16, 28, 4, 128) == 2
