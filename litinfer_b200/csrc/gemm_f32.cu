@@ -236,7 +236,9 @@ f32_tile_kernel(const float* __restrict__ A, const float* __restrict__ W, const 
     TileSmem<TM>& sm = *reinterpret_cast<TileSmem<TM>*>(raw4);
     constexpr int BM = 8 * TM, kLoadsA = (BM + 31) / 32;
     const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;             // a thread: rows 4 ty .. (and 32 + 4 ty ..), columns 4 tx .. and 64 + 4 tx ..
-    const int m0 = (int)blockIdx.x * BM, n0 = (int)blockIdx.y * kBN;
+    // tiles of rows run fastest, so that a tile of w is read by neighbours; all tiles along x, which has room for any N
+    const int mt = (M + BM - 1) / BM;
+    const int m0 = (int)blockIdx.x % mt * BM, n0 = (int)blockIdx.x / mt * kBN;
     const int csize = (int)gridDim.z, rank = (int)blockIdx.z;
     const int nseg = (K + kSegment - 1) / kSegment;
     const int lr = tid >> 2, lk = (tid & 3) * 4;           // loads: rows lr + 32 r, four k from lk on
@@ -442,9 +444,9 @@ int launch_stream(const float* a, const float* w, const float* bias, float* out,
 
 template <int TM, bool kVec>
 int launch_tile(const float* a, const float* w, const float* bias, float* out, int M, int N, int K, cudaStream_t stream) {
-    const int mt = ceil_div(M, 8 * TM), nt = ceil_div(N, kBN);
-    LI_REQUIRE(nt <= 65535, "linear: N=%d is too large for one launch", N);
-    const int c = tile_cluster((long long)mt * nt, ceil_div(K, kSegment));
+    const long long tiles = ceil_div_ll(M, 8 * TM) * ceil_div_ll(N, kBN);
+    LI_REQUIRE(tiles <= 2147483647LL, "linear: M=%d, N=%d are too large for one launch", M, N);
+    const int c = tile_cluster(tiles, ceil_div(K, kSegment));
     const size_t most = sizeof(TileSmem<TM>) + (TM - 1) * sizeof(float4) * kThreadsT;      // room for a cluster of two
     const size_t smem = sizeof(TileSmem<TM>) + (c > 1 ? (ceil_div(2 * TM, c) - 1) * sizeof(float4) * kThreadsT : 0);
     static bool raised = false;
@@ -453,7 +455,7 @@ int launch_tile(const float* a, const float* w, const float* bias, float* out, i
         if (e != cudaSuccess) return li_fail("linear (float32): cannot raise shared memory to %zu: %s", most, cudaGetErrorString(e));
         raised = true;
     }
-    li_launch_pdl(f32_tile_kernel<TM, kVec>, dim3(mt, nt, c), dim3(kThreadsT), smem, stream, dim3(1, 1, c), a, w, bias, out, M, N, K);
+    li_launch_pdl(f32_tile_kernel<TM, kVec>, dim3((unsigned)tiles, 1, c), dim3(kThreadsT), smem, stream, dim3(1, 1, c), a, w, bias, out, M, N, K);
     return li_check_launch("linear (float32)");
 }
 

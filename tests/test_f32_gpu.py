@@ -142,3 +142,18 @@ def test_attention_in_clusters_of_every_size(longest):
         seen.add(K().library().li_attention_f32_blocks(n, nh, nkv, dh))
         assert torch.equal(run(n), whole[:n])
     assert {2, 4, 8} <= seen
+
+
+@pytest.mark.parametrize("rows", [3, 17, 70])
+def test_more_columns_than_a_grid_has_rows_of_blocks(rows):
+    """8.4 million columns, 65,537 tiles of 128, in products of small whole numbers."""
+    N = 65536 * 128 + 5
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    a = torch.randint(-3, 4, (rows, 4), generator=g, device="cuda").float()
+    w = torch.randint(-3, 4, (N, 4), generator=g, device="cuda").float()
+    out = torch.empty((rows, N), device="cuda")
+    K().linear(a, w, None, out)
+    for r in range(0, rows, 16):
+        assert torch.equal(out[r], (w * a[r]).sum(1))
+    assert torch.equal(out[rows - 1], (w * a[rows - 1]).sum(1))
+
