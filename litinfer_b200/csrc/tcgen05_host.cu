@@ -9,6 +9,9 @@ static EncodeTiledFn g_encode = nullptr;
 static int* g_error_host = nullptr;       // mapped pinned memory: the kernels write, the host reads without a sync
 static int* g_error_dev = nullptr;
 
+// The first call may come inside a stream capture: the products in float32 use these kernels' tensor maps and status word, and a
+// program may capture one before it has launched any.  (The allocation of pinned memory is a call that a capture forbids
+// unless the thread asks for the relaxed mode meanwhile; it puts nothing on a stream.)
 int setup(EncodeTiledFn* encode, int** error_host, int** error_dev) {
     if (!g_encode) {
         void* fn = nullptr;
@@ -19,11 +22,19 @@ int setup(EncodeTiledFn* encode, int** error_host, int** error_dev) {
         g_encode = reinterpret_cast<EncodeTiledFn>(fn);
     }
     if (!g_error_host) {
-        cudaError_t e = cudaHostAlloc((void**)&g_error_host, 1024 * sizeof(int), cudaHostAllocMapped);      // [0]: the status word; the rest: progress marks of kernels that are asked to leave them
-        if (e != cudaSuccess) return li_fail("tcgen05: cannot allocate the status word: %s", cudaGetErrorString(e));
-        for (int i = 0; i < 1024; ++i) g_error_host[i] = 0;
-        e = cudaHostGetDevicePointer((void**)&g_error_dev, g_error_host, 0);
-        if (e != cudaSuccess) return li_fail("tcgen05: cannot map the status word: %s", cudaGetErrorString(e));
+        int *host = nullptr, *dev = nullptr;
+        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+        cudaThreadExchangeStreamCaptureMode(&mode);
+        cudaError_t e = cudaHostAlloc((void**)&host, 1024 * sizeof(int), cudaHostAllocMapped);      // [0]: the status word; the rest: progress marks of kernels that are asked to leave them
+        if (e == cudaSuccess) {
+            for (int i = 0; i < 1024; ++i) host[i] = 0;
+            e = cudaHostGetDevicePointer((void**)&dev, host, 0);
+            if (e != cudaSuccess) cudaFreeHost(host);
+        }
+        cudaThreadExchangeStreamCaptureMode(&mode);
+        if (e != cudaSuccess) return li_fail("tcgen05: cannot allocate and map the status word: %s", cudaGetErrorString(e));
+        g_error_dev = dev;
+        g_error_host = host;
     }
     *encode = g_encode;
     *error_host = g_error_host;

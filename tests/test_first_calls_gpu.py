@@ -1,0 +1,37 @@
+"""The first call of a process where a program may make it: inside a stream capture."""
+
+from __future__ import annotations
+
+import subprocess
+import sys
+from pathlib import Path
+
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+ROOT = Path(__file__).resolve().parent.parent
+
+CAPTURED = """
+import torch
+from litinfer_b200 import kernels as K
+a, w, out = torch.randn(ROWS, 256, device="cuda"), torch.randn(300, 256, device="cuda"), torch.zeros(ROWS, 300, device="cuda")
+torch.cuda.synchronize()
+g = torch.cuda.CUDAGraph()
+with torch.cuda.graph(g):
+    K.linear(a, w, None, out)
+g.replay()
+torch.cuda.synchronize()
+# float32 sums of 256 products of numbers about 1, in two orders
+assert float((out.double() - a.double() @ w.double().T).abs().max()) < 1e-3
+"""
+
+def run(program):
+    r = subprocess.run([sys.executable, "-c", program], cwd=ROOT, capture_output=True, text=True, timeout=240)
+    assert r.returncode == 0, r.stderr[-2000:]
+
+
+@pytest.mark.parametrize("rows", [3, 40])
+def test_float32_product_captured_before_any_other_call(rows):
+    run(CAPTURED.replace("ROWS", str(rows)))
+
