@@ -3,6 +3,8 @@
 // kernels raise when a bounded wait runs out, and the status query of the C interface.
 #include "tcgen05.cuh"
 
+#include <mutex>
+
 namespace tc {
 
 static EncodeTiledFn g_encode = nullptr;
@@ -12,7 +14,19 @@ static int* g_error_dev = nullptr;
 // The first call may come inside a stream capture: the products in float32 use these kernels' tensor maps and status word, and a
 // program may capture one before it has launched any.  (The allocation of pinned memory is a call that a capture forbids
 // unless the thread asks for the relaxed mode meanwhile; it puts nothing on a stream.)
+// Any thread may be the first, and several at once.  The driver's encoder of tensor maps wants a current context, which a thread
+// that has not called the runtime before does not have.
 int setup(EncodeTiledFn* encode, int** error_host, int** error_dev) {
+    static thread_local bool has_context = false;
+    if (!has_context) {
+        int dev = 0;
+        cudaError_t e = cudaGetDevice(&dev);
+        if (e == cudaSuccess) e = cudaSetDevice(dev);
+        if (e != cudaSuccess) return li_fail("tcgen05: no current device: %s", cudaGetErrorString(e));
+        has_context = true;
+    }
+    static std::mutex lock;
+    std::lock_guard<std::mutex> guard(lock);
     if (!g_encode) {
         void* fn = nullptr;
         cudaDriverEntryPointQueryResult q;

@@ -1,4 +1,4 @@
-"""The first call of a process where a program may make it: inside a stream capture."""
+"""The first call of a process where a program may make it: inside a stream capture, and on several threads at once."""
 
 from __future__ import annotations
 
@@ -26,6 +26,35 @@ torch.cuda.synchronize()
 assert float((out.double() - a.double() @ w.double().T).abs().max()) < 1e-3
 """
 
+THREADS = """
+import threading, torch
+from litinfer_b200 import kernels as K
+K.library()
+a, w = torch.randn(3, 256, device="cuda"), torch.randn(300, 256, device="cuda")
+outs, failed = [torch.zeros(3, 300, device="cuda") for _ in range(16)], []
+torch.cuda.synchronize()
+start = threading.Barrier(16)
+def work(out):
+    start.wait()
+    try:
+        with torch.cuda.stream(torch.cuda.Stream()):
+            K.linear(a, w, None, out)
+            torch.cuda.current_stream().synchronize()
+    except Exception as e:
+        failed.append(e)
+threads = [threading.Thread(target=work, args=(o,)) for o in outs]
+[t.start() for t in threads]
+[t.join() for t in threads]
+start = threading.Barrier(1)
+outs.append(torch.zeros(3, 300, device="cuda"))
+late = threading.Thread(target=work, args=(outs[-1],))
+late.start()
+late.join()
+assert not failed, failed
+assert all(torch.equal(o, outs[0]) for o in outs)
+"""
+
+
 def run(program):
     r = subprocess.run([sys.executable, "-c", program], cwd=ROOT, capture_output=True, text=True, timeout=240)
     assert r.returncode == 0, r.stderr[-2000:]
@@ -35,3 +64,6 @@ def run(program):
 def test_float32_product_captured_before_any_other_call(rows):
     run(CAPTURED.replace("ROWS", str(rows)))
 
+
+def test_float32_product_first_called_by_many_threads():
+    run(THREADS)
