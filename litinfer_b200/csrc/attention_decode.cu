@@ -207,11 +207,7 @@ int launch(const void* qkv, void* out, const void* kcache, const void* vcache, c
     // that takes; with one unit per pair, the kernel without a merge takes it.
     constexpr int KBS = DH <= 128 ? 32 : 16;
     const long long pairs = (long long)(expected > 0 && expected < S ? expected : S) * nkv;
-    static const int sms = [] {
-        int dev = 0, n = 0;
-        if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) n = 148;
-        return n;
-    }();
+    const int sms = li_multiprocessors();
     const int blocks = ceil_div(max_ctx_len > 0 ? max_ctx_len : 1, KBS * kWarps);          // units of one round that the longest context can have
     const int want = (int)(pairs >= sms ? 1 : sms / pairs);                              // units per pair that fill the GPU once
     if (want == 1 && blocks > 1) {
@@ -220,11 +216,10 @@ int launch(const void* qkv, void* out, const void* kcache, const void* vcache, c
         constexpr int W = kColumns ? 12 : 8, KB = KBS;
         const size_t wsmem = (2 * W * 16 + (size_t)W * G * DH) * sizeof(float);
         if (wsmem <= 200 * 1024) {
-            static bool raised = false;
-            if (!raised && wsmem > 48 * 1024) {
-                cudaError_t e = cudaFuncSetAttribute(decode_attention_whole_kernel<DH, W, KB, kMod, kColumns>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+            if (wsmem > 48 * 1024) {
+                static LiOncePerDevice raised;
+                cudaError_t e = li_raise_shared(raised, (const void*)decode_attention_whole_kernel<DH, W, KB, kMod, kColumns>, 200 * 1024);
                 if (e != cudaSuccess) return li_fail("attention (decode): cannot raise shared memory: %s", cudaGetErrorString(e));
-                raised = true;
             }
             // Launched plainly: with CTAs that were there before the q|k|v product had finished a step of 64 sequences took longer
             // (1.5B shape 2.78 against 2.53 ms, 61 sequences of the 7B shape 5.16 against 4.88 ms).
@@ -249,12 +244,11 @@ int launch(const void* qkv, void* out, const void* kcache, const void* vcache, c
     size_t smem_floats = 2 * kWarps * 16 + (size_t)kWarps * G * DH;
     if (smem_floats < (size_t)G * (nsplit + 1)) smem_floats = (size_t)G * (nsplit + 1);      // the final merge reuses the buffer
     const size_t smem = smem_floats * sizeof(float);
-    static bool attr_set = false;
-    if (!attr_set && smem > 48 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(decode_attention_kernel<DH, KBS, false, kMod, kColumns>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(decode_attention_kernel<DH, KBS, true, kMod, kColumns>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+    if (smem > 48 * 1024) {
+        static LiOncePerDevice raised[2];
+        cudaError_t e = li_raise_shared(raised[0], (const void*)decode_attention_kernel<DH, KBS, false, kMod, kColumns>, 200 * 1024);
+        if (e == cudaSuccess) e = li_raise_shared(raised[1], (const void*)decode_attention_kernel<DH, KBS, true, kMod, kColumns>, 200 * 1024);
         if (e != cudaSuccess) return li_fail("attention (decode): cannot raise shared memory: %s", cudaGetErrorString(e));
-        attr_set = true;
     }
     LI_REQUIRE(smem <= 200 * 1024, "attention (decode): shared memory %zu too large", smem);
     LI_REQUIRE(S <= 65535 && nkv <= 65535, "attention (decode): batch %d or kv heads %d too large for one launch", S, nkv);

@@ -274,12 +274,9 @@ int launch(const void* qkv, void* out, const void* kcache, const void* vcache, c
            cudaStream_t stream) {
     const int groups = ceil_div(nh / nkv, NH);
     const int csize = attention_f32_cluster((long long)T * nkv * groups, dh);
-    static bool raised = false;
-    if (!raised) {
-        cudaError_t e = cudaFuncSetAttribute(attention_f32_kernel<NH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(shared_floats(kMaxDim) * sizeof(float)));
-        if (e != cudaSuccess) return li_fail("attention (float32): cannot raise shared memory: %s", cudaGetErrorString(e));
-        raised = true;
-    }
+    static LiOncePerDevice raised;
+    cudaError_t e = li_raise_shared(raised, (const void*)attention_f32_kernel<NH>, shared_floats(kMaxDim) * sizeof(float));
+    if (e != cudaSuccess) return li_fail("attention (float32): cannot raise shared memory: %s", cudaGetErrorString(e));
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(T, nkv * groups, csize);
     cfg.blockDim = dim3(kThreads);

@@ -334,11 +334,10 @@ int launch(const void* qkv, void* out, const void* kcache, const void* vcache, c
            int max_q_len, int skip_single, attn::ScoreMod mod, cudaStream_t stream) {
     LI_REQUIRE(S <= 65535 && ceil_div(max_q_len > 0 ? max_q_len : 1, kTile) <= 65535, "attention (prefill): batch %d or portions of %d tokens too large for one launch", S, max_q_len);
     constexpr size_t smem = 2 * (size_t)(kKeys * DH * 2 + DH * kKeys * 2);
-    static bool raised = false;
-    if (!raised && smem > 48 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(prefill_attention_kernel<DH, kMod>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (smem > 48 * 1024) {
+        static LiOncePerDevice raised;
+        cudaError_t e = li_raise_shared(raised, (const void*)prefill_attention_kernel<DH, kMod>, smem);
         if (e != cudaSuccess) return li_fail("attention (prefill): cannot raise shared memory to %zu: %s", smem, cudaGetErrorString(e));
-        raised = true;
     }
     dim3 grid(nh, ceil_div(max_q_len > 0 ? max_q_len : 1, kTile), S);
     prefill_attention_kernel<DH, kMod><<<grid, kWarps * 32, smem, stream>>>((const bf16*)qkv, (bf16*)out, (const bf16*)kcache,

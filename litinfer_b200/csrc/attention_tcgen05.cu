@@ -587,12 +587,9 @@ int launch(const void* qkv, void* out, const void* kcache, const void* vcache, c
     if (int rc = make_map_ex(&map_k, kcache, (unsigned long long)num_pages * nkv * page_size, DH, 64, 16, 128)) return rc;
     if (int rc = make_map_ex(&map_v, vcache, (unsigned long long)num_pages * nkv * DH, (unsigned long long)page_size, 16, DH, 32)) return rc;
     const size_t smem = sizeof(Smem<DH>) + smem_pad<DH>();
-    static bool raised = false;
-    if (!raised) {
-        cudaError_t e = cudaFuncSetAttribute(prefill_attention_tc_kernel<DH, kForm>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return li_fail("attention (tcgen05): cannot raise shared memory to %zu: %s", smem, cudaGetErrorString(e));
-        raised = true;
-    }
+    static LiOncePerDevice raised;
+    cudaError_t e = li_raise_shared(raised, (const void*)prefill_attention_tc_kernel<DH, kForm>, smem);
+    if (e != cudaSuccess) return li_fail("attention (tcgen05): cannot raise shared memory to %zu: %s", smem, cudaGetErrorString(e));
     LI_REQUIRE(S <= 65535 && ceil_div(max_q_len, kRows) <= 65535, "attention (tcgen05): batch %d or portions of %d tokens too large for one launch", S, max_q_len);
     // With a work list the grid is (head, entry); a step with few tiles of tokens (a portion of a prompt behind a long
     // context) would leave multiprocessors idle while each CTA walks many key tiles, so its list shares the key tiles of

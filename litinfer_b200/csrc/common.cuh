@@ -10,6 +10,9 @@
 
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
+
+#include "device_once.h"
+
 #include <cstdarg>
 #include <cstdint>
 #include <cstdio>

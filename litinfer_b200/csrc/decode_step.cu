@@ -915,12 +915,9 @@ int launch(const LiDecodeStep& p, cudaStream_t stream) {
     const int row_stride = p.stage_k * 2 + kRowPad;
     const size_t smem = (size_t)kHeaderBytes + scratch + xbytes_for(p.M, p.x_cols) + (size_t)p.stages * 16 * row_stride;
     LI_REQUIRE(smem <= (size_t)kSmemBudget, "decode step: %zu bytes of shared memory do not fit (stage_k %d, %d stages)", smem, p.stage_k, p.stages);
-    static bool raised = false;
-    if (!raised) {
-        e = cudaFuncSetAttribute(decode_step_kernel<NT, DH>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBudget);
-        if (e != cudaSuccess) return li_fail("decode step: cannot raise shared memory: %s", cudaGetErrorString(e));
-        raised = true;
-    }
+    static LiOncePerDevice raised;
+    e = li_raise_shared(raised, (const void*)decode_step_kernel<NT, DH>, kSmemBudget);
+    if (e != cudaSuccess) return li_fail("decode step: cannot raise shared memory: %s", cudaGetErrorString(e));
     DeviceInfo& info = g_info[dev];
     if (info.sms == 0) {
         int sms = 0, coop = 0;

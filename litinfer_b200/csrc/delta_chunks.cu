@@ -480,9 +480,9 @@ delta_chunk_output_kernel(const float* __restrict__ prep_qk, const int4* __restr
 }
 
 template <typename K>
-int raise_smem(K kernel, size_t bytes, const char* what) {
+int raise_smem(LiOncePerDevice& once, K kernel, size_t bytes, const char* what) {
     if (bytes <= 48 * 1024) return 0;
-    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    const cudaError_t e = li_raise_shared(once, (const void*)kernel, bytes);
     return e == cudaSuccess ? 0 : li_fail("%s: cannot raise shared memory to %zu: %s", what, bytes, cudaGetErrorString(e));
 }
 
@@ -490,14 +490,11 @@ template <int DP>
 int launch(const float* prep_qk, const float* prep_g, const float* v, float* state, long long state_stride, const int* seg, int chunks, const int* runs,
            int nruns, float* wm, float* xm, float* pt, float* sums, float* s0, float* u, float* out, const void* gate, int dtype, int gate_ld, int gate_off,
            const float* norm_w, float eps, void* y, int heads, int kv_heads, int d, int dv, cudaStream_t stream) {
-    static bool raised = false;
-    if (!raised) {
-        if (int rc = raise_smem(delta_chunk_solve_kernel<DP>, solve_smem<DP>(), "delta chunks")) return rc;
-        if (int rc = raise_smem(delta_chunk_carry_kernel<DP>, carry_smem<DP>() > kMoreThanHalf ? carry_smem<DP>() : kMoreThanHalf, "delta chunks")) return rc;
-        if (int rc = raise_smem(delta_chunk_output_kernel<float, DP>, output_smem<DP>(), "delta chunks")) return rc;
-        if (int rc = raise_smem(delta_chunk_output_kernel<bf16, DP>, output_smem<DP>(), "delta chunks")) return rc;
-        raised = true;
-    }
+    static LiOncePerDevice raised[4];
+    if (int rc = raise_smem(raised[0], delta_chunk_solve_kernel<DP>, solve_smem<DP>(), "delta chunks")) return rc;
+    if (int rc = raise_smem(raised[1], delta_chunk_carry_kernel<DP>, carry_smem<DP>() > kMoreThanHalf ? carry_smem<DP>() : kMoreThanHalf, "delta chunks")) return rc;
+    if (int rc = raise_smem(raised[2], delta_chunk_output_kernel<float, DP>, output_smem<DP>(), "delta chunks")) return rc;
+    if (int rc = raise_smem(raised[3], delta_chunk_output_kernel<bf16, DP>, output_smem<DP>(), "delta chunks")) return rc;
     cudaError_t e = li_launch_pdl(delta_chunk_solve_kernel<DP>, dim3(heads, chunks), dim3(kThreads), solve_smem<DP>(), stream, prep_qk, prep_g, v, (const int4*)seg,
                                   wm, xm, pt, sums, heads, kv_heads, dv);
     if (e == cudaSuccess) {

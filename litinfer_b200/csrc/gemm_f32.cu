@@ -375,15 +375,6 @@ f32_tile_kernel(const float* __restrict__ A, const float* __restrict__ W, const 
     }
 }
 
-int sm_count() {
-    static const int sms = [] {
-        int dev = 0, n = 0;
-        if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) n = 148;
-        return n;
-    }();
-    return sms;
-}
-
 // Few rows: blocks of a cluster that share a tile's segments: 1, 2, 4 or 8 (clusters of three left multiprocessors idle: 3 rows,
 // N 1536, K 8960 25.4 us against 16.7 with two), whichever has the least of waves of blocks x (segments a block takes one
 // after the other + 1.5 for its start and its merge).
@@ -393,7 +384,7 @@ int stream_cluster(int tiles, int nseg, int slots) {
     for (int c = 1; c <= kMaxCluster && c <= nseg; c *= 2) {
         const int each = ceil_div(nseg, c);
         if (c > 1 && each > slots) continue;
-        const double cost = ceil_div(tiles * c, sm_count()) * (each + 1.5);
+        const double cost = ceil_div(tiles * c, li_multiprocessors()) * (each + 1.5);
         if (least == 0.0 || cost < least) least = cost, best = c;
     }
     return best;
@@ -403,7 +394,7 @@ int stream_cluster(int tiles, int nseg, int slots) {
 // of six, 318 with 32 rows a tile in clusters of two; N 1536, K 1536 59 us in clusters of three, 78 in clusters of two).
 int tile_cluster(long long tiles, int nseg) {
     int c = 1;
-    while (c < nseg && c < kMaxCluster && tiles * (c + 1) <= 2 * sm_count()) ++c;
+    while (c < nseg && c < kMaxCluster && tiles * (c + 1) <= 2 * li_multiprocessors()) ++c;
     return ceil_div(nseg, ceil_div(nseg, c));
 }
 
@@ -427,16 +418,13 @@ int launch_stream(const float* a, const float* w, const float* bias, float* out,
     CUtensorMap map_w, map_x;
     if (int rc = make_map_f32(encode, &map_w, w, N, K, kRows)) return rc;
     if (int rc = make_map_f32(encode, &map_x, a, M, K, StreamSmem<MT>::XR)) return rc;
-    const int tiles = ceil_div(N, kRows), nseg = ceil_div(K, kSegment), sms = sm_count();
+    const int tiles = ceil_div(N, kRows), nseg = ceil_div(K, kSegment), sms = li_multiprocessors();
     const int c = stream_cluster(tiles, nseg, StreamSmem<MT>::kSlots);
     const size_t smem = sizeof(StreamSmem<MT>) + 1024;
     static_assert(sizeof(StreamSmem<MT>) + 1024 <= 227 * 1024, "a block's shared memory");
-    static bool raised = false;
-    if (!raised) {
-        cudaError_t e = cudaFuncSetAttribute(f32_stream_kernel<MT, R, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return li_fail("linear (float32): cannot raise shared memory to %zu: %s", smem, cudaGetErrorString(e));
-        raised = true;
-    }
+    static LiOncePerDevice raised;
+    cudaError_t e = li_raise_shared(raised, (const void*)f32_stream_kernel<MT, R, T>, smem);
+    if (e != cudaSuccess) return li_fail("linear (float32): cannot raise shared memory to %zu: %s", smem, cudaGetErrorString(e));
     li_launch_pdl(f32_stream_kernel<MT, R, T>, dim3(c == 1 ? (tiles < sms ? tiles : sms) : tiles, c), dim3(kThreadsS), smem, stream, dim3(1, c, 1), map_w,
                   map_x, bias, out, M, N, K, tiles, c, err_dev);
     return li_check_launch("linear (float32, few rows)");
@@ -449,12 +437,9 @@ int launch_tile(const float* a, const float* w, const float* bias, float* out, i
     const int c = tile_cluster(tiles, ceil_div(K, kSegment));
     const size_t most = sizeof(TileSmem<TM>) + (TM - 1) * sizeof(float4) * kThreadsT;      // room for a cluster of two
     const size_t smem = sizeof(TileSmem<TM>) + (c > 1 ? (ceil_div(2 * TM, c) - 1) * sizeof(float4) * kThreadsT : 0);
-    static bool raised = false;
-    if (!raised) {
-        cudaError_t e = cudaFuncSetAttribute(f32_tile_kernel<TM, kVec>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
-        if (e != cudaSuccess) return li_fail("linear (float32): cannot raise shared memory to %zu: %s", most, cudaGetErrorString(e));
-        raised = true;
-    }
+    static LiOncePerDevice raised;
+    cudaError_t e = li_raise_shared(raised, (const void*)f32_tile_kernel<TM, kVec>, most);
+    if (e != cudaSuccess) return li_fail("linear (float32): cannot raise shared memory to %zu: %s", most, cudaGetErrorString(e));
     li_launch_pdl(f32_tile_kernel<TM, kVec>, dim3((unsigned)tiles, 1, c), dim3(kThreadsT), smem, stream, dim3(1, 1, c), a, w, bias, out, M, N, K);
     return li_check_launch("linear (float32)");
 }

@@ -476,12 +476,9 @@ int launch_tile(const void* a, const void* w, const float* bias, void* out, int 
     if (int rc = make_map(&map_a, a, M, K, BM)) return rc;
     if (int rc = make_map(&map_w, w, N * groups, K, Tile<BM, BN, kPair>::kRowsB)) return rc;       // (groups: their matrices one below the other)
     const size_t smem = sizeof(SharedStorage<BM, BN, kPair>) + 1024;
-    static bool raised = false;
-    if (!raised) {
-        cudaError_t e = cudaFuncSetAttribute(gemm_tcgen05_kernel<BM, BN, Tout, kSwiglu, kPair, kRope>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return li_fail("linear (tcgen05): cannot raise shared memory to %zu: %s", smem, cudaGetErrorString(e));
-        raised = true;
-    }
+    static LiOncePerDevice raised;
+    cudaError_t e = li_raise_shared(raised, (const void*)gemm_tcgen05_kernel<BM, BN, Tout, kSwiglu, kPair, kRope>, smem);
+    if (e != cudaSuccess) return li_fail("linear (tcgen05): cannot raise shared memory to %zu: %s", smem, cudaGetErrorString(e));
     dim3 grid(ceil_div(N, BN), ceil_div(M, BM), ksplit);
     if (kPair) {                                           // pairs along x; a tile of rows past the matrix reads zeros and stores nothing
         grid.x *= 2;

@@ -177,21 +177,11 @@ int launch(const void* a, const void* w, const float* bias, void* out, int M, in
     if (int rc = make_map(&map_a, a, M, K, kRows)) return rc;
     if (int rc = make_map(&map_w, w, G * N, K, BN / 2)) return rc;
     const size_t smem = sizeof(Smem) + 1024;
-    static bool raised = false;
-    if (!raised) {
-        cudaError_t e = cudaFuncSetAttribute(gemm_tcgen05_persistent_kernel<Tout, kSwiglu>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return li_fail("linear (tcgen05, persistent): cannot raise shared memory to %zu: %s", smem, cudaGetErrorString(e));
-        raised = true;
-    }
-    static int sms = 0;
-    if (!sms) {
-        int dev = 0;
-        cudaError_t e = cudaGetDevice(&dev);
-        if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        if (e != cudaSuccess || sms < 2) return li_fail("linear (tcgen05, persistent): cannot read the number of multiprocessors: %s", cudaGetErrorString(e));
-    }
+    static LiOncePerDevice raised;
+    cudaError_t e = li_raise_shared(raised, (const void*)gemm_tcgen05_persistent_kernel<Tout, kSwiglu>, smem);
+    if (e != cudaSuccess) return li_fail("linear (tcgen05, persistent): cannot raise shared memory to %zu: %s", smem, cudaGetErrorString(e));
     const int total = ((ceil_div(M, kRows) + 1) / 2) * ceil_div(N, BN);
-    int pairs = sms / 2;
+    int pairs = li_multiprocessors() / 2;
     if (pairs > total) pairs = total;
     li_launch_pdl(gemm_tcgen05_persistent_kernel<Tout, kSwiglu>, dim3(2 * pairs), dim3(kThreads), smem, stream, dim3(2, 1, 1), map_a, map_w, bias,
                   (Tout*)out, M, N, K, err_dev, tile_group);

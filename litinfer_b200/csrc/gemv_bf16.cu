@@ -276,12 +276,9 @@ int launch_kernel(const void* a, const void* w, const float* bias, void* out, in
     dim3 grid(ceil_div(N, 16), ksplit);
     constexpr size_t smem = (size_t)WARPS * NT * 128 * sizeof(float);
     if (smem > 48 * 1024) {
-        static bool raised = false;
-        if (!raised) {
-            cudaError_t e = cudaFuncSetAttribute(gemv_bf16_kernel<NT, WARPS, Tout, kSwiglu>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-            if (e != cudaSuccess) return li_fail("linear (gemv): cannot raise shared memory to %zu: %s", smem, cudaGetErrorString(e));
-            raised = true;
-        }
+        static LiOncePerDevice raised;
+        cudaError_t e = li_raise_shared(raised, (const void*)gemv_bf16_kernel<NT, WARPS, Tout, kSwiglu>, smem);
+        if (e != cudaSuccess) return li_fail("linear (gemv): cannot raise shared memory to %zu: %s", smem, cudaGetErrorString(e));
     }
     li_launch_pdl(gemv_bf16_kernel<NT, WARPS, Tout, kSwiglu>, grid, dim3(WARPS * 32), smem, stream, (const bf16*)a, (const bf16*)w, bias,
                   (Tout*)out, ws->partial, ws->counters, M, N, K, ksplit, rope, rs, add);

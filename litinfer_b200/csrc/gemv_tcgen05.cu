@@ -469,13 +469,11 @@ int clusters_at_once(int csize) {
 
 template <int BT, typename Tout, int kEpi, int kStages>
 int raise_shared() {
-    static bool raised = false;
-    if (raised) return 0;
+    static LiOncePerDevice raised[2];
     const size_t smem = sizeof(Smem<BT, kStages>) + 1024;
-    cudaError_t e = cudaFuncSetAttribute(gemv_tcgen05_kernel<BT, Tout, kEpi, false, kStages>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(gemv_tcgen05_kernel<BT, Tout, kEpi, true, kStages>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = li_raise_shared(raised[0], (const void*)gemv_tcgen05_kernel<BT, Tout, kEpi, false, kStages>, smem);
+    if (e == cudaSuccess) e = li_raise_shared(raised[1], (const void*)gemv_tcgen05_kernel<BT, Tout, kEpi, true, kStages>, smem);
     if (e != cudaSuccess) return li_fail("linear (tcgen05 gemv): cannot raise shared memory to %zu: %s", smem, cudaGetErrorString(e));
-    raised = true;
     return 0;
 }
 
