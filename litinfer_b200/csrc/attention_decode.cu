@@ -221,11 +221,18 @@ int launch(const void* qkv, void* out, const void* kcache, const void* vcache, c
                 cudaError_t e = li_raise_shared(raised, (const void*)decode_attention_whole_kernel<DH, W, KB, kMod, kColumns>, 200 * 1024);
                 if (e != cudaSuccess) return li_fail("attention (decode): cannot raise shared memory: %s", cudaGetErrorString(e));
             }
-            // Launched plainly: with CTAs that were there before the q|k|v product had finished a step of 64 sequences took longer
-            // (1.5B shape 2.78 against 2.53 ms, 61 sequences of the 7B shape 5.16 against 4.88 ms).
-            decode_attention_whole_kernel<DH, W, KB, kMod, kColumns><<<dim3(nkv, S), dim3(W * 32), wsmem, stream>>>(
-                (const bf16*)qkv, (const bf16*)kcache, (const bf16*)vcache, block_table, max_blocks, ctx_lens, q_start, (bf16*)out, nh, nkv, page_size,
-                num_pages, scale, window, mod);
+            // The column form is launched plainly: with CTAs that were there before the q|k|v product had finished a step of 64
+            // sequences took longer (1.5B shape 2.78 against 2.53 ms, 61 sequences of the 7B shape 5.16 against 4.88 ms).  The others gain by
+            // being there early, about 0.6 us a launch (80 sequences of 24 heads on 2, steps of six layers 620 -> 616 us; heads of
+            // 32, 150 sequences 490 -> 486 us).
+            if constexpr (kColumns)
+                decode_attention_whole_kernel<DH, W, KB, kMod, kColumns><<<dim3(nkv, S), dim3(W * 32), wsmem, stream>>>(
+                    (const bf16*)qkv, (const bf16*)kcache, (const bf16*)vcache, block_table, max_blocks, ctx_lens, q_start, (bf16*)out, nh, nkv, page_size,
+                    num_pages, scale, window, mod);
+            else
+                li_launch_pdl(decode_attention_whole_kernel<DH, W, KB, kMod, kColumns>, dim3(nkv, S), dim3(W * 32), wsmem, stream, (const bf16*)qkv,
+                              (const bf16*)kcache, (const bf16*)vcache, block_table, max_blocks, ctx_lens, q_start, (bf16*)out, nh, nkv, page_size, num_pages,
+                              scale, window, mod);
             return li_check_launch("attention (decode, whole context)");
         }
     }

@@ -6,6 +6,7 @@ a limit."""
 
 from __future__ import annotations
 
+import ctypes
 import re
 from pathlib import Path
 
@@ -66,3 +67,41 @@ def test_streaming_product_behind_attention_with_heads_of_64():
         assert torch.equal(att, alone)
         # float32 sums of 4,096 terms and one rounding to bfloat16
         assert bool(((y.float() - ref).abs() <= 2.0 ** -8 * ref.abs() + 1e-4).all())
+
+
+def dependent_launches(fn):
+    """Of the launches of a call: (all that have one before them, those that may begin while it still runs)."""
+    fn()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(graph):
+        fn()
+    runtime, handle, n = ctypes.CDLL("libcudart.so.12"), ctypes.c_void_p(graph.raw_cuda_graph()), ctypes.c_size_t()
+    assert runtime.cudaGraphGetEdges_v2(handle, None, None, None, ctypes.byref(n)) == 0
+    ends, data = [(ctypes.c_void_p * n.value)() for _ in range(2)], (ctypes.c_ubyte * (8 * n.value))()
+    assert runtime.cudaGraphGetEdges_v2(handle, ends[0], ends[1], data, ctypes.byref(n)) == 0
+    return n.value, sum(data[8 * i + 2] == 1 for i in range(n.value))          # the third byte: programmatic
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("heads,options,early", [((12, 2, 128), {}, False), ((16, 2, 64), {}, False), ((24, 2, 128), {}, True), ((14, 2, 80), {}, True),
+                                                 ((12, 2, 128), {"softcap": 20.0}, True)], ids=str)
+def test_whole_contexts_start_early_but_for_the_column_form(heads, options, early):
+    """Many sequences, a CTA a whole context: only the form that was measured to lose by it waits for its launch."""
+    from test_kernels_gpu import make_attention_case
+
+    from litinfer_b200 import kernels as K
+
+    nh, nkv, dh = heads
+    S, ctx = 80, 300
+    c = make_attention_case([1] * S, [ctx] * S, nh, nkv, dh, 16, torch.bfloat16, seed=2)
+    caches = [torch.randn((c["pages"], nkv, *shape), device="cuda").to(torch.bfloat16) for shape in ((16, dh), (dh, 16))]
+    ints = [torch.as_tensor(c[k], dtype=torch.int32).cuda() for k in ("bt", "q_start", "ctx_lens", "seq_of", "pos")]
+    qkv, out = c["qkv"].cuda(), torch.empty((S, nh * dh), dtype=torch.bfloat16, device="cuda")
+
+    def twice():
+        for _ in range(2):
+            K.paged_attention(qkv, out, *caches, *ints, nh, nkv, dh, dh ** -0.5, None, 1, ctx, **options)
+
+    assert dependent_launches(twice) == (1, 1 if early else 0)
+
