@@ -1533,15 +1533,16 @@ def argmax(logits: torch.Tensor, out: torch.Tensor) -> None:
     _check(library().li_argmax(_p(logits), _p(out), _i(R), _i(V), _stream(out)), "argmax")
 
 
-def sample(logits: torch.Tensor, params: torch.Tensor, out: torch.Tensor, small_top_k: bool = True) -> None:
+def sample(logits: torch.Tensor, params: torch.Tensor, out: torch.Tensor) -> None:
     """One token per row.  ``params`` int32 [R, 6]: temperature (float bits; <= 0
     is argmax), top_k, top_p (float bits), seed low, seed high, output index.
-    ``small_top_k=False``: no row has a top_k of 2 to 256, so the kernel for those need not be launched."""
+    Who packed them may leave ``params.small_top_k = False`` on the tensor: no row has a top_k of 2 to 256, so the kernel
+    for those need not be launched."""
     R, V = logits.shape
     _need(logits, "logits", torch.float32)
     _need(params, "sampling parameters", torch.int32, (R, 6))
     _need(out, "sample output", torch.int32, (R,))
-    _check(library().li_sample_rows(_p(logits), _p(params), _p(out), _i(R), _i(V), _i(1 if small_top_k else 0), _stream(out)), "sample")
+    _check(library().li_sample_rows(_p(logits), _p(params), _p(out), _i(R), _i(V), _i(1 if getattr(params, "small_top_k", True) else 0), _stream(out)), "sample")
 
 
 # --------------------------------------------------------------------------

@@ -96,7 +96,9 @@ class Sampler:
         packed[:, 3] = (seeds & np.uint64(0xFFFF_FFFF)).astype(np.uint32).view(np.int32)
         packed[:, 4] = (seeds >> np.uint64(32)).astype(np.uint32).view(np.int32)
         packed[:, 5] = [int(i) for i in output_index]
-        K.sample(logits, self._upload(packed), out, small_top_k=any(1 < p.top_k <= 256 for p in params))
+        rows = self._upload(packed)
+        rows.small_top_k = any(1 < p.top_k <= 256 for p in params)
+        K.sample(logits, rows, out)
         return out
 
 

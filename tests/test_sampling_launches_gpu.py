@@ -33,7 +33,8 @@ def test_no_kernel_for_options_that_a_call_does_not_have(option):
     assert kernels_of(lambda: K().sample(x, p, out)) == 2
     if not 1 < option[1] <= 256:
         told = torch.empty_like(out)
-        assert kernels_of(lambda: K().sample(x, p, told, small_top_k=False)) == 2
+        p.small_top_k = False
+        assert kernels_of(lambda: K().sample(x, p, told)) == 2
         assert told.tolist() == out.tolist()
 
 
@@ -41,7 +42,7 @@ def test_the_sampler_says_which_options_its_rows_have(monkeypatch):
     from litinfer_b200.sampling import sampler as S
 
     said, sample = [], S.K.sample
-    monkeypatch.setattr(S.K, "sample", lambda *a, **kw: (said.append(kw["small_top_k"]), sample(*a, **kw))[1])
+    monkeypatch.setattr(S.K, "sample", lambda x, rows, out: (said.append(rows.small_top_k), sample(x, rows, out))[1])
     x = torch.randn((3, 20000), device="cuda")
     for ks in ((0, 257, 1), (0, 50, 1), (2, 0, 0), (0, 0, 0)):
         S.Sampler("cuda:0").sample(x, [S.SamplingParams(0.8, k, 0.9, 7) for k in ks], [0, 1, 2])
