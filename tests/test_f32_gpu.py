@@ -157,3 +157,24 @@ def test_more_columns_than_a_grid_has_rows_of_blocks(rows):
         assert torch.equal(out[r], (w * a[r]).sum(1))
     assert torch.equal(out[rows - 1], (w * a[rows - 1]).sum(1))
 
+
+@pytest.mark.parametrize("width", [12 * 64, 12 * 64 + 4, 12 * 64 + 33, 1500])
+def test_attention_of_queries_in_rows_of_their_own(width):
+    """Rows of another length than q|k|v: queries alone, or beside something else, not on 16-byte boundaries."""
+    nh, nkv, dh, page = 12, 2, 64, 16
+    for q_lens, ctx_lens in (([1, 1], [1, 300]), ([40, 1, 20], [40, 333, 150])):
+        c = on_device(make_attention_case(q_lens, ctx_lens, nh, nkv, dh, page, torch.float32, seed=6))
+        T = c["qkv"].shape[0]
+        rows = torch.full((T, width), float("nan"), device="cuda")
+        rows[:, :nh * dh] = c["qkv"][:, :nh * dh]
+
+        def run(qkv, which):
+            out = torch.full((T, nh * dh), float("nan"), device="cuda")
+            K().paged_attention(qkv, out, c["k_cache"], c["v_cache"], c["block_table"], c["q_start"], c["ctx_lens"], c["seq_of_token"], c["positions"], nh, nkv, dh,
+                                dh ** -0.5, None, max(q_lens), max(ctx_lens), implementation=which)
+            return out
+
+        got = run(rows, "float32")
+        assert torch.equal(got, run(c["qkv"], "float32"))
+        assert float((got - run(rows, "general")).abs().max()) <= 2e-5
+

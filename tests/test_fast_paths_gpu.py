@@ -110,3 +110,35 @@ def test_splits_of_k_in_clusters_do_not_depend_on_the_batch(shape):
             if whole is not None:
                 assert torch.equal(out, whole[:m]), (tile, m)
             whole = out if whole is None else whole
+
+
+@pytest.mark.parametrize("heads", [(12, 2, 128), (24, 2, 64), (4, 1, 80)])
+@pytest.mark.parametrize("options", [{}, {"window": 40}, {"window": 40, "keep_first": 20}, {"window": 300, "sinks": True}, {"chunk": 128, "gate": True}], ids=str)
+def test_a_unit_that_is_its_sequences_only_one(heads, options):
+    """Contexts, or what a window or a chunk leaves of them, within 256 keys at an absolute place: nothing is merged over units; beside
+    them sequences of two units and more, in the same launch."""
+    from test_f32_gpu import on_device
+
+    nh, nkv, dh = heads
+    ctx_lens = [1, 255, 256, 257, 511, 513, 600, 700]        # alone without options: the first three; with a window of 40 all but 257, 513
+    c = on_device(T.make_attention_case([1] * 8, ctx_lens, nh, nkv, dh, 16, torch.float32, seed=12))
+    for k in ("qkv", "k_cache", "v_cache"):
+        c[k] = torch.nan_to_num(c[k]).to(torch.bfloat16)
+    kw = {k: v for k, v in options.items() if k in ("keep_first", "chunk")}
+    if "sinks" in options:
+        kw["sinks"] = torch.linspace(-1, 2, nh, device="cuda")
+    if "gate" in options:
+        kw["gate"] = torch.linspace(-3, 3, 8 * nh, device="cuda").view(8, nh).to(torch.bfloat16)
+
+    def run(dtype, which):
+        q, k, v = (c[x].to(dtype) for x in ("qkv", "k_cache", "v_cache"))
+        out = torch.full((8, nh * dh), float("nan"), dtype=dtype, device="cuda")
+        more = {n: x.to(dtype) if n == "gate" else x for n, x in kw.items()}
+        K().paged_attention(q, out, k, v, c["block_table"], c["q_start"], c["ctx_lens"], c["seq_of_token"], c["positions"], nh, nkv, dh, dh ** -0.5,
+                            options.get("window"), 1, max(ctx_lens), implementation=which, **more)
+        return out.float()
+
+    got, ref = run(torch.bfloat16, "decode"), run(torch.float32, "general")
+    # probabilities rounded to bfloat16 (2^-9 of each, values about 1) and the result once more
+    assert float((got - ref).abs().max()) <= 2.0 ** -8 * float(ref.abs().max()) + 2.0 ** -8
+

@@ -54,6 +54,23 @@ assert not failed, failed
 assert all(torch.equal(o, outs[0]) for o in outs)
 """
 
+FORM_CAPTURED = """
+import torch
+from litinfer_b200 import kernels as K
+g = torch.Generator(device="cuda").manual_seed(1)
+w = (torch.randn(1536, 8960, generator=g, device="cuda") * 8960 ** -0.5).to(torch.bfloat16)
+a = torch.randn(64, 8960, generator=g, device="cuda").to(torch.bfloat16)
+one, out = torch.zeros(1, 1536, device="cuda"), torch.zeros(64, 1536, device="cuda")
+K.linear(a[:1], w, None, one)
+torch.cuda.synchronize()
+graph = torch.cuda.CUDAGraph()
+with torch.cuda.graph(graph):
+    K.linear(a, w, None, out)
+graph.replay()
+torch.cuda.synchronize()
+assert float((out - a.float() @ w.float().T).abs().max()) < 1e-4
+"""
+
 
 def run(program):
     r = subprocess.run([sys.executable, "-c", program], cwd=ROOT, capture_output=True, text=True, timeout=240)
@@ -67,3 +84,9 @@ def test_float32_product_captured_before_any_other_call(rows):
 
 def test_float32_product_first_called_by_many_threads():
     run(THREADS)
+
+
+def test_another_form_of_the_streaming_product_first_called_inside_a_capture():
+    """Its workspace is there from a call with one token; its limits and its depth are asked for inside the capture."""
+    run(FORM_CAPTURED)
+
