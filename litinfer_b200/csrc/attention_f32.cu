@@ -13,7 +13,6 @@
 // Scores, exponentials (full precision), sums and weighted values are float.
 //
 // All of AttentionOptions but several maps a query row (attention.cu sends those to the general kernel).
-#define LI_PDL_KIND 4
 #include "attention_options.h"
 #include "common.cuh"
 

@@ -1,7 +1,7 @@
 // Causal grouped-query attention of a ragged batch over the paged cache:
-// the general kernel.  It serves the true 32-bit path for every batch shape
-// and is the fall-back of the bfloat16 path for head sizes the tensor-core
-// kernels refuse.
+// the general kernel, for what the others refuse: float32 with heads of more
+// than 128 elements, not of a multiple of 4, or with several maps a query row,
+// and head sizes that the tensor-core kernels do not take.
 //
 // One warp per (token, query head).  The token at position p of sequence s
 // reads keys lo..p of s with lo = max(0, p - window + 1) (window 0: lo = 0),

@@ -8,10 +8,10 @@
 // tensor memory) with 3 stages.  A multiprocessor takes in operand bytes from
 // L2 at a limited rate (about 55 GB/s measured here, 8 TB/s over the GPU); a
 // 128 x 128 tile needs 32 KB per 256 tensor-core cycles and is bound by that,
-// a 256 x 256 tile needs 64 KB per 1024 cycles.  The large tile is used where it
-// still fills the GPU (wide products: gate|up, lm_head of many rows; with a
-// split of k: down), the middle one for narrow products with a short k
-// (q|k|v, o).  Roles, by warp:
+// a 256 x 256 tile needs 64 KB per 1024 cycles.  Products of many tiles go to
+// gemm_tcgen05_persistent.cu; the large tile is used where it fills the GPU in
+// one wave or with a split of k, the middle one for narrow products with a short
+// k (q|k|v, o), pairs of CTAs in between.  Roles, by warp:
 //   warp 0   producer: one lane issues the TMA loads of a BM x 64 tile of a and
 //            a BN x 64 tile of w per k-block (64 bfloat16 = one 128-byte swizzle
 //            row) into a ring of stages, each guarded by a full/empty mbarrier pair;
@@ -495,7 +495,8 @@ int launch_tile(const void* a, const void* w, const float* bias, void* out, int 
     return li_check_launch("linear (tcgen05)");
 }
 
-// 256 x 256 tiles where they still fill most of the GPU (measured: better from about 120 CTAs on), else 128 x 128.
+// What the persistent kernel leaves: 256 x 256 tiles where they fill most of the GPU in one wave (120 to 148 of them with a very
+// long k) or with a split of k, pairs of CTAs on 256 columns, and smaller tiles below.
 // tile: 0 chooses, 1 forces the small tile, 2 the large one (for tests and measurements).
 template <typename Tout, int kSwiglu>
 int launch(const void* a, const void* w, const float* bias, void* out, int M, int N, int K, cudaStream_t stream, int tile) {
@@ -647,7 +648,7 @@ int li_linear_tcgen05_persistent(const void* a, const void* w, const float* bias
 
 int li_linear_tcgen05(const void* a, const void* w, const float* bias, void* out, int dtype_out, int M, int N, int K,
                       int epilogue, cudaStream_t stream) {
-    // wide products with a short k (gate|up): the persistent kernel, whose epilogue overlaps the next tile's products
+    // many tiles: the persistent kernel, whose epilogue overlaps the next tile's products
     if (g_forced_tile == 6 || (g_forced_tile == 0 && g_forced_ksplit == 0 && li_tcgen05_persistent_wanted(M, N, K)))
         return li_linear_tcgen05_persistent(a, w, bias, out, dtype_out, M, N, K, epilogue, stream);
     if (li_epilogue_is_gated(epilogue)) {

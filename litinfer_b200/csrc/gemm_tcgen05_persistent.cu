@@ -1,5 +1,5 @@
-// out[M, N] = a[M, K] w[N, K]^T for wide products with a short k (gate|up of a prefill step): a persistent form of the
-// tcgen05 GEMM in which the epilogue of one tile runs while the tensor cores work on the next.
+// out[M, N] = a[M, K] w[N, K]^T for products of many tiles (a prefill step's): a persistent form of the tcgen05 GEMM in
+// which the epilogue of one tile runs while the tensor cores work on the next.
 //
 // With k = 1536 a tile's main loop is only 24 k-blocks long; filling the pipeline and, above all, the epilogue (SwiGLU and
 // the stores of a 256 x 256 tile) then cost as much as the products, and a kernel that does one tile per CTA cannot

@@ -2,8 +2,9 @@
 //
 //   float32            -> CUDA-core kernels (gemm_f32.cu), always: a true 32-bit product
 //   bfloat16, M <= 64  -> decode is bound by reading every weight once: wide matrices go to
-//                         the tcgen05 kernel with swapped operands (gemv_tcgen05.cu), narrow
-//                         ones to the register-fed weight-streaming kernel (gemv_bf16.cu)
+//                         the tcgen05 kernel with swapped operands (gemv_tcgen05.cu), and so do
+//                         narrow ones with a long k or many tiles; the others to the
+//                         register-fed weight-streaming kernel (gemv_bf16.cu)
 //   bfloat16, larger M -> tcgen05 kernel with TMA-fed operands and the accumulator
 //                         in tensor memory (gemm_tcgen05.cu), when the sizes meet its
 //                         alignment rules (K a multiple of 8 elements = 16 bytes per row)
@@ -30,8 +31,9 @@ int li_gemv_tcgen05_tiles(int N);
 bool li_gemv_tcgen05_accepts(const void* a, const void* w, int M, int N, int K);
 
 // Whether a product of few rows goes to the tcgen05 kernel with swapped operands rather than to the register-fed one
-// (register-fed / tcgen05, us, 1 and 64 rows: 3584 x 3584 9.4 / 8.1 and 20.8 / 12.6; 4608 x 3584 10.3 / 9.6 and 21.4 / 13.8; but
-// 1536 x 3584 4.5 / 7.2 and 10.4 / 12.2, 1536 x 1536 2.9 / 6.2 and 5.8 / 10.6: few short tiles leave a split too little to do).
+// (register-fed / tcgen05, us, 8 and 64 rows: 3072 x 3072, the edge, 8.6 / 7.2 and 19.0 / 12.8; 3584 x 3584 9.4 / 8.1 and 20.8 /
+// 12.6; but 1536 x 3584 4.5 / 7.2 and 10.4 / 12.2, 1536 x 1536 2.9 / 6.2 and 5.8 / 10.6: few short tiles leave a split too little
+// to do).
 static bool few_rows_take_tcgen05(int N, int K) {
     const int tiles = (N + 127) / 128, nkb = (K + 63) / 64;
     if (tiles >= 96) return true;                              // fills the GPU without a split of k
@@ -43,9 +45,6 @@ namespace {
 
 // Which of the two kernels for few rows (decode) takes a bfloat16 product: 0 neither, 1 the register-fed one
 // (gemv_bf16.cu), 3 the tcgen05 kernel with swapped operands (gemv_tcgen05.cu); numbered as in li_linear_with.
-// Wide matrices (at least 96 tiles of 128 rows: gate|up, lm_head) and narrow ones with a long k (down) stream best
-// through TMA and the swapped tcgen05 kernel; narrow and short ones (q|k|v, o) would be cut into splits of two or
-// three k-blocks there, which the register-fed kernel does with less latency.
 int few_rows_kernel(const void* a, const void* w, const void* out, int M, int N, int K) {
     const bool aligned = ((uintptr_t)a % 16 == 0) && ((uintptr_t)w % 16 == 0) && ((uintptr_t)out % 16 == 0);
     if (!aligned || M > 64) return 0;
