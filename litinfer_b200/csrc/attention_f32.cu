@@ -136,7 +136,8 @@ attention_f32_kernel(const float* __restrict__ qkv, float* __restrict__ out, con
                 if (opt.slopes && h < heads) v -= opt.slopes[h0 + h] * (float)(p - key);
                 v = seen ? v : -INFINITY;
                 m[h] = warp_max(v);
-                const float e = seen ? expf(v - m[h]) : 0.0f;
+                // (a score of minus infinity has no weight, also where the unit has no other; NaN stays NaN)
+                const float e = seen && v != -INFINITY ? expf(v - m[h]) : 0.0f;
                 l[h] = warp_sum(e);
                 p_sm[h * kUnit + lane] = e;
             }
@@ -240,7 +241,8 @@ attention_f32_kernel(const float* __restrict__ qkv, float* __restrict__ out, con
             L[j] = L[j] * fo + expf(sk - mn);
             O[j] *= fo;
         }
-        float inv = L[j] > 0.0f ? 1.0f / L[j] : 0.0f;
+        // (keys, but no score above minus infinity: undefined)
+        float inv = L[j] > 0.0f ? 1.0f / L[j] : Mx[j] == -INFINITY && p >= 0 && !opt.sinks ? NAN : 0.0f;
         if (gate && !opt.gate_elements) inv *= 1.0f / (1.0f + expf(-gate[h]));
         if (d < dh) {
             float r = O[j] * inv;

@@ -178,3 +178,26 @@ def test_attention_of_queries_in_rows_of_their_own(width):
         assert torch.equal(got, run(c["qkv"], "float32"))
         assert float((got - run(rows, "general")).abs().max()) <= 2e-5
 
+
+
+@pytest.mark.parametrize("tokens", [1, 40])
+@pytest.mark.parametrize("lost", [(64, 65), (32, 64), (0, 40), (0, 65)])
+def test_scores_of_minus_infinity(lost, tokens):
+    """Keys whose scores are minus infinity have no weight, also where a unit of 32 keys has no others; a token that sees nothing
+    else has no softmax (the same tokens of one block and of a cluster of them)."""
+    nh, nkv, dh, page, ctx = 6, 2, 64, 16, 65
+    c = make_attention_case([tokens], [ctx], nh, nkv, dh, page, torch.float32, seed=14)
+    c["qkv"].view(tokens, -1, dh)[:, :nh, 0].abs_().add_(0.1)
+    keys, vals = c["keys"][0], c["vals"][0]
+    keys[lost[0]:lost[1], :, 0] = float("-inf")
+    q = c["qkv"][:, :nh * dh].view(tokens, nh, dh).double()
+    scores = torch.einsum("thd,khd->thk", q, keys.double().repeat_interleave(nh // nkv, 1)) * dh ** -0.5
+    unseen = torch.arange(ctx)[None, :] > torch.arange(ctx - tokens, ctx)[:, None]
+    exact = torch.einsum("thk,khd->thd", scores.masked_fill(unseen[:, None], float("-inf")).softmax(-1), vals.double().repeat_interleave(nh // nkv, 1))
+    d = on_device(c)
+    out = torch.empty((tokens, nh * dh), device="cuda")
+    K().paged_attention(d["qkv"], out, d["k_cache"], d["v_cache"], d["block_table"], d["q_start"], d["ctx_lens"], d["seq_of_token"], d["positions"], nh, nkv, dh,
+                        dh ** -0.5, None, tokens, ctx, implementation="float32")
+    got = out.double().cpu().view(tokens, nh, dh)
+    assert torch.equal(got.isnan(), exact.isnan())
+    assert float((got - exact).nan_to_num().abs().max()) <= 2e-5
