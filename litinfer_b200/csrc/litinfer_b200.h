@@ -446,8 +446,9 @@ int li_argmax(const float* logits, int* out, int R, int V, cudaStream_t stream);
  * max with a counter-based generator, independent of the batch. */
 int li_sample(const float* logits, const int* params, int* out, int R, int V, cudaStream_t stream);
 
-/* The same; small_top_k 0 says that no row has a top_k of 2 to 256. */
-int li_sample_rows(const float* logits, const int* params, int* out, int R, int V, int small_top_k, cudaStream_t stream);
+/* The same; bit 0 of `rows` clear says that no row has a top_k of 2 to 256, bit 1 set that none has temperature as its only
+   option. */
+int li_sample_rows(const float* logits, const int* params, int* out, int R, int V, int rows, cudaStream_t stream);
 
 /* Tests: 1 leaves -1 in the rows that the pass for a small top_k does not settle by itself (0: they are drawn another way). */
 void li_sample_leave_rows(int on);

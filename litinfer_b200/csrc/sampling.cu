@@ -697,8 +697,11 @@ LI_EXPORT int li_argmax(const float* logits, int* out, int R, int V, cudaStream_
     return li_check_launch("argmax");
 }
 
-// small_top_k: whether some row may have a top_k of 2 to 256 (else its kernel is not launched).
-LI_EXPORT int li_sample_rows(const float* logits, const int* params, int* out, int R, int V, int small_top_k, cudaStream_t stream) {
+// rows, what the caller knows of them: bit 0 whether some row may have a top_k of 2 to 256 (else its kernel is not launched), bit 1
+// that none has temperature as its only option (else a row of a large vocabulary is drawn by a kernel of its own, 5 us that
+// the launch costs where there is no such row).
+LI_EXPORT int li_sample_rows(const float* logits, const int* params, int* out, int R, int V, int rows, cudaStream_t stream) {
+    const bool small_top_k = rows & 1, none_alone = rows & 2;
     LI_REQUIRE(R >= 0 && V > 0, "sample: bad sizes R=%d V=%d", R, V);
     LI_REQUIRE(V < (1 << 24), "sample: vocabulary %d is too large", V);
     if (R == 0) return 0;
@@ -716,7 +719,7 @@ LI_EXPORT int li_sample_rows(const float* logits, const int* params, int* out, i
         li_launch_pdl(sample_kernel, dim3(R), dim3(kThreads), 0, stream, logits, params, out, V, chunked_plain);
     }
     if (int rc = li_check_launch("sample")) return rc;
-    if (chunked_plain) {
+    if (chunked_plain && !none_alone) {
         li_launch_pdl(sample_temperature_chunks_kernel, dim3(kDrawChunks, R), dim3(256), 0, stream, logits, params, out, V);
         return li_check_launch("sample (temperature, chunks)");
     }

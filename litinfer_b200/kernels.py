@@ -1537,12 +1537,14 @@ def sample(logits: torch.Tensor, params: torch.Tensor, out: torch.Tensor) -> Non
     """One token per row.  ``params`` int32 [R, 6]: temperature (float bits; <= 0
     is argmax), top_k, top_p (float bits), seed low, seed high, output index.
     Who packed them may leave ``params.small_top_k = False`` on the tensor: no row has a top_k of 2 to 256, so the kernel
-    for those need not be launched."""
+    for those need not be launched; and ``params.draws_alone = False``: no row has temperature as its only option, so the
+    kernel that draws those over many CTAs need not be either."""
     R, V = logits.shape
     _need(logits, "logits", torch.float32)
     _need(params, "sampling parameters", torch.int32, (R, 6))
     _need(out, "sample output", torch.int32, (R,))
-    _check(library().li_sample_rows(_p(logits), _p(params), _p(out), _i(R), _i(V), _i(1 if getattr(params, "small_top_k", True) else 0), _stream(out)), "sample")
+    rows = (1 if getattr(params, "small_top_k", True) else 0) | (0 if getattr(params, "draws_alone", True) else 2)
+    _check(library().li_sample_rows(_p(logits), _p(params), _p(out), _i(R), _i(V), _i(rows), _stream(out)), "sample")
 
 
 # --------------------------------------------------------------------------

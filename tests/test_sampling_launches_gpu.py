@@ -49,6 +49,23 @@ def test_the_sampler_says_which_options_its_rows_have(monkeypatch):
     assert said == [False, True, True, False]
 
 
+def test_the_sampler_says_whether_a_row_is_drawn_by_temperature_alone(monkeypatch):
+    from litinfer_b200.sampling import sampler as S
+
+    x = torch.randn((2, 20000), device="cuda")
+    said, sample = [], S.K.sample
+    monkeypatch.setattr(S.K, "sample", lambda x, rows, out: (said.append(rows), sample(x, rows, out))[1])
+    for k, p in ((0, 0.9), (50, 1.0), (0, 1.0), (19999, 1.0)):
+        both = [S.SamplingParams(0.8, k, p, 7), S.SamplingParams(0.8, 30, 0.9, 8)]
+        got = S.Sampler("cuda:0").sample(x, both, [0, 1])
+        rows, all_kernels = said[-1].clone(), torch.empty_like(got)
+        sample(x, rows, all_kernels)
+        assert got.tolist() == all_kernels.tolist()
+        rows.draws_alone = said[-1].draws_alone
+        assert kernels_of(lambda: sample(x, rows, all_kernels)) == (2 if rows.draws_alone else 1)
+    assert [r.draws_alone for r in said] == [False, False, True, True]
+
+
 @pytest.mark.parametrize("V", [16384, 16387, 32000, 151936])
 @pytest.mark.parametrize("R", [1, 15, 16, 32, 33, 64])
 def test_ordinary_rows_are_settled_in_one_pass(R, V):
