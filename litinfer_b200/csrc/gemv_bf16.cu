@@ -142,6 +142,8 @@ gemv_bf16_kernel(const bf16* __restrict__ X, const bf16* __restrict__ W, const f
         }
     };
     if (kFactorsFirst && pre_fits) finish_factors();
+    [[maybe_unused]] RopeAhead ahead;
+    if constexpr (kEpi == kEpiRope) ahead = rope_ask<NT>((int)threadIdx.x, bias, tile, M, rope);
     constexpr int kXPre = kEpi == kEpiAddScaled ? (NT * 128 + WARPS * 32 - 1) / (WARPS * 32) : 1;
     float xpre[kXPre];
     if constexpr (kEpi == kEpiAddScaled) {
@@ -195,7 +197,7 @@ gemv_bf16_kernel(const bf16* __restrict__ X, const bf16* __restrict__ W, const f
         return v;
     };
     if (kEpi == kEpiRope) {
-        store_rope<NT>(warps_sum, bias, reinterpret_cast<bf16*>(out), tile, M, N, rope, (int)threadIdx.x, WARPS * 32, factors);       // never split along k
+        store_rope<NT>(warps_sum, bias, reinterpret_cast<bf16*>(out), tile, M, N, rope, (int)threadIdx.x, WARPS * 32, factors, &ahead);       // never split along k
         return;
     }
     auto finish = [&](auto get) {

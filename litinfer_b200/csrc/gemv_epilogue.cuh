@@ -24,9 +24,30 @@ struct RopeArgs {
     int extra = 0;
 };
 
+// What the epilogue needs from memory for one element: a thread's first one is asked for ahead of the weights, since the load and the
+// sine that hangs on it would follow the last of them otherwise.
+struct RopeAhead {
+    float position = 0.0f, denom = 1.0f, b0 = 0.0f, b1 = 0.0f;
+    int slot = -1;
+};
+
+template <int NT>
+__device__ __forceinline__ RopeAhead rope_ask(int q, const float* __restrict__ bias, int tile, int M, const RopeArgs& ra) {
+    RopeAhead a;
+    const int tiles_per_head = ra.dh >> 4, half = ra.dh >> 1;
+    const int head = tile / tiles_per_head, jt = tile - head * tiles_per_head;
+    const int l = q & 31, tok = (q >> 6) * 8 + ((l & 3) << 1) + ((q >> 5) & 1);
+    if (q >= NT * 64 || tok >= M) return a;
+    const int jj = jt * 8 + (l >> 2), r0 = head * ra.dh + jj;
+    if (bias) a.b0 = bias[r0], a.b1 = bias[r0 + half];
+    if (ra.write && head >= ra.nh && head < ra.nh + 2 * ra.nkv) a.slot = ra.slot_mapping[tok];
+    if (ra.denom != nullptr && head < ra.nh + ra.nkv) a.position = (float)ra.positions[tok], a.denom = ra.denom[jj];
+    return a;
+}
+
 template <int NT, typename Get>
 __device__ __forceinline__ void store_rope(Get get, const float* __restrict__ bias, bf16* __restrict__ out, int tile, int M, int N,
-                                           const RopeArgs& ra, int tid, int nthreads, const float* rs_sm) {
+                                           const RopeArgs& ra, int tid, int nthreads, const float* rs_sm, const RopeAhead* ahead = nullptr) {
     const int tiles_per_head = ra.dh >> 4, half = ra.dh >> 1;
     const int head = tile / tiles_per_head, jt = tile - head * tiles_per_head;
     for (int q = tid; q < NT * 64; q += nthreads) {
@@ -41,14 +62,15 @@ __device__ __forceinline__ void store_rope(Get get, const float* __restrict__ bi
             x0 *= rs_sm[tok];
             x1 *= rs_sm[tok];
         }
+        const RopeAhead a = ahead && q == tid ? *ahead : rope_ask<NT>(q, bias, tile, M, ra);
         if (bias) {
-            x0 += bias[r0];
-            x1 += bias[r1];
+            x0 += a.b0;
+            x1 += a.b1;
         }
         float y0 = x0, y1 = x1;
         if (ra.denom != nullptr && head < ra.nh + ra.nkv) {          // (no denominators: no rotation)
             float sn, cs;
-            sincosf((float)ra.positions[tok] / ra.denom[jj], &sn, &cs);
+            sincosf(a.position / a.denom, &sn, &cs);
             // q and k are rounded to bfloat16 by the projection before they are rotated, as in the unfused path
             x0 = __bfloat162float(__float2bfloat16_rn(x0));
             x1 = __bfloat162float(__float2bfloat16_rn(x1));
@@ -64,7 +86,7 @@ __device__ __forceinline__ void store_rope(Get get, const float* __restrict__ bi
             out[tok * ld + r0] = __float2bfloat16_rn(y0);
             out[tok * ld + r1] = __float2bfloat16_rn(y1);
         } else if (ra.write) {
-            const int slot = ra.slot_mapping[tok];
+            const int slot = a.slot;
             const int page = slot / ra.page_size, off = slot - page * ra.page_size;
             if (slot < 0 || page >= ra.num_pages) continue;        // validated on the host; never write outside the cache
             if (head < ra.nh + ra.nkv) {

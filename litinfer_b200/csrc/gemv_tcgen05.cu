@@ -10,16 +10,13 @@
 // tensor-memory allocation and MMA issue, warps 2-5: epilogue.  The weight tiles of
 // the first stages are requested before griddepcontrol.wait (weights do not depend
 // on the kernel before), the activation tiles after it.  With several splits the
-// CTAs of a tile form clusters of up to eight: each leaves its float partial tile
-// in its shared memory, and CTA r of a cluster takes the tokens r, r + size, ...,
+// CTAs of a tile form a cluster of up to eight: each leaves its float partial tile
+// in its shared memory, and CTA r of the cluster takes the tokens r, r + size, ...,
 // adds their sums in split order through distributed shared memory and does their
-// epilogue.  More than eight splits (up to 16 tokens): clusters of four, whose sums
-// meet in a workspace where the last one to arrive (a counter per tile and place in
-// the cluster) adds them in order.  The splits are a function of N, K and the token
-// tile (up to 16, 32 or 64 tokens): within a tile a token's result does not depend
-// on how many others there are; from one tile to the next the order of its sums may
-// change.  (One CTA that read every split's partial tile from the workspace took
-// several round trips for itself: 64 tokens, eight splits, 262 KB.)
+// epilogue.  What that costs is the trips through the cluster: sixteen loads are in
+// flight at a time (64 tokens, N 1536, K 8960, eight splits: a load after the other
+// 15.6 us, so 11.7; N 2048, K 1536 10.4 and 6.8).  The splits are a function of N
+// and K: a token's result does not depend on how many others there are.
 // Epilogue: bias, or the SwiGLU of gate and up rows interleaved in groups of 8
 // (up * gate / (1 + exp(-gate)), src/ops/swiglu/op.cpp:17-23).
 //
@@ -38,8 +35,7 @@ using namespace tc;
 constexpr int BR = 128;                  // weight rows per CTA
 constexpr int kThreads = 192;
 constexpr int kTargetCtas = 148;
-constexpr size_t kWorkspaceFloats = 4u << 20;
-constexpr int kMaxTiles = 1 << 16;
+constexpr int kMaxCluster = 8;
 
 // Stages: six (deep), or as many as two CTAs a multiprocessor leave room for.  Two are better where the CTAs come in several waves,
 // since the next tile streams in while the other's epilogue runs (64 tokens, N 37888, K 3584: 61 -> 49 us).  Where every CTA of
@@ -56,16 +52,9 @@ struct __align__(1024) Smem {
     unsigned long long empty[kStages];
     unsigned long long accum;
     unsigned tmem_base;
-    int is_last;
     float factor[64];                // per token: the reciprocal root of the norm before this product
     float squares[4][64];            // per epilogue warp and token: sums of squares of the new residual values
 };
-
-struct Workspace {
-    float* partial = nullptr;
-    unsigned* counters = nullptr;
-};
-Workspace g_ws[16];
 
 template <int N>
 __device__ __forceinline__ void tmem_ld(unsigned taddr, float (&v)[N]);
@@ -116,7 +105,7 @@ __device__ __forceinline__ float peer_load(unsigned addr) {
 
 enum { kEpiNone = 0, kEpiSwiglu = 1, kEpiAddScaled = 2, kEpiGluClamped = 3, kEpiGeglu = 4, kEpiRope = 5 };     // (3 and 4: SwiGLU's layout, another activation)
 
-// kSplit: k is split over the CTAs of clusters of `csize` (the grid's y: splits, a cluster's consecutive).
+// kSplit: k is split over the `csize` CTAs of a cluster (the grid's y).
 // The sum into the residual stream is held to two CTAs a multiprocessor: without the bound its 33 to 64 tokens took 255
 // registers, one CTA a multiprocessor, and clusters of five, six and eight, of which the GPU then holds 26, 22 and 15, no longer
 // ran all at once (64 tokens, N 3584, K 8960, 28 clusters of five: 40.5 us, with the bound 22.3; N 2048, K 8960 35.9 and 20.1).
@@ -124,8 +113,7 @@ enum { kEpiNone = 0, kEpiSwiglu = 1, kEpiAddScaled = 2, kEpiGluClamped = 3, kEpi
 template <int BT, typename Tout, int kEpi, bool kSplit, int kStages>
 __global__ void __launch_bounds__(kThreads, kEpi == kEpiAddScaled && BT >= 32 ? 2 : 0)
 gemv_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
-                    const float* __restrict__ bias, Tout* __restrict__ out, float* __restrict__ partial,
-                    unsigned* __restrict__ counters, int M, int N, int K, int ksplit, int csize, int* __restrict__ error_flag, const RowScale rs,
+                    const float* __restrict__ bias, Tout* __restrict__ out, int M, int N, int K, int csize, int* __restrict__ error_flag, const RowScale rs,
                     const AddScaled add, const RopeArgs rope) {
     constexpr int kSwiglu = kEpi == kEpiSwiglu ? LI_EPILOGUE_SWIGLU : kEpi == kEpiGluClamped ? LI_EPILOGUE_GLU_CLAMPED : kEpi == kEpiGeglu ? LI_EPILOGUE_GEGLU : 0;
     constexpr bool kAdd = kEpi == kEpiAddScaled;
@@ -135,7 +123,7 @@ gemv_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
     const int tile = blockIdx.x, split = blockIdx.y;
     const int n0 = tile * BR;
     const int nkb_total = (K + BK - 1) / BK;
-    const int kb0 = (int)((long long)split * nkb_total / ksplit), kb1 = (int)((long long)(split + 1) * nkb_total / ksplit);
+    const int kb0 = (int)((long long)split * nkb_total / csize), kb1 = (int)((long long)(split + 1) * nkb_total / csize);
     const int nkb = kb1 - kb0;
     constexpr unsigned kStageBytes = BR * BK * 2 + BT * BK * 2;
     constexpr unsigned kCols = BT < 32 ? 32 : BT;
@@ -221,7 +209,7 @@ gemv_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
             asm volatile("bar.sync 1, 128;" ::: "memory");
         }
         // the tokens this CTA finishes: all of them, or every csize-th of a cluster's
-        const int rank = kSplit ? split % csize : 0, step = kSplit ? csize : 1;
+        const int rank = kSplit ? split : 0, step = kSplit ? csize : 1;
         float xold[kAdd ? kMine : 1];
         auto load_old = [&]() {
             if constexpr (kAdd) {
@@ -232,6 +220,22 @@ gemv_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
                 }
             }
         };
+        // The rotation's angles and the tokens' places in the cache, of this CTA's tokens: worked out while the weights stream.  (In
+        // the epilogue itself, a token after the other, each of them a load and a sine: 61 tokens, N 4608, K 3584 22.2 us.)
+        float2* rot = reinterpret_cast<float2*>(&sm + 1);
+        const int tokens_here = rank < M ? (M - rank + step - 1) / step : 0;
+        int* place = reinterpret_cast<int*>(rot + tokens_here * (BR / 2));
+        if constexpr (kEpi == kEpiRope) {
+            const int t = (int)threadIdx.x - 64;
+            if (rope.denom != nullptr && tile < rope.nh + rope.nkv)
+                for (int e = t; e < tokens_here * (BR / 2); e += 128) {
+                    float sn, cs;
+                    sincosf((float)rope.positions[rank + e / (BR / 2) * step] / rope.denom[e % (BR / 2)], &sn, &cs);
+                    rot[e] = make_float2(cs, sn);
+                }
+            if (rope.write)
+                for (int e = t; e < tokens_here; e += 128) place[e] = rope.slot_mapping[rank + e * step];
+        }
         // (32 tokens with a split: asked for when the partial tile has left its registers, else some of them spill)
         if constexpr (!kSplit || BT != 32) load_old();
         const bool ok = mbar_wait(&sm.accum, 0);
@@ -239,7 +243,7 @@ gemv_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         float v[BT];
         tmem_ld<BT>(tmem_acc + ((unsigned)(quarter * 32) << 16), v);
-        bool write = ok;
+        const bool write = ok;
         if constexpr (kSplit) {
             // (every load into the stages has been multiplied: their room holds the partial tile [token][row] now)
             float* mine = reinterpret_cast<float*>(sm.w[0]) + r_in_tile;
@@ -248,48 +252,32 @@ gemv_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
                 if (j < M) mine[j * BR] = v[j];
             if constexpr (BT == 32) load_old();
             cluster_arrive_wait();
-            float t[kMine];
+            // sixteen loads in flight, of four tokens and four CTAs: without branches around them (tokens that are not there read
+            // the last one's place), since a load that waits for the one before costs a trip through the cluster each
+            constexpr int kTok = 4, kPeers = 4;
+            const unsigned own = smem_u32(mine);
 #pragma unroll
-            for (int i = 0; i < kMine; ++i) t[i] = 0.0f;
-            for (int r = 0; r < csize; ++r) {
-                const unsigned src = peer_address(smem_u32(mine), (unsigned)r);
+            for (int i0 = 0; i0 < kMine; i0 += kTok) {
+                float t[kTok] = {};
+                if (rank + i0 * step < M) {
+#pragma unroll 1
+                    for (int r0 = 0; r0 < csize; r0 += kPeers) {
+                        float x[kPeers][kTok];
 #pragma unroll
-                for (int i = 0; i < kMine; ++i) {
-                    const int j = rank + i * step;
-                    if (j < M) t[i] += peer_load(src + (unsigned)j * (BR * 4));
-                }
-            }
+                        for (int q = 0; q < kPeers; ++q) {
+                            const unsigned src = peer_address(own, (unsigned)min(r0 + q, csize - 1));
 #pragma unroll
-            for (int i = 0; i < kMine; ++i) v[i] = t[i];
-            const int groups = ksplit / csize;
-            if (groups > 1) {
-                const int group = split / csize;
-                const size_t tiles = gridDim.x;
-                float* to = partial + (((size_t)group * tiles + tile) * BT) * BR + r_in_tile;
+                            for (int i = 0; i < kTok; ++i) x[q][i] = peer_load(src + (unsigned)min(rank + (i0 + i) * step, M - 1) * (BR * 4));
+                        }
 #pragma unroll
-                for (int i = 0; i < kMine; ++i)
-                    if (rank + i * step < M) to[(size_t)(rank + i * step) * BR] = v[i];
-                __threadfence();
-                asm volatile("bar.sync 1, 128;" ::: "memory");
-                if (warp == 2 && lane == 0) {
-                    const unsigned prev = atomicAdd(&counters[tile * csize + rank], 1u);
-                    sm.is_last = (prev == (unsigned)(groups - 1));
-                }
-                asm volatile("bar.sync 1, 128;" ::: "memory");
-                write = write && sm.is_last != 0;
-                if (sm.is_last != 0) {
-                    __threadfence();
+                        for (int q = 0; q < kPeers; ++q)
 #pragma unroll
-                    for (int i = 0; i < kMine; ++i) v[i] = 0.0f;
-                    for (int g = 0; g < groups; ++g) {
-                        const float* src = partial + (((size_t)g * tiles + tile) * BT) * BR + r_in_tile;
-#pragma unroll
-                        for (int i = 0; i < kMine; ++i)
-                            if (rank + i * step < M) v[i] += __ldcg(src + (size_t)(rank + i * step) * BR);
+                            for (int i = 0; i < kTok; ++i)
+                                if (r0 + q < csize) t[i] += x[q][i];
                     }
-                    asm volatile("bar.sync 1, 128;" ::: "memory");
-                    if (warp == 2 && lane == 0) counters[tile * csize + rank] = 0;          // ready for the next launch on this stream
                 }
+#pragma unroll
+                for (int i = 0; i < kTok; ++i) v[i0 + i] = t[i];
             }
         }
         if (write && rs.ssq) {
@@ -302,17 +290,28 @@ gemv_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
                 // into the residual stream, and on to the next product as bfloat16(norm_weight * x) with the sums of x^2
                 const float b = (bias && row < N) ? bias[row] : 0.0f;
                 const float nw = row < N ? add.norm_weight[row] : 0.0f;
+                constexpr int kTok = 4;                                    // tokens whose squares are added up side by side
 #pragma unroll
-                for (int i = 0; i < kMine; ++i) {
-                    const int j = rank + i * step;
-                    if (j < M) {                                           // uniform
-                        const float x = row < N ? xold[i] + (v[i] + b) : 0.0f;
-                        if (row < N) {
-                            __stcg(add.x32 + (size_t)j * N + row, x);
-                            add.hprime[(size_t)j * N + row] = __float2bfloat16_rn(nw * x);
+                for (int i0 = 0; i0 < kMine; i0 += kTok) {
+                    if (rank + i0 * step < M) {                            // uniform
+                        float sq[kTok];
+#pragma unroll
+                        for (int i = 0; i < kTok; ++i) {
+                            const int j = rank + (i0 + i) * step;
+                            const float x = j < M && row < N ? xold[i0 + i] + (v[i0 + i] + b) : 0.0f;
+                            if (j < M && row < N) {
+                                __stcg(add.x32 + (size_t)j * N + row, x);
+                                add.hprime[(size_t)j * N + row] = __float2bfloat16_rn(nw * x);
+                            }
+                            sq[i] = x * x;
                         }
-                        const float sq = warp_sum(x * x);
-                        if (lane == 0) sm.squares[quarter][j] = sq;
+#pragma unroll
+                        for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+                            for (int i = 0; i < kTok; ++i) sq[i] += __shfl_xor_sync(0xffffffffu, sq[i], o);
+#pragma unroll
+                        for (int i = 0; i < kTok; ++i)
+                            if (lane == 0 && rank + (i0 + i) * step < M) sm.squares[quarter][rank + (i0 + i) * step] = sq[i];
                     }
                 }
                 asm volatile("bar.sync 1, 128;" ::: "memory");
@@ -331,18 +330,15 @@ gemv_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
                     both[i * BR] = rotate ? __bfloat162float(__float2bfloat16_rn(v[i])) : v[i];
                 }
                 asm volatile("bar.sync 1, 128;" ::: "memory");
-                const float den = rotate ? rope.denom[d & 63] : 1.0f;
                 const size_t ld = (size_t)(rope.nh + 2 * rope.nkv) * BR;
-#pragma unroll 1
-                for (int i = 0; i < kMine; ++i) {
+#pragma unroll 4
+                for (int i = 0; i < tokens_here; ++i) {
                     const int j = rank + i * step;
-                    if (j >= M) break;
                     float y = both[i * BR];
                     if (rotate) {
-                        float sn, cs;
-                        sincosf((float)rope.positions[j] / den, &sn, &cs);
+                        const float2 cs = rot[i * (BR / 2) + (d & 63)];
                         const float other = d < 64 ? both[i * BR + 64] : both[i * BR - 64];
-                        y = d < 64 ? y * cs - other * sn : y * cs + other * sn;
+                        y = d < 64 ? y * cs.x - other * cs.y : y * cs.x + other * cs.y;
                     }
                     const bf16 r = __float2bfloat16_rn(y);
                     if (head >= rope.nh + 2 * rope.nkv) {
@@ -350,7 +346,7 @@ gemv_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
                     } else if (head < rope.nh) {
                         reinterpret_cast<bf16*>(out)[j * ld + (size_t)head * BR + d] = r;
                     } else if (rope.write) {
-                        const int slot = rope.slot_mapping[j];
+                        const int slot = place[i];
                         const int page = slot / rope.page_size, off = slot - page * rope.page_size;
                         if (slot < 0 || page >= rope.num_pages) continue;      // validated on the host; never write outside the cache
                         if (head < rope.nh + rope.nkv)
@@ -396,47 +392,25 @@ gemv_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
     }
 }
 
-int ensure_workspace(Workspace** ws) {
-    int dev = 0;
-    cudaError_t e = cudaGetDevice(&dev);
-    if (e != cudaSuccess) return li_fail("linear (tcgen05 gemv): cudaGetDevice: %s", cudaGetErrorString(e));
-    LI_REQUIRE(dev >= 0 && dev < 16, "linear (tcgen05 gemv): device index %d out of range", dev);
-    Workspace& w = g_ws[dev];
-    if (!w.partial) {
-        // first call on this device; must happen outside stream capture
-        e = cudaMalloc(&w.partial, kWorkspaceFloats * sizeof(float));
-        if (e != cudaSuccess) return li_fail("linear (tcgen05 gemv): cannot allocate the split-k workspace: %s", cudaGetErrorString(e));
-        e = cudaMalloc(&w.counters, kMaxTiles * sizeof(unsigned));
-        if (e == cudaSuccess) e = cudaMemset(w.counters, 0, kMaxTiles * sizeof(unsigned));
-        if (e != cudaSuccess) return li_fail("linear (tcgen05 gemv): cannot allocate the tile counters: %s", cudaGetErrorString(e));
-    }
-    *ws = &w;
-    return 0;
-}
+// Shared memory of a CTA that finishes `tokens` tokens: the stages, and the rotation's angles and places in the cache.
+template <int BT, int kEpi, int kStages>
+constexpr size_t shared_bytes(int tokens) { return sizeof(Smem<BT, kStages>) + 1024 + (kEpi == kEpiRope ? tokens * (BR / 2 * sizeof(float2) + sizeof(int)) : 0); }
 
 int g_forced_ksplit = 0;          // > 0: this many splits of k whatever the shape (measurements)
 
-// Splits of k: a function of N, K and the token tile (16, 32 or 64 columns), never of the number of tokens itself.
-int choose_ksplit(int N, int K, int bt) {
-    const int tiles = ceil_div(N, BR), nkb = ceil_div(K, BK);
-    int ks;
-    if (g_forced_ksplit > 0) {
-        ks = g_forced_ksplit < nkb ? g_forced_ksplit : nkb;
-    } else {
-        ks = kTargetCtas / tiles;
-        if (ks < 1) ks = 1;
-        const int by_work = nkb / 2 > 0 ? nkb / 2 : 1;                // at least two k-blocks a CTA
-        if (ks > by_work) ks = by_work;
-    }
-    while (ks > 1 && (size_t)ks * tiles * 64 * BR > kWorkspaceFloats) --ks;      // the partial sums fit the workspace: sized for 64 tokens whatever M is
-    // more than 16 tokens: one cluster a tile.  Clusters of four whose sums meet in the workspace write and read every CTA's share
-    // of the tokens once more (64 tokens, N 1536, K 8960: 21.8 us with three of them, 16.4 with one cluster of eight; 32 tokens
-    // 16.2 and 12.5, N 512, K 4096 19.7 and 8.2; up to 16 tokens, N 1536, K 18944 15.4 and 16.0)
-    if (bt >= 32 && ks > 8) ks = 8;
-    if (ks > 8) ks -= ks % 4;                                         // clusters of four
-    return ks;
+// Splits of k: a function of N and K alone, never of the number of tokens.  One cluster a tile; the sums are read four CTAs at a time,
+// and two CTAs a multiprocessor hold 30 clusters of eight and 66 of four.  Measured (us; 1, 8, 32, 64 tokens): N 3584, K 18944, five
+// splits 26.1 27.1 29.2 33.8, four 27.1 27.1 28.2 29.7, eight 24.0 25.6 26.1 28.7; N 3584, K 3584, five 8.4 9.1 10.8 13.4, four 8.0 8.2
+// 9.3 10.4, eight 7.8 8.6 8.6 10.2; N 4608, K 3584 four 9.8 9.8 10.9 12.1, eight 13.2 14.3 15.0 18.0; N 7168, K 5120 two 16.9 17.4 18.4
+// 20.5, four 15.4 15.9 16.9 18.4; N 5120, K 5120 two 15.6 16.0 17.6 19.3, three 13.1 13.1 14.3 16.0.  (N 1536, K 8960 with twelve, three
+// clusters of four that met in a workspace, 10.4 10.7, with eight 9.2 9.8.)
+int choose_ksplit(int N, int K) {
+    const int tiles = ceil_div(N, BR), nkb = ceil_div(K, BK), by_work = nkb / 2 > 0 ? nkb / 2 : 1;      // at least two k-blocks a CTA
+    int ks = g_forced_ksplit;
+    if (ks <= 0) ks = tiles <= 18 || (tiles <= 28 && nkb >= 112) ? 8 : tiles <= 37 ? 4 : tiles <= 49 ? 3 : tiles <= 60 ? 4 : tiles <= 74 ? 2 : 1;
+    if (ks > by_work) ks = by_work;
+    return ks < kMaxCluster ? ks : kMaxCluster;
 }
-int cluster_of(int ksplit) { return ksplit <= 8 ? ksplit : 4; }
 int token_tile(int M) { return M <= 16 ? 16 : M <= 32 ? 32 : 64; }
 
 // How many clusters of `csize` CTAs of a kernel the current device holds at once (asked once a size and device; a size that is asked
@@ -451,7 +425,7 @@ int clusters_at_once(int csize) {
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(1, csize);
         cfg.blockDim = dim3(kThreads);
-        cfg.dynamicSmemBytes = sizeof(Smem<BT, kStages>) + 1024;
+        cfg.dynamicSmemBytes = shared_bytes<BT, kEpi, kStages>(ceil_div(BT, csize));
         cudaLaunchAttribute attr[1];
         attr[0].id = cudaLaunchAttributeClusterDimension;
         attr[0].val.clusterDim.x = attr[0].val.clusterDim.z = 1;
@@ -470,7 +444,7 @@ int clusters_at_once(int csize) {
 template <int BT, typename Tout, int kEpi, int kStages>
 int raise_shared() {
     static LiOncePerDevice raised[2];
-    const size_t smem = sizeof(Smem<BT, kStages>) + 1024;
+    const size_t smem = shared_bytes<BT, kEpi, kStages>(BT);
     cudaError_t e = li_raise_shared(raised[0], (const void*)gemv_tcgen05_kernel<BT, Tout, kEpi, false, kStages>, smem);
     if (e == cudaSuccess) e = li_raise_shared(raised[1], (const void*)gemv_tcgen05_kernel<BT, Tout, kEpi, true, kStages>, smem);
     if (e != cudaSuccess) return li_fail("linear (tcgen05 gemv): cannot raise shared memory to %zu: %s", smem, cudaGetErrorString(e));
@@ -489,24 +463,21 @@ int choose_deep(int tiles, int ksplit, bool* deep) {
         return 0;
     }
     if (int rc = raise_shared<BT, Tout, kEpi, kDeep>()) return rc;
-    *deep = (long long)tiles * ksplit <= (long long)clusters_at_once<BT, Tout, kEpi, kDeep>(cluster_of(ksplit)) * cluster_of(ksplit);
+    *deep = (long long)tiles * ksplit <= (long long)clusters_at_once<BT, Tout, kEpi, kDeep>(ksplit) * ksplit;
     return 0;
 }
 
 template <int BT, typename Tout, int kEpi, int kStages>
-int launch_stages(const CUtensorMap& map_w, const CUtensorMap& map_x, const float* bias, void* out, Workspace* ws, int M, int N, int K, int tiles, int ksplit,
+int launch_stages(const CUtensorMap& map_w, const CUtensorMap& map_x, const float* bias, void* out, int M, int N, int K, int tiles, int ksplit,
                   int* err_dev, const RowScale& rs, const AddScaled& add, const RopeArgs& rope, cudaStream_t stream) {
     if (int rc = raise_shared<BT, Tout, kEpi, kStages>()) return rc;
-    const size_t smem = sizeof(Smem<BT, kStages>) + 1024;
-    if (ksplit == 1) {
-        li_launch_pdl(gemv_tcgen05_kernel<BT, Tout, kEpi, false, kStages>, dim3(tiles, 1), dim3(kThreads), smem, stream, map_w, map_x, bias, (Tout*)out,
-                      ws->partial, ws->counters, M, N, K, 1, 1, err_dev, rs, add, rope);
-    } else {
-        const int csize = cluster_of(ksplit);
-        LI_REQUIRE(tiles * csize <= kMaxTiles, "linear (tcgen05 gemv): N=%d has too many tiles for a split of k", N);
-        li_launch_pdl(gemv_tcgen05_kernel<BT, Tout, kEpi, true, kStages>, dim3(tiles, ksplit), dim3(kThreads), smem, stream, dim3(1, csize, 1), map_w, map_x, bias,
-                      (Tout*)out, ws->partial, ws->counters, M, N, K, ksplit, csize, err_dev, rs, add, rope);
-    }
+    const size_t smem = shared_bytes<BT, kEpi, kStages>(ceil_div(M, ksplit));
+    if (ksplit == 1)
+        li_launch_pdl(gemv_tcgen05_kernel<BT, Tout, kEpi, false, kStages>, dim3(tiles, 1), dim3(kThreads), smem, stream, map_w, map_x, bias, (Tout*)out, M, N, K,
+                      1, err_dev, rs, add, rope);
+    else
+        li_launch_pdl(gemv_tcgen05_kernel<BT, Tout, kEpi, true, kStages>, dim3(tiles, ksplit), dim3(kThreads), smem, stream, dim3(1, ksplit, 1), map_w, map_x,
+                      bias, (Tout*)out, M, N, K, ksplit, err_dev, rs, add, rope);
     return li_check_launch("linear (tcgen05 gemv)");
 }
 
@@ -518,20 +489,15 @@ int launch(const void* a, const void* w, const float* bias, void* out, int M, in
     if (int rc = setup(&encode, &err_host, &err_dev)) return rc;
     if (*err_host != 0)
         return li_fail("linear (tcgen05 gemv): an earlier launch gave up waiting on a barrier (status %d); the results since then are invalid", *err_host);
-    Workspace* ws = nullptr;
-    if (int rc = ensure_workspace(&ws)) return rc;
     const int tiles = ceil_div(N, BR);
-    const int ksplit = choose_ksplit(N, K, BT);
-    LI_REQUIRE(tiles <= kMaxTiles, "linear (tcgen05 gemv): N=%d has too many tiles", N);
-    LI_REQUIRE(ksplit == 1 || (size_t)ksplit * tiles * BT * BR <= kWorkspaceFloats, "linear (tcgen05 gemv): %d splits of %d tiles do not fit the workspace",
-               ksplit, tiles);
+    const int ksplit = choose_ksplit(N, K);
     CUtensorMap map_w, map_x;
     if (int rc = make_map(&map_w, w, N, K, BR)) return rc;
     if (int rc = make_map(&map_x, a, M, K, BT)) return rc;
     bool deep = false;
     if (int rc = choose_deep<BT, Tout, kEpi>(tiles, ksplit, &deep)) return rc;
-    return deep ? launch_stages<BT, Tout, kEpi, kDeep>(map_w, map_x, bias, out, ws, M, N, K, tiles, ksplit, err_dev, rs, add, rope, stream)
-                : launch_stages<BT, Tout, kEpi, kShallow<BT>>(map_w, map_x, bias, out, ws, M, N, K, tiles, ksplit, err_dev, rs, add, rope, stream);
+    return deep ? launch_stages<BT, Tout, kEpi, kDeep>(map_w, map_x, bias, out, M, N, K, tiles, ksplit, err_dev, rs, add, rope, stream)
+                : launch_stages<BT, Tout, kEpi, kShallow<BT>>(map_w, map_x, bias, out, M, N, K, tiles, ksplit, err_dev, rs, add, rope, stream);
 }
 
 template <typename Tout, int kEpi>
@@ -544,7 +510,7 @@ int launch_bt(const void* a, const void* w, const float* bias, void* out, int M,
 
 }  // namespace
 
-// 0: splits of k by shape; n > 0: n splits, as far as there are k-blocks, room in the workspace and whole clusters for them
+// 0: splits of k by shape; n > 0: n splits, as far as there are k-blocks for them and a cluster holds them
 // (li_gemv_tcgen05_plan says how many it became).  For measurements.
 LI_EXPORT void li_gemv_tcgen05_force_ksplit(int n) { g_forced_ksplit = n; }
 
@@ -552,8 +518,8 @@ LI_EXPORT void li_gemv_tcgen05_force_ksplit(int n) { g_forced_ksplit = n; }
 // whether its plain form takes the deep pipeline.  For tests.
 LI_EXPORT int li_gemv_tcgen05_plan(int M, int N, int K, int* splits, int* cluster, int* deep) {
     LI_REQUIRE(M >= 1 && M <= 64 && N >= 1 && K >= 8 && splits && cluster, "linear (tcgen05 gemv): no plan for M=%d N=%d K=%d", M, N, K);
-    *splits = choose_ksplit(N, K, token_tile(M));
-    *cluster = cluster_of(*splits);
+    *splits = choose_ksplit(N, K);
+    *cluster = *splits;
     if (deep) {
         bool d = false;
         const int tiles = ceil_div(N, BR);

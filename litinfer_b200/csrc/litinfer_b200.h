@@ -270,13 +270,9 @@ int li_linear_gemv_static(const void* a, const void* w, const float* bias, void*
     K, cudaStream_t stream);
 
 /* ---- gemv_tcgen05.cu ---- */
-/* Measurements: force the splits of k of the swapped tcgen05 product (0: by shape), as far as there are k-blocks, room in the
- * workspace and whole clusters for them. */
+/* Measurements: force the splits of k of the swapped tcgen05 product (0: by shape), as far as there are k-blocks for them and
+ * a cluster holds them. */
 void li_gemv_tcgen05_force_ksplit(int n);
-
-/* Tests: how a product of M <= 64 rows is cut: the splits of k, and how many of them form a cluster; with deep (needs a device)
- * whether its plain form takes the deep pipeline (all three in host memory). */
-int li_gemv_tcgen05_plan(int M, int N, int K, int* splits, int* cluster, int* deep);
 
 /* ---- linear.cu ---- */
 /* out[M, N] = a[M, K] w[N, K]^T (+ bias), epilogue 0 none / 1 SwiGLU, 2 bounded unit, 3 GEGLU over interleaved gate|up rows; float32 in

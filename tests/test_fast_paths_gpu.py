@@ -142,3 +142,44 @@ def test_a_unit_that_is_its_sequences_only_one(heads, options):
     # probabilities rounded to bfloat16 (2^-9 of each, values about 1) and the result once more
     assert float((got - ref).abs().max()) <= 2.0 ** -8 * float(ref.abs().max()) + 2.0 ** -8
 
+
+
+@pytest.mark.parametrize("splits", [2, 3, 4, 5, 8])
+@pytest.mark.parametrize("M", [1, 2, 9, 16, 17, 31, 33, 50, 64])
+def test_streaming_product_with_its_splits_in_a_cluster(splits, M):
+    """Tokens and CTAs that do not come out in fours: the product and its sum into the residual stream."""
+    N, Kd = 300, 1048
+    a = T.rnd(M, Kd, dtype=torch.bfloat16, seed=M)
+    w = T.rnd(N, Kd, dtype=torch.bfloat16, seed=splits, scale=0.05)
+    bias, norm = T.rnd(N, seed=3), T.rnd(N, seed=4)
+    exact = a.double() @ w.double().T + bias.double()
+    K().library().li_gemv_tcgen05_force_ksplit(splits)
+    try:
+        out = torch.full((M, N), float("nan"), dtype=torch.float32, device="cuda")
+        K().linear_with("gemv_tcgen05", a, w, bias, out)
+        # the same sums of exact products in float32, in another order
+        assert float((out - exact).abs().max()) <= 1e-4
+        # a product that the rule sends there, into the residual stream
+        Nr, Kr = 1152, 4160
+        a, w = T.rnd(M, Kr, dtype=torch.bfloat16, seed=M + 1), T.rnd(Nr, Kr, dtype=torch.bfloat16, seed=splits + 1, scale=0.05)
+        x, bias, norm = T.rnd(M, Nr, seed=5), T.rnd(Nr, seed=6), T.rnd(Nr, seed=7)
+        want = x.double() + a.double() @ w.double().T + bias.double()
+        h = torch.empty((M, Nr), dtype=torch.bfloat16, device="cuda")
+        parts = K().linear_add_scaled_parts(a, w, x, h)
+        assert parts == Nr // 128
+        ssq = torch.full((M, parts), float("nan"), device="cuda")
+        K().linear_add_scaled(a, w, bias, x, norm, h, ssq)
+        assert float((x - want).abs().max()) <= 2e-4
+        assert float((h - want * norm.double()).abs().max()) <= 2.0 ** -8 * float((want * norm.double()).abs().max()) + 2e-4
+        assert torch.allclose(ssq.double(), (want * want).view(M, parts, 128).sum(2), rtol=1e-4)
+    finally:
+        K().library().li_gemv_tcgen05_force_ksplit(0)
+    assert K().library().li_tcgen05_status() == 0
+
+
+@pytest.mark.parametrize("heads", [(20, 4), (28, 4), (40, 8), (60, 8), (90, 9)], ids=str)
+@pytest.mark.parametrize("tokens", [1, 7, 16, 30, 45, 64])
+def test_rotation_in_the_streaming_product_of_every_split(heads, tokens):
+    """q|k|v with four, three, two CTAs a cluster or none: every CTA rotates the tokens it finishes."""
+    nh, nkv = heads
+    T.test_linear_rope_kv_fused(torch.bfloat16, (nh, nkv, 128, tokens, 4160))

@@ -31,6 +31,13 @@ def test_splits_of_the_streaming_product(N, K):
             assert splits == cluster
 
 
+def test_splits_are_few_enough_for_one_cluster():
+    """Eight for few tiles, or up to 28 with a long k; four or three where those are about a wave of CTAs."""
+    assert [plan(8, 128 * t, 4096)[0] for t in (1, 18, 19, 37, 38, 49, 50, 60, 61, 74, 75)] == [8, 8, 4, 4, 3, 3, 4, 4, 2, 2, 1]
+    assert [plan(8, 128 * t, 7168)[0] for t in (19, 28, 29)] == [8, 8, 4]
+    assert plan(8, 1536, 512)[0] == 4                     # two k-blocks a CTA at least
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("M", [32, 64])
 def test_pipeline_depth_of_the_streaming_product(M):
