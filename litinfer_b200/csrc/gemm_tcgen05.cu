@@ -588,12 +588,21 @@ int g_rope_single_tiles = 1;      // 0: the rope epilogue only on paired tiles (
 LI_EXPORT void li_tcgen05_rope_single_tiles(int on) { g_rope_single_tiles = on; }
 
 static bool rope_pairs(int M, int N) {
-    return g_forced_tile == 0 && g_forced_ksplit == 0 && M > 128 && (long long)((ceil_div(M, 128) + 1) & ~1) * ceil_div(N, 256) >= 74;
+    return (g_forced_tile == 0 || g_forced_tile == 11) && g_forced_ksplit == 0 && M > 128 && (long long)((ceil_div(M, 128) + 1) & ~1) * ceil_div(N, 256) >= 74;
+}
+
+bool li_tcgen05_tokens_wanted(int M, int N, int K, bool rope);
+int li_linear_tcgen05_tokens(const void* a, const void* w, const float* bias, void* out, int dtype_out, int M, int N, int K, int epilogue, cudaStream_t stream);
+int li_linear_tcgen05_tokens_rope(const void* a, const void* w, const float* bias, void* out, int M, int N, int K, const RopeEpilogue& rope, cudaStream_t stream);
+
+// Tokens as columns (gemm_tcgen05_persistent.cu).
+static bool takes_tokens(const void* out, int M, int N, int K, bool rope = false) {
+    return (uintptr_t)out % 4 == 0 && (g_forced_tile == 10 || (g_forced_tile == 0 && g_forced_ksplit == 0 && li_tcgen05_tokens_wanted(M, N, K, rope)));
 }
 
 bool li_tcgen05_rope_wanted(const void* a, const void* w, const void* out, int M, int N, int K) {
     if (!li_tcgen05_accepts(a, w, out, LI_BF16, M, N, K) || N % 128 != 0) return false;
-    return rope_pairs(M, N) || (g_forced_tile == 0 && g_forced_ksplit == 0 && g_rope_single_tiles && !li_tcgen05_persistent_wanted(M, N, K));
+    return takes_tokens(out, M, N, K, true) || rope_pairs(M, N) || ((g_forced_tile == 0 || g_forced_tile == 11) && g_forced_ksplit == 0 && g_rope_single_tiles && !li_tcgen05_persistent_wanted(M, N, K));
 }
 
 int li_linear_tcgen05_rope(const void* a, const void* w, const float* bias, void* out, int M, int N, int K, const RopeEpilogue& rope,
@@ -601,6 +610,7 @@ int li_linear_tcgen05_rope(const void* a, const void* w, const float* bias, void
     LI_REQUIRE(li_tcgen05_rope_wanted(a, w, out, M, N, K), "linear + rope (tcgen05): refuses M=%d N=%d K=%d", M, N, K);
     LI_REQUIRE(N == (rope.nh + 2 * rope.nkv) * 128 && rope.cos_sin && rope.slot_mapping && rope.kcache && rope.vcache,
                "linear + rope (tcgen05): N=%d does not match %d + 2 x %d heads of 128, or a null operand", N, rope.nh, rope.nkv);
+    if (takes_tokens(out, M, N, K, true)) return li_linear_tcgen05_tokens_rope(a, w, bias, out, M, N, K, rope, stream);
     if (rope_pairs(M, N)) return launch_tile<128, 256, bf16, false, true, true>(a, w, bias, out, M, N, K, stream, 1, rope);
     return launch_tile<128, 128, bf16, false, false, true>(a, w, bias, out, M, N, K, stream, 1, rope);
 }
@@ -631,7 +641,8 @@ int li_linear_tcgen05_grouped(const void* a, const void* w, void* out, int M, in
 
 // 0: tile size by shape; 1: 128 x 128 always; 2: 256 x 256 always, one CTA a tile; 3: 256 x 128 always; 4: pairs of CTAs on
 // 512 x 256 (two accumulators each); 5: pairs of CTAs on 256 x 256 (one accumulator each); 6: the persistent kernel
-// (gemm_tcgen05_persistent.cu); 7: pairs of CTAs on 256 x 192; 8: 128 x 64; 9: 128 x 32.  For tests and measurements.
+// (gemm_tcgen05_persistent.cu); 7: pairs of CTAs on 256 x 192; 8: 128 x 64; 9: 128 x 32; 10: tokens as columns
+// (gemm_tcgen05_persistent.cu); 11: by shape without those.  For tests and measurements.
 LI_EXPORT void li_tcgen05_force_tile(int tile) { g_forced_tile = tile; }
 
 // 0: splits of k by shape; n > 0: n splits always.  For tests and measurements.
@@ -648,17 +659,18 @@ int li_linear_tcgen05_persistent(const void* a, const void* w, const float* bias
 
 int li_linear_tcgen05(const void* a, const void* w, const float* bias, void* out, int dtype_out, int M, int N, int K,
                       int epilogue, cudaStream_t stream) {
+    if (takes_tokens(out, M, N, K)) return li_linear_tcgen05_tokens(a, w, bias, out, dtype_out, M, N, K, epilogue, stream);
     // many tiles: the persistent kernel, whose epilogue overlaps the next tile's products
-    if (g_forced_tile == 6 || (g_forced_tile == 0 && g_forced_ksplit == 0 && li_tcgen05_persistent_wanted(M, N, K)))
+    if (g_forced_tile == 6 || ((g_forced_tile == 0 || g_forced_tile == 11) && g_forced_ksplit == 0 && li_tcgen05_persistent_wanted(M, N, K)))
         return li_linear_tcgen05_persistent(a, w, bias, out, dtype_out, M, N, K, epilogue, stream);
     if (li_epilogue_is_gated(epilogue)) {
         LI_REQUIRE(N % 16 == 0 && li_epilogue_bias_ok(epilogue, bias) && dtype_out == LI_BF16,
                    "linear (tcgen05): the swiglu epilogue needs N a multiple of 16, no bias and bfloat16 output");
         return epilogue == LI_EPILOGUE_GLU_CLAMPED ? launch<bf16, 2>(a, w, bias, out, M, N, K, stream, g_forced_tile)
                : epilogue == LI_EPILOGUE_GEGLU     ? launch<bf16, 3>(a, w, bias, out, M, N, K, stream, g_forced_tile)
-                                                   : launch<bf16, 1>(a, w, bias, out, M, N, K, stream, g_forced_tile);
+                                                   : launch<bf16, 1>(a, w, bias, out, M, N, K, stream, g_forced_tile == 11 ? 0 : g_forced_tile);
     }
-    if (dtype_out == LI_BF16) return launch<bf16, 0>(a, w, bias, out, M, N, K, stream, g_forced_tile);
-    if (dtype_out == LI_F32) return launch<float, 0>(a, w, bias, out, M, N, K, stream, g_forced_tile);
+    if (dtype_out == LI_BF16) return launch<bf16, 0>(a, w, bias, out, M, N, K, stream, g_forced_tile == 11 ? 0 : g_forced_tile);
+    if (dtype_out == LI_F32) return launch<float, 0>(a, w, bias, out, M, N, K, stream, g_forced_tile == 11 ? 0 : g_forced_tile);
     return li_fail("linear (tcgen05): unsupported output dtype %d", dtype_out);
 }

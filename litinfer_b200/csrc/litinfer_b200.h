@@ -256,6 +256,13 @@ void li_tcgen05_force_tile(int tile);
 /* Tests and measurements: force the splits of k of the tcgen05 product (0: by shape). */
 void li_tcgen05_force_ksplit(int n);
 
+/* ---- gemm_tcgen05_persistent.cu ---- */
+/* Tests and measurements: this many tokens a tile (32 to 512 in steps of 32) of the product with tokens as columns, 0: by shape. */
+int li_tcgen05_tokens_force_width(int width);
+
+/* Tests: whether the product of M rows has its tokens as columns. */
+int li_tcgen05_takes_tokens(int M, int N, int K);
+
 /* ---- attention_f32.cu ---- */
 /* Tests: how many blocks share a token's keys in the float32 attention of a step of T tokens. */
 int li_attention_f32_blocks(int T, int nh, int nkv, int dh);

@@ -149,19 +149,23 @@ def test_a_unit_that_is_its_sequences_only_one(heads, options):
 def test_streaming_product_with_its_splits_in_a_cluster(splits, M):
     """Tokens and CTAs that do not come out in fours: the product and its sum into the residual stream."""
     N, Kd = 300, 1048
-    a = T.rnd(M, Kd, dtype=torch.bfloat16, seed=M)
+    a = T.rnd(M, Kd, dtype=torch.bfloat16, seed=100 + M)
     w = T.rnd(N, Kd, dtype=torch.bfloat16, seed=splits, scale=0.05)
-    bias, norm = T.rnd(N, seed=3), T.rnd(N, seed=4)
+    bias = T.rnd(N, seed=13)
+
+    def bound(a, w):
+        # exact products, added in float32 sixteen at a time: each of these sums may lose a last place of what has come together
+        return a.shape[1] / 16 * 2.0 ** -23 * float((a.abs().float() @ w.abs().float().T).max()) + 1e-5
+
     exact = a.double() @ w.double().T + bias.double()
     K().library().li_gemv_tcgen05_force_ksplit(splits)
     try:
         out = torch.full((M, N), float("nan"), dtype=torch.float32, device="cuda")
         K().linear_with("gemv_tcgen05", a, w, bias, out)
-        # the same sums of exact products in float32, in another order
-        assert float((out - exact).abs().max()) <= 1e-4
+        assert float((out - exact).abs().max()) <= bound(a, w)
         # a product that the rule sends there, into the residual stream
         Nr, Kr = 1152, 4160
-        a, w = T.rnd(M, Kr, dtype=torch.bfloat16, seed=M + 1), T.rnd(Nr, Kr, dtype=torch.bfloat16, seed=splits + 1, scale=0.05)
+        a, w = T.rnd(M, Kr, dtype=torch.bfloat16, seed=200 + M), T.rnd(Nr, Kr, dtype=torch.bfloat16, seed=splits + 20, scale=0.05)
         x, bias, norm = T.rnd(M, Nr, seed=5), T.rnd(Nr, seed=6), T.rnd(Nr, seed=7)
         want = x.double() + a.double() @ w.double().T + bias.double()
         h = torch.empty((M, Nr), dtype=torch.bfloat16, device="cuda")
@@ -169,9 +173,9 @@ def test_streaming_product_with_its_splits_in_a_cluster(splits, M):
         assert parts == Nr // 128
         ssq = torch.full((M, parts), float("nan"), device="cuda")
         K().linear_add_scaled(a, w, bias, x, norm, h, ssq)
-        assert float((x - want).abs().max()) <= 2e-4
-        assert float((h - want * norm.double()).abs().max()) <= 2.0 ** -8 * float((want * norm.double()).abs().max()) + 2e-4
-        assert torch.allclose(ssq.double(), (want * want).view(M, parts, 128).sum(2), rtol=1e-4)
+        assert float((x - want).abs().max()) <= bound(a, w)
+        assert float((h - want * norm.double()).abs().max()) <= 2.0 ** -8 * float((want * norm.double()).abs().max()) + bound(a, w) * float(norm.abs().max())
+        assert torch.allclose(ssq.double(), (want * want).view(M, parts, 128).sum(2), rtol=1e-3)
     finally:
         K().library().li_gemv_tcgen05_force_ksplit(0)
     assert K().library().li_tcgen05_status() == 0
@@ -183,3 +187,69 @@ def test_rotation_in_the_streaming_product_of_every_split(heads, tokens):
     """q|k|v with four, three, two CTAs a cluster or none: every CTA rotates the tokens it finishes."""
     nh, nkv = heads
     T.test_linear_rope_kv_fused(torch.bfloat16, (nh, nkv, 128, tokens, 4160))
+
+
+def forced(tile, width=0):
+    lib = K().library()
+    lib.li_tcgen05_force_tile(tile)
+    assert lib.li_tcgen05_tokens_force_width(width) == 0
+
+
+@pytest.mark.parametrize("width", [0, 32, 96, 256, 288, 416, 512])
+@pytest.mark.parametrize("M", [1, 33, 129, 300, 544, 1100])
+@pytest.mark.parametrize("N,Kd", [(256, 64), (384, 520), (1000, 256), (1026, 72), (1333, 200), (2064, 1536)])
+def test_product_with_tokens_as_columns(N, Kd, M, width):
+    """Tiles of every kind of width, rows of w and tokens that fill no tile, odd row lengths: against the tiles of 128 x 128, whose sums
+    are the same ones in the same order."""
+    a = T.rnd(M, Kd, dtype=torch.bfloat16, seed=M)
+    w = T.rnd(N, Kd, dtype=torch.bfloat16, seed=N, scale=0.1)
+    bias = T.rnd(N, seed=5)
+    try:
+        for epilogue, dtype in ((None, torch.bfloat16), (None, torch.float32), ("swiglu", torch.bfloat16), ("geglu", torch.bfloat16)):
+            if epilogue and N % 16:
+                continue
+            out = torch.full((M, N // 2 if epilogue else N), float("nan"), dtype=dtype, device="cuda")
+            ref = torch.full_like(out, float("nan"))
+            forced(10, width)
+            K().linear_with("tcgen05", a, w, None if epilogue else bias, out, epilogue)
+            forced(1)
+            K().linear_with("tcgen05", a, w, None if epilogue else bias, ref, epilogue)
+            T.close(out, ref, dtype, f"tokens as columns {epilogue} {dtype}")
+    finally:
+        forced(0)
+    assert K().library().li_tcgen05_status() == 0
+
+
+@pytest.mark.parametrize("first", [0, 5])
+@pytest.mark.parametrize("heads", [(28, 4), (3, 2)], ids=str)
+@pytest.mark.parametrize("tokens", [70, 200, 530])
+def test_rotation_with_tokens_as_columns(heads, tokens, first):
+    """A last tile with one head, places in the cache that follow one another (values leave eight at a time where they are aligned),
+    that do not, and that are not there; the rest of the cache is left alone."""
+    nh, nkv = heads
+    N, width, page = (nh + 2 * nkv) * 128, 264, 16
+    pages = (tokens + first) // page + 3
+    a, w = T.rnd(tokens, width, dtype=torch.bfloat16, seed=1), T.rnd(N, width, dtype=torch.bfloat16, seed=2, scale=0.1)
+    bias = T.rnd(N, seed=3)
+    positions = (torch.arange(tokens, dtype=torch.int32) % 300).cuda()
+    denom = torch.pow(torch.tensor(10000.0), torch.arange(64, dtype=torch.float32) / 64).cuda()
+    slots = torch.arange(first, first + tokens, dtype=torch.int32)
+    slots[40:48] = slots[40:48].flip(0)
+    slots[63] = -1
+    table = torch.empty(tokens, 64, 2, device="cuda")
+    K().rope_table(positions, denom, table)
+    results = []
+    try:
+        for tile in (10, 11):
+            forced(tile)
+            qkv = torch.zeros(tokens, N, dtype=torch.bfloat16, device="cuda")
+            kc = torch.full((pages, nkv, page, 128), 3.0, dtype=torch.bfloat16, device="cuda")
+            vc = torch.full((pages, nkv, 128, page), 3.0, dtype=torch.bfloat16, device="cuda")
+            K().linear_rope_kv(a, w, bias, qkv, positions, denom, 128, slots.cuda(), kc, vc, nh, nkv, 128, True, cos_sin=table)
+            results.append((qkv[:, :nh * 128], kc, vc))
+    finally:
+        forced(0)
+    for got, ref in zip(*results):
+        assert torch.equal(got == 3.0, ref == 3.0)
+        T.close(got, ref, torch.bfloat16, "rotation with tokens as columns")
+    assert K().library().li_tcgen05_status() == 0

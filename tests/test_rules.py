@@ -83,3 +83,11 @@ def test_blocks_that_share_a_token_in_float32_attention():
     assert [blocks(T, 12, 2, 128) for T in (1, 9, 10, 18, 19, 37, 38, 2048)] == [8, 8, 4, 4, 2, 2, 1, 1]
     assert [blocks(T, 32, 1, 64) for T in (9, 10, 18, 19, 37, 38)] == [8, 4, 4, 2, 2, 1]          # 32 heads: four parts
     assert blocks(16, 28, 4, 128) == 2
+
+
+@pytest.mark.parametrize("M,N,K,taken", [(640, 7168, 5120, 1), (640, 27648, 5120, 1), (640, 5120, 5120, 1), (320, 37888, 3584, 1), (1536, 3584, 18944, 1),
+                                         (2048, 7168, 5120, 1), (2048, 1536, 1536, 1), (2048, 17920, 1536, 0), (1024, 37888, 3584, 0), (128, 37888, 3584, 0),
+                                         (640, 1536, 8960, 0), (256, 2048, 1536, 0)])
+def test_which_products_have_their_tokens_as_columns(M, N, K, taken):
+    """Where the padding of 256 tokens or half-empty waves cost more than the narrower tiles; never where k is split."""
+    assert library().li_tcgen05_takes_tokens(M, N, K) == taken
