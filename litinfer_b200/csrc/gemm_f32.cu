@@ -5,7 +5,8 @@
 // Every output is summed in one order that K alone decides, whatever M is and whichever of the two kernels below takes the
 // product, so that the value of a row does not depend on how many other rows are in the batch:
 //   chunk:   32 consecutive k, one chain of multiply-adds in ascending order;
-//   segment: 512 consecutive k, its chunks added in ascending order;
+//   half:    256 consecutive k, its chunks added in ascending order;
+//   segment: 512 consecutive k, its two halves added;
 //   total:   the segments added in ascending order, then the bias.
 // That order leaves three places to cut the work: chunks over the warps of a block, segments over the blocks of a cluster
 // (their sums meet through distributed shared memory: no workspace, no counters), rows and columns over the grid.  Its
@@ -13,8 +14,7 @@
 // with the chain).
 //
 // Measured against one 64 x 64 kernel for every size, single chain, scalar loads (us): 3 rows, N 17920, K 1536 21.4 (5.1 TB/s),
-// N 1536, K 8960 16.7, N 151936 153 (6.1 TB/s; that kernel: 307 on average over a step's products); 192 rows, N 17920, K 1536
-// 252 (42 TFLOP/s; 370 on average).  A step of 3 tokens of the 1.5B shape 61.2 -> 2.4 ms, of 145 tokens 46.6 -> 18.0 ms.
+// N 1536, K 8960 16.7, N 151936 153 (6.1 TB/s; that kernel: 307 on average over a step's products).
 //
 // f32_stream_kernel, M <= 16: bound by reading w once.  A block takes 32 rows of w; whole segments of those rows come
 // through two stages of 64 KB by TMA, a tile of 32 rows a chunk (128-byte swizzle: eight lanes on consecutive rows meet
@@ -22,12 +22,18 @@
 // and tokens (2 x 4, 4 x 4 or 4 x 8), since with one row a lane the reads of the activations from shared memory cost more
 // than memory needs for w.  One block a multiprocessor walks over the tiles; where there are fewer tiles than
 // multiprocessors the segments of a tile go to a cluster.
-// f32_tile_kernel, M > 16 (and operands that are not 16-byte aligned): bound by the multiply-add pipes and the latencies of
-// two warps a scheduler.  128 columns by 64 (32) rows a block of 128 threads, 8 x 8 (4 x 8) outputs a thread, packed
-// multiply-adds over pairs of columns, tiles of 16 k through registers into two transposed buffers.
+// f32_tile_kernel, M > 16 (and operands that are not 16-byte aligned): bound by the multiply-add pipes (packed multiply-adds
+// from registers alone reach 57 to 62 TFLOP/s here), the latencies of two warps a scheduler, and by how the tiles fill the GPU.
+// 128 columns by 32, 48, 64 or 80 rows a group of 128 threads, 4 x 8 to 10 x 8 outputs a thread, packed multiply-adds over pairs of
+// columns, tiles of 16 k through registers into two transposed buffers.  The halves of a tile's segments are shared out over the
+// groups of a block (one or two) and the blocks of a cluster; tile_plan chooses.  Against 64 (or 32) rows, whole segments and
+// blocks of one group (us): 64 rows N 2048, K 1536 38.9 -> 27.1, N 17920 119 -> 96, N 1536, K 8960 125 -> 97; 128 rows N 1536, K 8960
+// 182 -> 130; 192 rows N 1536, K 1536 50 -> 34.
 #define LI_PDL_KIND 2
 #include "tcgen05.cuh"
 
+#include <algorithm>
+#include <atomic>
 #include <cooperative_groups.h>
 
 namespace {
@@ -35,7 +41,7 @@ namespace {
 namespace cg = cooperative_groups;
 using namespace tc;
 
-constexpr int kChunk = 32, kSegment = 512, kChunks = kSegment / kChunk;
+constexpr int kChunk = 32, kSegment = 512, kChunks = kSegment / kChunk, kHalf = kSegment / 2;
 constexpr int kMaxCluster = 8;
 
 // ---------------------------------------------------------------------------------------------
@@ -173,9 +179,10 @@ f32_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
                 consumers_sync();
                 if (tid < kPartTokens * kRows) {
                     const int pm = tid / kRows, m = pm / TR * T + r * TR + pm % TR, n = n0 + (tid & (kRows - 1));
-                    float v = 0.0f;
+                    float v = 0.0f, second = 0.0f;
 #pragma unroll
-                    for (int c = 0; c < kChunks; ++c) v += sm.part[c][tid];
+                    for (int c = 0; c < kChunks / 2; ++c) v += sm.part[c][tid], second += sm.part[kChunks / 2 + c][tid];
+                    v += second;
                     if (csize == 1) {
                         sum[r] += v;
                         if (last) {
@@ -211,12 +218,18 @@ f32_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
 
 constexpr int kBN = 128, kBK = 16, kThreadsT = 128;
 
+// What a group of 128 threads works with.  TM rows a thread: TM / 4 times four (rows 32 h + 4 ty ..), then two where TM is not a
+// multiple of four.
 template <int TM>
-struct __align__(16) TileSmem {
+struct __align__(16) GroupSmem {
     float w[2][kBK][kBN + 4];
     float a[2][kBK][8 * TM + 4];
-    float4 sums[2 * TM][kThreadsT];                        // a segment's sums of this block (alone: the running totals), per thread
-    float4 total[1][kThreadsT];                            // of a cluster: this block's slice of the totals, ceil(2 TM / blocks) of them
+    float4 sums[2 * TM][kThreadsT];                        // the sums of a half segment, per thread
+};
+template <int TM, int kGroups>
+struct __align__(16) TileSmem {
+    GroupSmem<TM> g[kGroups];
+    float4 total[1][kGroups * kThreadsT];                  // running totals: all of a group's own (alone), or its share of the tile's
 };
 __device__ __forceinline__ unsigned long long pack2(float lo, float hi) {
     unsigned long long r;
@@ -228,36 +241,45 @@ __device__ __forceinline__ void unpack2(unsigned long long v, float& lo, float& 
 __device__ __forceinline__ void fma2(unsigned long long& d, unsigned long long a, unsigned long long b) {
     asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b));
 }
+__device__ __forceinline__ float4 add4(float4 a, float4 b) { return make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w); }
 
-template <int TM, bool kVec>
-__global__ void __launch_bounds__(kThreadsT, 2)
-f32_tile_kernel(const float* __restrict__ A, const float* __restrict__ W, const float* __restrict__ bias, float* __restrict__ out, int M, int N, int K) {
+template <int TM, int kGroups, bool kVec>
+__global__ void __launch_bounds__(kGroups * kThreadsT, kGroups == 1 ? 2 : 1)
+f32_tile_kernel(const float* __restrict__ A, const float* __restrict__ W, const float* __restrict__ bias, float* __restrict__ out, int M, int N, int K,
+                bool wide_stores) {
     extern __shared__ float4 raw4[];
-    TileSmem<TM>& sm = *reinterpret_cast<TileSmem<TM>*>(raw4);
-    constexpr int BM = 8 * TM, kLoadsA = (BM + 31) / 32;
-    const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;             // a thread: rows 4 ty .. (and 32 + 4 ty ..), columns 4 tx .. and 64 + 4 tx ..
+    TileSmem<TM, kGroups>& sm = *reinterpret_cast<TileSmem<TM, kGroups>*>(raw4);
+    constexpr int BM = 8 * TM, kLoadsA = (BM + 31) / 32, kFours = TM / 4;
+    static_assert(TM % 2 == 0 && kGroups <= 2, "rows in fours and a two");
+    const int grp = (int)threadIdx.x / kThreadsT, tid = (int)threadIdx.x % kThreadsT, tx = tid & 15, ty = tid >> 4;      // columns 4 tx .. and 64 + 4 tx ..
+    GroupSmem<TM>& gs = sm.g[grp];
     // tiles of rows run fastest, so that a tile of w is read by neighbours; all tiles along x, which has room for any N
     const int mt = (M + BM - 1) / BM;
     const int m0 = (int)blockIdx.x % mt * BM, n0 = (int)blockIdx.x / mt * kBN;
-    const int csize = (int)gridDim.z, rank = (int)blockIdx.z;
-    const int nseg = (K + kSegment - 1) / kSegment;
+    // the half segments of a tile are shared out over the groups of a cluster's blocks: group v takes v, v + vr, ...
+    const int csize = (int)gridDim.z, rank = (int)blockIdx.z, vr = csize * kGroups, v = rank * kGroups + grp;
+    const int halves = (K + kHalf - 1) / kHalf;
     const int lr = tid >> 2, lk = (tid & 3) * 4;           // loads: rows lr + 32 r, four k from lk on
+    auto group_sync = [&] {
+        if constexpr (kGroups == 1) __syncthreads();
+        else asm volatile("bar.sync %0, 128;" ::"r"(1 + grp) : "memory");
+    };
 
     float4 pa[kLoadsA], pw[4];
     auto load4 = [&](const float* base, int row, int rows, int k) {
-        float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        float4 x = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         if (row < rows) {
             const float* p = base + (size_t)row * K + k;
             if constexpr (kVec) {
-                if (k < K) v = __ldg(reinterpret_cast<const float4*>(p));
+                if (k < K) x = __ldg(reinterpret_cast<const float4*>(p));
             } else {
-                if (k < K) v.x = p[0];
-                if (k + 1 < K) v.y = p[1];
-                if (k + 2 < K) v.z = p[2];
-                if (k + 3 < K) v.w = p[3];
+                if (k < K) x.x = p[0];
+                if (k + 1 < K) x.y = p[1];
+                if (k + 2 < K) x.z = p[2];
+                if (k + 3 < K) x.w = p[3];
             }
         }
-        return v;
+        return x;
     };
     auto fetch = [&](int k0) {
 #pragma unroll
@@ -269,14 +291,14 @@ f32_tile_kernel(const float* __restrict__ A, const float* __restrict__ W, const 
     auto put = [&](int b) {
 #pragma unroll
         for (int r = 0; r < 4; ++r) {
-            sm.w[b][lk][lr + 32 * r] = pw[r].x, sm.w[b][lk + 1][lr + 32 * r] = pw[r].y;
-            sm.w[b][lk + 2][lr + 32 * r] = pw[r].z, sm.w[b][lk + 3][lr + 32 * r] = pw[r].w;
+            gs.w[b][lk][lr + 32 * r] = pw[r].x, gs.w[b][lk + 1][lr + 32 * r] = pw[r].y;
+            gs.w[b][lk + 2][lr + 32 * r] = pw[r].z, gs.w[b][lk + 3][lr + 32 * r] = pw[r].w;
         }
 #pragma unroll
         for (int r = 0; r < kLoadsA; ++r) {
             if (lr + 32 * r < BM) {
-                sm.a[b][lk][lr + 32 * r] = pa[r].x, sm.a[b][lk + 1][lr + 32 * r] = pa[r].y;
-                sm.a[b][lk + 2][lr + 32 * r] = pa[r].z, sm.a[b][lk + 3][lr + 32 * r] = pa[r].w;
+                gs.a[b][lk][lr + 32 * r] = pa[r].x, gs.a[b][lk + 1][lr + 32 * r] = pa[r].y;
+                gs.a[b][lk + 2][lr + 32 * r] = pa[r].z, gs.a[b][lk + 3][lr + 32 * r] = pa[r].w;
             }
         }
     };
@@ -291,36 +313,46 @@ f32_tile_kernel(const float* __restrict__ A, const float* __restrict__ W, const 
         for (int j = 0; j < 8; ++j) seg[i][j] = 0.0f;
     }
     // float4 q of a thread: its row q / 2, columns 4 tx .. (q even) or 64 + 4 tx .. (q odd)
-    for (int q = rank; q < 2 * TM; q += csize) (csize == 1 ? sm.sums[q] : sm.total[q / csize])[tid] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    for (int q = v; q < 2 * TM; q += vr) sm.total[q / vr][threadIdx.x] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
 
-    const int waves = (nseg + csize - 1) / csize;
+    const int waves = (halves + vr - 1) / vr;
     int buf = 0;
     pdl_launch_dependents();
     pdl_wait();
-    if (rank < nseg) fetch(rank * kSegment);
+    if (v < halves) fetch(v * kHalf);
     for (int wave = 0; wave < waves; ++wave) {
-        const int g = wave * csize + rank;
-        if (g < nseg) {
-            const int k_begin = g * kSegment, k_end = min(K, k_begin + kSegment);
+        const int g = wave * vr + v;
+        if (g < halves) {
+            const int k_begin = g * kHalf, k_end = min(K, k_begin + kHalf);
             for (int k0 = k_begin; k0 < k_end; k0 += kBK) {
                 put(buf);
-                __syncthreads();                           // (two buffers: one barrier a tile)
-                const int next = k0 + kBK < k_end ? k0 + kBK : (g + csize) * kSegment;
+                group_sync();                              // (two buffers: one barrier a tile)
+                const int next = k0 + kBK < k_end ? k0 + kBK : (g + vr) * kHalf;
                 if (next < K) fetch(next);
 #pragma unroll
                 for (int kk = 0; kk < kBK; ++kk) {
-                    const ulonglong2 u = *reinterpret_cast<const ulonglong2*>(&sm.w[buf][kk][4 * tx]);
-                    const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(&sm.w[buf][kk][64 + 4 * tx]);
-                    const unsigned long long w2[4] = {u.x, u.y, v.x, v.y};
+                    const ulonglong2 w01 = *reinterpret_cast<const ulonglong2*>(&gs.w[buf][kk][4 * tx]);
+                    const ulonglong2 w23 = *reinterpret_cast<const ulonglong2*>(&gs.w[buf][kk][64 + 4 * tx]);
+                    const unsigned long long w2[4] = {w01.x, w01.y, w23.x, w23.y};
 #pragma unroll
-                    for (int h = 0; h < TM / 4; ++h) {
-                        const float4 a4 = *reinterpret_cast<const float4*>(&sm.a[buf][kk][32 * h + 4 * ty]);
+                    for (int h = 0; h < kFours; ++h) {
+                        const float4 a4 = *reinterpret_cast<const float4*>(&gs.a[buf][kk][32 * h + 4 * ty]);
                         const float av[4] = {a4.x, a4.y, a4.z, a4.w};
 #pragma unroll
                         for (int i = 0; i < 4; ++i) {
                             const unsigned long long aa = pack2(av[i], av[i]);
 #pragma unroll
                             for (int j = 0; j < 4; ++j) fma2(acc[4 * h + i][j], aa, w2[j]);
+                        }
+                    }
+                    if constexpr (TM % 4 != 0) {
+                        const float2 a2 = *reinterpret_cast<const float2*>(&gs.a[buf][kk][32 * kFours + 2 * ty]);
+                        const float av[2] = {a2.x, a2.y};
+#pragma unroll
+                        for (int i = 0; i < 2; ++i) {
+                            const unsigned long long aa = pack2(av[i], av[i]);
+#pragma unroll
+                            for (int j = 0; j < 4; ++j) fma2(acc[4 * kFours + i][j], aa, w2[j]);
                         }
                     }
                 }
@@ -338,40 +370,53 @@ f32_tile_kernel(const float* __restrict__ A, const float* __restrict__ W, const 
                 }
             }
         }
+        // alone: the first half of a segment waits in `sums` for the second; else every group's halves meet, two by two
+        const bool pair = vr > 1 || ((g & 1) == 0 && g + 1 < halves);
 #pragma unroll
         for (int q = 0; q < 2 * TM; ++q) {
             float* sg = &seg[q >> 1][4 * (q & 1)];
-            float4 v = make_float4(sg[0], sg[1], sg[2], sg[3]);
-            if (csize == 1) {
-                const float4 o = sm.sums[q][tid];
-                v.x += o.x, v.y += o.y, v.z += o.z, v.w += o.w;
-            }
-            sm.sums[q][tid] = v;
+            const float4 x = make_float4(sg[0], sg[1], sg[2], sg[3]);
+            if (pair) gs.sums[q][tid] = x;
+            else sm.total[q][tid] = add4(sm.total[q][tid], (g & 1) ? add4(gs.sums[q][tid], x) : x);
             sg[0] = sg[1] = sg[2] = sg[3] = 0.0f;
         }
-        if (csize > 1) {
+        if (vr > 1) {
             cg::cluster_group cluster = cg::this_cluster();
-            cluster.sync();
-            const int here = min(csize, nseg - wave * csize);
-            for (int q = rank; q < 2 * TM; q += csize) {
-                float4 v = sm.total[q / csize][tid];
-                for (int r = 0; r < here; ++r) {
-                    const float4 o = *cluster.map_shared_rank(&sm.sums[q][tid], r);
-                    v.x += o.x, v.y += o.y, v.z += o.z, v.w += o.w;
-                }
-                sm.total[q / csize][tid] = v;
+            if (csize > 1) cluster.sync();
+            else __syncthreads();
+            const int here = min(vr, halves - wave * vr);
+            auto of = [&](int q, int r) {
+                const float4* p = &sm.g[r % kGroups].sums[q][tid];
+                return csize > 1 ? *cluster.map_shared_rank(p, r / kGroups) : *p;
+            };
+            for (int q = v; q < 2 * TM; q += vr) {
+                float4 x = sm.total[q / vr][threadIdx.x];
+                int r = 0;
+                for (; r + 1 < here; r += 2) x = add4(x, add4(of(q, r), of(q, r + 1)));
+                if (r < here) x = add4(x, of(q, r));
+                sm.total[q / vr][threadIdx.x] = x;
             }
-            cluster.sync();                                // before the next segment's sums, and before anyone leaves
+            if (csize > 1) cluster.sync();                 // before the next sums, and before anyone leaves
+            else __syncthreads();
         }
     }
-    for (int q = rank; q < 2 * TM; q += csize) {
-        const float4 v = csize == 1 ? sm.sums[q][tid] : sm.total[q / csize][tid];
-        const int m = m0 + (q >> 3) * 32 + 4 * ty + ((q >> 1) & 3), n = n0 + (q & 1) * 64 + 4 * tx;
+    for (int q = v; q < 2 * TM; q += vr) {
+        const float4 x = sm.total[q / vr][threadIdx.x];
+        const int i = q >> 1, row = i < 4 * kFours ? (i >> 2) * 32 + 4 * ty + (i & 3) : 32 * kFours + 2 * ty + (i - 4 * kFours);
+        const int m = m0 + row, n = n0 + (q & 1) * 64 + 4 * tx;
         if (m >= M) continue;
-        const float r[4] = {v.x, v.y, v.z, v.w};
+        float r[4] = {x.x, x.y, x.z, x.w};
 #pragma unroll
         for (int j = 0; j < 4; ++j)
-            if (n + j < N) out[(size_t)m * N + n + j] = r[j] + (bias ? bias[n + j] : 0.0f);
+            if (bias && n + j < N) r[j] += bias[n + j];
+        float* to = out + (size_t)m * N + n;
+        if (wide_stores && n + 3 < N) {
+            *reinterpret_cast<float4*>(to) = make_float4(r[0], r[1], r[2], r[3]);
+        } else {
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                if (n + j < N) to[j] = r[j];
+        }
     }
 }
 
@@ -390,12 +435,83 @@ int stream_cluster(int tiles, int nseg, int slots) {
     return best;
 }
 
-// More rows: as many as two blocks a multiprocessor leave room for, in equal waves (192 rows: N 1536, K 8960 198 us in clusters
-// of six, 318 with 32 rows a tile in clusters of two; N 1536, K 1536 59 us in clusters of three, 78 in clusters of two).
-int tile_cluster(long long tiles, int nseg) {
-    int c = 1;
-    while (c < nseg && c < kMaxCluster && tiles * (c + 1) <= 2 * li_multiprocessors()) ++c;
-    return ceil_div(nseg, ceil_div(nseg, c));
+// More rows: the shape of a launch.
+struct TilePlan {
+    int tm, groups, cluster;                               // rows a thread (tiles of 8 tm rows), groups a block, blocks that share a tile
+};
+TilePlan g_forced_tile{0, 0, 0};
+
+template <int TM, int kGroups>
+size_t tile_shared(int c) {
+    return sizeof(TileSmem<TM, kGroups>) + (ceil_div(2 * TM, c * kGroups) - 1) * sizeof(float4) * kThreadsT * kGroups;
+}
+
+// How many clusters of c blocks the current device holds at once (asked once a size and device; two threads that ask at the same time
+// both ask).
+template <int TM, int kGroups>
+int clusters_at_once(int c) {
+    static std::atomic<int> known[16][kMaxCluster + 1];
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 16) return 1;
+    int n = known[dev][c].load(std::memory_order_relaxed);
+    if (n == 0) {
+        static LiOncePerDevice raised;
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(1, 1, c);
+        cfg.blockDim = dim3(kThreadsT * kGroups);
+        cfg.dynamicSmemBytes = tile_shared<TM, kGroups>(c);
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = attr[0].val.clusterDim.y = 1;
+        attr[0].val.clusterDim.z = c;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        if (li_raise_shared(raised, (const void*)f32_tile_kernel<TM, kGroups, true>, tile_shared<TM, kGroups>(1)) != cudaSuccess ||
+            (c == 1 ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, f32_tile_kernel<TM, kGroups, true>, kThreadsT * kGroups, tile_shared<TM, kGroups>(1))
+                    : cudaOccupancyMaxActiveClusters(&n, f32_tile_kernel<TM, kGroups, true>, &cfg)) != cudaSuccess || n < 1) {
+            cudaGetLastError();
+            n = 1;
+        }
+        if (c == 1) n *= li_multiprocessors();
+        known[dev][c].store(n, std::memory_order_relaxed);
+    }
+    return n;
+}
+
+// What a launch should take, in microseconds: a half segment is 256 k of `step` cycles, the longer of the thread's multiply-adds and the
+// reads of their operands; one, two or three groups on a multiprocessor take 2.4 (blocks that come when others have gone 1.8), 3.25 or
+// 4.5 times that; a cluster's merge 1.5 us.  (145 rows: N 17920, K 1536 says 211, takes 209; N 1536, K 8960 150 and 150; N 1536, K 1536 32 and 31; 45 rows, N 1536, K
+// 8960 80 and 83.)
+template <int TM>
+void consider(int M, int N, int K, bool vec, TilePlan& best, double& least) {
+    const long long tiles = ceil_div_ll(M, 8 * TM) * ceil_div_ll(N, kBN);
+    const int halves = ceil_div(K, kHalf), sms = li_multiprocessors();
+    const double half = (TM * 8 > (TM + 8) * 4 ? TM * 8 : (TM + 8) * 4) * kHalf / 1920.0;
+    const double times[4] = {0.0, 2.4, 3.25, 4.5};
+    for (int groups = 1; groups <= (vec ? 2 : 1); ++groups)
+        for (int c = 1; c <= kMaxCluster; c += (groups == 1 && c > 1) ? 2 : 1) {
+            const int vr = c * groups;
+            if (vr > 1 && vr > halves + 1) break;
+            const int most = groups == 1 ? clusters_at_once<TM, 1>(c) : clusters_at_once<TM, 2>(c), alone = clusters_at_once<TM, 2>(c);
+            const int dense = groups == 2 ? 2 : std::min(3, std::max(1, most * c / sms + (most * c % sms > sms / 2)));       // groups on a multiprocessor that is full
+            auto round = [&](long long t) { return times[groups == 1 && t <= alone ? 1 : groups == 1 && t <= 2 * alone ? std::min(2, dense) : dense]; };
+            const long long full = tiles / most, rest = tiles % most;
+            const double each = (full * times[dense] + (rest == 0 ? 0.0 : full > 0 && c == 1 && groups == 1 && rest <= alone ? 1.8 : round(rest))) * (groups == 2 ? 1.05 : 1.0);
+            const double us = 2.0 + ceil_div(halves, vr) * (each * half + (vr > 1 ? 1.5 * (full + (rest > 0)) : 0.0));
+            if (least == 0.0 || us < least) least = us, best = TilePlan{TM, groups, c};
+        }
+}
+TilePlan tile_plan(int M, int N, int K, bool vec) {
+    if (g_forced_tile.tm > 0 && vec) return g_forced_tile;
+    TilePlan best{8, 1, 1};
+    double least = 0.0;
+    consider<4>(M, N, K, vec, best, least);
+    consider<8>(M, N, K, vec, best, least);
+    if (vec) {
+        consider<6>(M, N, K, vec, best, least);
+        consider<10>(M, N, K, vec, best, least);
+    }
+    return best;
 }
 
 // Row-major [rows, K] float32 in tiles of box_rows x 32, 128-byte swizzle, zeros outside.
@@ -430,26 +546,54 @@ int launch_stream(const float* a, const float* w, const float* bias, float* out,
     return li_check_launch("linear (float32, few rows)");
 }
 
-template <int TM, bool kVec>
-int launch_tile(const float* a, const float* w, const float* bias, float* out, int M, int N, int K, cudaStream_t stream) {
+template <int TM, int kGroups, bool kVec>
+int launch_tile(const float* a, const float* w, const float* bias, float* out, int M, int N, int K, int c, cudaStream_t stream) {
     const long long tiles = ceil_div_ll(M, 8 * TM) * ceil_div_ll(N, kBN);
     LI_REQUIRE(tiles <= 2147483647LL, "linear: M=%d, N=%d are too large for one launch", M, N);
-    const int c = tile_cluster(tiles, ceil_div(K, kSegment));
-    const size_t most = sizeof(TileSmem<TM>) + (TM - 1) * sizeof(float4) * kThreadsT;      // room for a cluster of two
-    const size_t smem = sizeof(TileSmem<TM>) + (c > 1 ? (ceil_div(2 * TM, c) - 1) * sizeof(float4) * kThreadsT : 0);
+    using Smem = TileSmem<TM, kGroups>;
+    const size_t most = tile_shared<TM, kGroups>(1), smem = tile_shared<TM, kGroups>(c);
+    static_assert(sizeof(Smem) + (2 * TM / kGroups - 1) * sizeof(float4) * kThreadsT * kGroups <= (kGroups == 1 ? 113 : 227) * 1024, "a block's shared memory");
     static LiOncePerDevice raised;
-    cudaError_t e = li_raise_shared(raised, (const void*)f32_tile_kernel<TM, kVec>, most);
+    cudaError_t e = li_raise_shared(raised, (const void*)f32_tile_kernel<TM, kGroups, kVec>, most);
     if (e != cudaSuccess) return li_fail("linear (float32): cannot raise shared memory to %zu: %s", most, cudaGetErrorString(e));
-    li_launch_pdl(f32_tile_kernel<TM, kVec>, dim3((unsigned)tiles, 1, c), dim3(kThreadsT), smem, stream, dim3(1, 1, c), a, w, bias, out, M, N, K);
+    li_launch_pdl(f32_tile_kernel<TM, kGroups, kVec>, dim3((unsigned)tiles, 1, c), dim3(kThreadsT * kGroups), smem, stream, dim3(1, 1, c), a, w, bias, out,
+                  M, N, K, N % 4 == 0 && (uintptr_t)out % 16 == 0);
     return li_check_launch("linear (float32)");
 }
 
 template <bool kVec>
 int tile_of(const float* a, const float* w, const float* bias, float* out, int M, int N, int K, cudaStream_t stream) {
-    return M <= 32 ? launch_tile<4, kVec>(a, w, bias, out, M, N, K, stream) : launch_tile<8, kVec>(a, w, bias, out, M, N, K, stream);
+    const TilePlan p = tile_plan(M, N, K, kVec);
+    if constexpr (kVec) {
+        if (p.groups == 2) {
+            switch (p.tm) {
+                case 4: return launch_tile<4, 2, true>(a, w, bias, out, M, N, K, p.cluster, stream);
+                case 6: return launch_tile<6, 2, true>(a, w, bias, out, M, N, K, p.cluster, stream);
+                case 8: return launch_tile<8, 2, true>(a, w, bias, out, M, N, K, p.cluster, stream);
+                default: return launch_tile<10, 2, true>(a, w, bias, out, M, N, K, p.cluster, stream);
+            }
+        }
+        if (p.tm == 6) return launch_tile<6, 1, true>(a, w, bias, out, M, N, K, p.cluster, stream);
+        if (p.tm == 10) return launch_tile<10, 1, true>(a, w, bias, out, M, N, K, p.cluster, stream);
+    }
+    return p.tm == 4 ? launch_tile<4, 1, kVec>(a, w, bias, out, M, N, K, p.cluster, stream)
+                     : launch_tile<8, 1, kVec>(a, w, bias, out, M, N, K, p.cluster, stream);
 }
 
 }  // namespace
+
+// This shape for the aligned products of more than 16 rows (rows a thread 4, 6, 8 or 10; groups a block; blocks of a cluster), 0: by
+// size.  Two blocks of a group pair the halves of a segment, so a cluster of groups of one is 1 or even.  For tests and measurements.
+LI_EXPORT int li_linear_f32_force_tile(int tm, int groups, int cluster) {
+    if (tm == 0) {
+        g_forced_tile = TilePlan{0, 0, 0};
+        return 0;
+    }
+    LI_REQUIRE((tm == 4 || tm == 6 || tm == 8 || tm == 10) && (groups == 1 || groups == 2) && cluster >= 1 && cluster <= kMaxCluster &&
+                   (groups == 2 || cluster == 1 || cluster % 2 == 0), "linear (float32): no tile of %d rows a thread, %d groups, cluster %d", tm, groups, cluster);
+    g_forced_tile = TilePlan{tm, groups, cluster};
+    return 0;
+}
 
 int li_linear_f32(const float* a, const float* w, const float* bias, float* out, int M, int N, int K, cudaStream_t stream) {
     const bool vec = K % 4 == 0 && (uintptr_t)a % 16 == 0 && (uintptr_t)w % 16 == 0;

@@ -281,6 +281,15 @@ int li_linear_gemv_static(const void* a, const void* w, const float* bias, void*
  * a cluster holds them. */
 void li_gemv_tcgen05_force_ksplit(int n);
 
+/* ---- gemm_f32.cu ---- */
+/* Tests and measurements: force the tiles of the aligned float32 products of more than 16 rows (rows a thread 4, 6, 8 or 10; groups of
+ * threads a block 1 or 2; blocks of a cluster), 0: by size. */
+int li_linear_f32_force_tile(int tm, int groups, int cluster);
+
+/* Tests: how a product of M <= 64 rows is cut: the splits of k, and how many of them form a cluster; with deep (needs a device)
+ * whether its plain form takes the deep pipeline (all three in host memory). */
+int li_gemv_tcgen05_plan(int M, int N, int K, int* splits, int* cluster, int* deep);
+
 /* ---- linear.cu ---- */
 /* out[M, N] = a[M, K] w[N, K]^T (+ bias), epilogue 0 none / 1 SwiGLU, 2 bounded unit, 3 GEGLU over interleaved gate|up rows; float32 in
  * float32 out, or bfloat16 in, bfloat16 or float out. */

@@ -201,3 +201,22 @@ def test_scores_of_minus_infinity(lost, tokens):
     got = out.double().cpu().view(tokens, nh, dh)
     assert torch.equal(got.isnan(), exact.isnan())
     assert float((got - exact).nan_to_num().abs().max()) <= 2e-5
+
+
+@pytest.mark.parametrize("tile", [(4, 1, 1), (4, 2, 3), (6, 1, 4), (6, 2, 1), (8, 1, 2), (8, 1, 6), (8, 2, 5), (10, 1, 1), (10, 2, 8), (10, 1, 8)], ids=str)
+@pytest.mark.parametrize("M,N,Kd", [(17, 130, 1540), (81, 300, 260), (150, 257, 4612), (97, 1536, 512), (33, 4, 36)])
+def test_product_gives_the_same_bits_in_every_tile(tile, M, N, Kd):
+    """Rows a thread, groups of threads and clusters that share a tile's halves of segments: a token alone, through the streaming kernel,
+    has the bits of all of them."""
+    g = torch.Generator(device="cuda").manual_seed(Kd + M)
+    a, w = torch.randn((M, Kd), generator=g, device="cuda"), torch.randn((N, Kd), generator=g, device="cuda")
+    bias = torch.randn(N, generator=g, device="cuda")
+    lib = K().library()
+    by_size = product(a, w, bias)
+    assert lib.li_linear_f32_force_tile(*tile) == 0
+    try:
+        assert torch.equal(product(a, w, bias), by_size)
+    finally:
+        lib.li_linear_f32_force_tile(0, 0, 0)
+    assert torch.equal(product(a[M - 1:].contiguous(), w, bias), by_size[M - 1:])
+    assert lib.li_linear_f32_force_tile(8, 1, 3) != 0 and lib.li_linear_f32_force_tile(5, 1, 1) != 0       # segments' halves come in pairs
