@@ -13,6 +13,7 @@
 // Scores, exponentials (full precision), sums and weighted values are float.
 //
 // All of AttentionOptions but several maps a query row (attention.cu sends those to the general kernel).
+#define LI_PDL_KIND 4
 #include "attention_options.h"
 #include "common.cuh"
 
@@ -54,6 +55,8 @@ attention_f32_kernel(const float* __restrict__ qkv, float* __restrict__ out, con
     const int kvh = (int)blockIdx.y / groups, h0 = kvh * G + ((int)blockIdx.y % groups) * NH;
     const int heads = min(NH, kvh * G + G - h0);
 
+    // (launched as a dependent, and lets the next one come: the o product asks for its weights meanwhile)
+    pdl_launch_dependents();
     const int s = seq_of_token[t], p = positions[t];
     const int lo = first_seen_key(p, window, opt.chunk);
     const int keep_first = window > 0 ? opt.keep_first : 0;
@@ -63,6 +66,7 @@ attention_f32_kernel(const float* __restrict__ qkv, float* __restrict__ out, con
     const int* bt = block_table + (size_t)s * max_blocks;
     const int quads = dh >> 2;
 
+    pdl_wait();
     const size_t row = opt.q_ld > 0 ? opt.q_ld : (nh + 2 * nkv) * dh;
     for (int e = tid; e < NH * dh; e += kThreads) q_sm[e] = e < heads * dh ? qkv[t * row + (size_t)h0 * dh + e] : 0.0f;
     __syncthreads();
@@ -278,19 +282,9 @@ int launch(const void* qkv, void* out, const void* kcache, const void* vcache, c
     static LiOncePerDevice raised;
     cudaError_t e = li_raise_shared(raised, (const void*)attention_f32_kernel<NH>, shared_floats(kMaxDim) * sizeof(float));
     if (e != cudaSuccess) return li_fail("attention (float32): cannot raise shared memory: %s", cudaGetErrorString(e));
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(T, nkv * groups, csize);
-    cfg.blockDim = dim3(kThreads);
-    cfg.dynamicSmemBytes = shared_floats(dh) * sizeof(float);
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = csize;
-    cfg.attrs = attr;
-    cfg.numAttrs = csize > 1 ? 1 : 0;
-    cudaLaunchKernelEx(&cfg, attention_f32_kernel<NH>, (const float*)qkv, (float*)out, (const float*)kcache, (const float*)vcache, block_table, max_blocks,
-                       seq_of_token, positions, nh, nkv, dh, page_size, num_pages, scale, window, csize, opt);
+    li_launch_pdl(attention_f32_kernel<NH>, dim3(T, nkv * groups, csize), dim3(kThreads), shared_floats(dh) * sizeof(float), stream, dim3(1, 1, csize),
+                  (const float*)qkv, (float*)out, (const float*)kcache, (const float*)vcache, block_table, max_blocks, seq_of_token, positions, nh, nkv, dh,
+                  page_size, num_pages, scale, window, csize, opt);
     return li_check_launch("attention (float32)");
 }
 

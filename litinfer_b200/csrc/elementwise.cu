@@ -340,9 +340,9 @@ LI_EXPORT int li_swiglu(const void* gate_up, void* out, int dtype, int T, int I,
     const long long n = (long long)T * I;
     if (n == 0) return 0;
     if (dtype == LI_F32)
-        swiglu_kernel<float><<<grid_for(n, 256), 256, 0, stream>>>((const float*)gate_up, (float*)out, I, n);
+        li_launch_pdl(swiglu_kernel<float>, dim3(grid_for(n, 256)), dim3(256), 0, stream, (const float*)gate_up, (float*)out, I, n);
     else if (dtype == LI_BF16)
-        swiglu_kernel<bf16><<<grid_for(n, 256), 256, 0, stream>>>((const bf16*)gate_up, (bf16*)out, I, n);
+        li_launch_pdl(swiglu_kernel<bf16>, dim3(grid_for(n, 256)), dim3(256), 0, stream, (const bf16*)gate_up, (bf16*)out, I, n);
     else
         return li_fail("swiglu: unknown dtype %d", dtype);
     return li_check_launch("swiglu");
