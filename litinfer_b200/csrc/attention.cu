@@ -13,8 +13,7 @@
 //                                       query rows for each head and read its keys once per query head.
 //   sizes those refuse               -> general kernel
 //
-// Every kernel takes all of AttentionOptions (the tcgen05 tiles: no cap together with a penalty linear in the distance, at most
-// two maps a query row).
+// Every kernel takes all of AttentionOptions (the tcgen05 tiles: at most two maps a query row).
 #include "attention_options.h"
 #include "common.cuh"
 

@@ -81,10 +81,10 @@ __device__ __forceinline__ float tanh_small(float x) {
 }
 
 // kForm: what becomes of the scores before the mask and the softmax.  kCapped: cap * tanh(s / cap) (`softcap` > 0); kSloped:
-// slopes[h] * (p - key) is taken off.  maps > 1: a query row of DH elements
+// slopes[h] * (p - key) is taken off; both: in this order.  maps > 1: a query row of DH elements
 // stands for that many heads, each with a part of it (attention_mma.cuh: ScoreMod): a head's product S takes the k-steps of
 // its own part only, and with head_dim 128 and two maps only that part's panel of the keys is brought in.
-enum { kAsTheyAre = 0, kCapped = 1, kSloped = 2 };
+enum { kAsTheyAre = 0, kCapped = 1, kSloped = 2, kCappedSloped = kCapped | kSloped };
 
 template <int DH, int kForm>
 __global__ void __launch_bounds__(kThreads, 1)
@@ -298,8 +298,8 @@ prefill_attention_tc_kernel(const bf16* __restrict__ qkv, long long row_elems, c
         const int lo = first_seen_key(p, window, opt.chunk);
         // (changed scores are brought to base-2 units as they are changed, and the factor below is 1)
         const float scale_log2 = kForm != kAsTheyAre ? 1.0f : scale * 1.4426950408889634f;
-        [[maybe_unused]] const float cap_in = kForm == kCapped ? scale / opt.softcap : 0.0f, cap_out = opt.softcap * 1.4426950408889634f;
-        [[maybe_unused]] const float slope2 = kForm == kSloped ? opt.slopes[h] * 1.4426950408889634f : 0.0f;
+        [[maybe_unused]] const float cap_in = (kForm & kCapped) ? scale / opt.softcap : 0.0f, cap_out = opt.softcap * 1.4426950408889634f;
+        [[maybe_unused]] const float slope2 = (kForm & kSloped) ? opt.slopes[h] * 1.4426950408889634f : 0.0f;
         // m: the maximum the exponentials are taken against.  It follows the true maximum lazily: only when that has grown by
         // more than kLazy (in powers of two) is the output so far, which accumulates in tensor memory, scaled down to the
         // new one.  Until then the probabilities may reach 2^kLazy, which costs bfloat16 and the float sums nothing, and
@@ -342,7 +342,7 @@ prefill_attention_tc_kernel(const bf16* __restrict__ qkv, long long row_elems, c
 #pragma unroll
                 for (int i = 0; i < HK; ++i) v[i] = fmaf(v[i], factor, fmaf(slope2, (float)i, first));
             }
-            if constexpr (kForm == kCapped) {
+            if constexpr ((kForm & kCapped) != 0) {
                 // cap * tanh(s scale / cap) in base-2 units: small arguments by a polynomial on the multiply-add pipe, and if
                 // any of the thread's is larger all of them through the exponential
                 float top = 0.0f;
@@ -354,6 +354,11 @@ prefill_attention_tc_kernel(const bf16* __restrict__ qkv, long long row_elems, c
                 } else {
 #pragma unroll
                     for (int i = 0; i < HK; ++i) v[i] = tanh_fast(v[i] * cap_in) * cap_out;
+                }
+                if constexpr ((kForm & kSloped) != 0) {
+                    const float first = slope2 * (float)(key0 - p);
+#pragma unroll
+                    for (int i = 0; i < HK; ++i) v[i] += fmaf(slope2, (float)i, first);
                 }
             }
             const bool whole = (key0 >= lo || key0 + HK <= keep) && key0 + HK - 1 <= p;
@@ -621,7 +626,7 @@ bool li_attention_tcgen05_accepts(const void* qkv, const void* kcache, const voi
 
 // which options these tiles take (the others are the mma.sync tiles' business)
 bool li_attention_tcgen05_takes(const AttentionOptions& opt) {
-    return opt.maps <= 2 && !(opt.softcap > 0.0f && opt.slopes != nullptr) && opt.q_ld % 8 == 0 &&
+    return opt.maps <= 2 && opt.q_ld % 8 == 0 &&
            (opt.gate == nullptr || opt.gate_elements == 0 || (opt.gate_ld % 8 == 0 && (uintptr_t)opt.gate % 16 == 0));
 }
 
@@ -629,14 +634,16 @@ int li_attention_tcgen05(const void* qkv, void* out, const void* kcache, const v
                          const int* q_start, const int* ctx_lens, int T, int S, int nh, int nkv, int dh, int page_size, int num_pages,
                          float scale, int window, int max_q_len, int skip_single, const int* units, int unit_slots, const AttentionOptions& opt, cudaStream_t stream) {
     LI_REQUIRE(opt.maps == 1 || opt.maps == 2, "attention (tcgen05): takes one or two maps a query row, not %d", opt.maps);
-    LI_REQUIRE(li_attention_tcgen05_takes(opt), "attention (tcgen05): a cap together with slopes, or rows that are not on 16-byte boundaries");
+    LI_REQUIRE(li_attention_tcgen05_takes(opt), "attention (tcgen05): more than two maps, or rows that are not on 16-byte boundaries");
     LI_REQUIRE(li_attention_tcgen05_accepts(qkv, kcache, vcache, nh, nkv, dh, page_size),
                "attention (tcgen05): refuses heads=%d/%d head_dim=%d page=%d (head_dim 64 or 128, pages a multiple of 16)", nh, nkv, dh, page_size);
     LI_REQUIRE(scale > 0.0f, "attention (tcgen05): the scale must be positive");
 #define LI_CASE(D, FORM)                                                                                                                       \
     launch<D, FORM>(qkv, out, kcache, vcache, block_table, max_blocks, q_start, ctx_lens, T, S, nh, nkv, page_size, num_pages, scale, window, \
                    max_q_len, skip_single, units, unit_slots, opt, stream)
-    if (dh == 64) return opt.softcap > 0.0f ? LI_CASE(64, kCapped) : opt.slopes ? LI_CASE(64, kSloped) : LI_CASE(64, kAsTheyAre);
-    return opt.softcap > 0.0f ? LI_CASE(128, kCapped) : opt.slopes ? LI_CASE(128, kSloped) : LI_CASE(128, kAsTheyAre);
+    const bool capped = opt.softcap > 0.0f, sloped = opt.slopes != nullptr;
+    if (dh == 64)
+        return capped && sloped ? LI_CASE(64, kCappedSloped) : capped ? LI_CASE(64, kCapped) : sloped ? LI_CASE(64, kSloped) : LI_CASE(64, kAsTheyAre);
+    return capped && sloped ? LI_CASE(128, kCappedSloped) : capped ? LI_CASE(128, kCapped) : sloped ? LI_CASE(128, kSloped) : LI_CASE(128, kAsTheyAre);
 #undef LI_CASE
 }

@@ -263,6 +263,17 @@ int li_tcgen05_tokens_force_width(int width);
 /* Tests: whether the product of M rows has its tokens as columns. */
 int li_tcgen05_takes_tokens(int M, int N, int K);
 
+/* ---- scan_chunks.cu ---- */
+/* The two passes over chunks of at most 64 tokens as products of small matrices; mode 1: end states from zeros (and, state space, the
+ * chunks' decays), 2: outputs.  The others of li_decay_scan and li_ssm_scan are theirs. */
+int li_decay_chunks_accepts(int length, int d);
+int li_ssm_chunks_accepts(int length, int heads, int P, int N, int groups);
+int li_decay_chunks(const void* qkv, int dtype, int stride, int q_off, int k_off, int v_off, const float* decay, float* out, int chunks,
+    int heads, int d, int dv, const int* seg, int mode, float* chunk_state, cudaStream_t stream);
+int li_ssm_chunks(const void* xbc, int dtype, int C, const void* dt_raw, int dt_stride, const float* dt_bias, const float* A_log,
+    const float* D, float* y, int chunks, int heads, int P, int N, int groups, const int* seg, int mode, float* chunk_state, float*
+    chunk_decay, cudaStream_t stream);
+
 /* ---- attention_f32.cu ---- */
 /* Tests: how many blocks share a token's keys in the float32 attention of a step of T tokens. */
 int li_attention_f32_blocks(int T, int nh, int nkv, int dh);

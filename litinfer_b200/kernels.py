@@ -774,7 +774,7 @@ class ScanChunks:
             for b in range(lo, hi, length):
                 seg.append((b, min(hi, b + length), len(seg), int(slot)))
             runs.append((first, len(seg) - first, int(slot)))
-        self.count, self.nruns = len(seg), len(runs)
+        self.count, self.nruns, self.length = len(seg), len(runs), int(length)
         self.seg = torch.tensor(seg, dtype=torch.int32).to(device)
         self.runs = torch.tensor(runs, dtype=torch.int32).to(device)
 
@@ -811,7 +811,13 @@ def ssm_scan(xbc: torch.Tensor, proj: torch.Tensor, dt_col: int, dt_bias: torch.
         raise KernelError("ssm_scan: the state or the projection is too small")
     dt_ptr = ctypes.c_void_p(proj.data_ptr() + dt_col * proj.element_size())
 
+    small = chunks is not None and library().li_ssm_chunks_accepts(_i(chunks.length), _i(heads), _i(head_dim), _i(state_size), _i(groups))
+
     def run(seg, n, mode, cstate, cdecay):
+        if small and mode:
+            _check(library().li_ssm_chunks(_p(xbc), _i(_dt(xbc)), _i(C), dt_ptr, _i(proj.shape[1]), _p(dt_bias), _p(A_log), _p(D), _p(y32), _i(n), _i(heads),
+                                           _i(head_dim), _i(state_size), _i(groups), _p(seg), _i(mode), _p(cstate), _p(cdecay), _stream(y32)), "ssm_scan")
+            return
         _check(library().li_ssm_scan(_p(xbc), _i(_dt(xbc)), _i(C), dt_ptr, _i(proj.shape[1]), _p(dt_bias), _p(A_log), _p(D), st, stride,
                                      _p(q_start), _p(slots), _p(y32), _i(n), _i(heads), _i(head_dim), _i(state_size), _i(groups),
                                      _p(seg), _i(mode), _p(cstate), _p(cdecay), _stream(y32)), "ssm_scan")
@@ -841,7 +847,13 @@ def decay_scan(qkv: torch.Tensor, q_col: int, k_col: int, v_col: int, decay: tor
     if heads * dim * vdim > state.shape[1]:
         raise KernelError("decay_scan: the state is too small")
 
+    small = chunks is not None and library().li_decay_chunks_accepts(_i(chunks.length), _i(dim))
+
     def run(seg, n, mode, cstate):
+        if small and mode:
+            _check(library().li_decay_chunks(_p(qkv), _i(_dt(qkv)), _i(qkv.shape[1]), _i(q_col), _i(k_col), _i(v_col), _p(decay), _p(out32), _i(n), _i(heads),
+                                             _i(dim), _i(vdim), _p(seg), _i(mode), _p(cstate), _stream(out32)), "decay_scan")
+            return
         _check(library().li_decay_scan(_p(qkv), _i(_dt(qkv)), _i(qkv.shape[1]), _i(q_col), _i(k_col), _i(v_col), _p(decay), st, stride, _p(q_start),
                                        _p(slots), _p(out32), _i(n), _i(heads), _i(dim), _i(vdim), _p(seg), _i(mode), _p(cstate), _stream(out32)),
                "decay_scan")

@@ -622,3 +622,69 @@ def test_stream_norm_and_gated_kernels(dtype):
                     fused = torch.empty_like(ref)
                     K.linear_with(which, a_in, inter, None, fused, epilogue="glu_clamped", epilogue_params=params)
                     _close(fused, ref, dtype, f"gated unit as the epilogue of {which}, {M} rows")
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("heads,d,dv", [(3, 128, 128), (2, 64, 200), (5, 100, 36), (1, 4, 128)])
+def test_decay_scan_in_chunks_as_products(heads, d, dv, dtype):
+    """Chunks of one token, of 64, of 63 and 65 (the general passes); heads that decay at once and not at all; values that are no finite
+    numbers reach the tokens behind them alone."""
+    import kernel_refs as R
+    from litinfer_b200 import kernels as K
+
+    dev, dt = torch.device("cuda:0"), _dt(dtype)
+    torch.manual_seed(heads * d + dv)
+    lens = [129, 64, 1, 63, 200]
+    q_start = torch.tensor([0] + list(torch.tensor(lens).cumsum(0)), dtype=torch.int32, device=dev)
+    T = sum(lens)
+    slots = torch.tensor([3, 0, 2, 1, 4], dtype=torch.int32, device=dev)
+    qkv = torch.randn(T, 2 * heads * d + heads * dv + 7, device=dev).to(dt)
+    decay = torch.tensor([0.9, 1.0, 0.0, 0.999, 0.5][:heads], dtype=torch.float32, device=dev)
+    state0 = 0.3 * torch.randn(5, heads * d * dv, device=dev)
+    at = (3, 3 + heads * d, 3 + 2 * heads * d)
+    assert K.library().li_decay_chunks_accepts(64, d) == 1 and K.library().li_decay_chunks_accepts(65, d) == 0
+    ref_s, ref_o = state0.clone(), torch.zeros(T, heads * dv, device=dev)
+    R.decay_scan(qkv, *at, decay, ref_s, q_start, slots, ref_o, heads, d, dv)
+    for length in (64, 17, 65):
+        s, o = state0.clone(), torch.full((T, heads * dv), 7.0, device=dev)
+        K.decay_scan(qkv, *at, decay, s, q_start, slots, o, heads, d, dv, chunks=K.ScanChunks(q_start.tolist(), slots.tolist(), dev, length))
+        _close(o, ref_o, "float32", f"outputs, chunks of {length}")
+        _close(s, ref_s, "float32", f"states, chunks of {length}")
+    bad = qkv.clone()
+    bad[40, at[2] + 5], bad[150, at[2]] = float("inf"), float("nan")
+    o = torch.zeros(T, heads * dv, device=dev)
+    K.decay_scan(bad, *at, decay, state0.clone(), q_start, slots, o, heads, d, dv, chunks=K.ScanChunks(q_start.tolist(), slots.tolist(), dev))
+    _close(o[:40], ref_o[:40], "float32", "tokens before an infinite value")
+    _close(o[129:150], ref_o[129:150], "float32", "tokens before a value that is no number")
+    assert not torch.isfinite(o[40, 5]) and torch.isnan(o[150, 0])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("heads,P,N,groups", [(4, 64, 128, 2), (3, 128, 60, 3), (2, 64, 4, 1), (6, 64, 96, 1)])
+def test_ssm_scan_in_chunks_as_products(heads, P, N, groups, dtype):
+    """Two heads of 64 a block or one of 128; a head whose decays leave nothing, and one whose step sizes are large."""
+    import kernel_refs as R
+    from litinfer_b200 import kernels as K
+
+    dev, dt = torch.device("cuda:0"), _dt(dtype)
+    torch.manual_seed(heads * P + N)
+    lens = [130, 64, 1, 63]
+    q_start = torch.tensor([0] + list(torch.tensor(lens).cumsum(0)), dtype=torch.int32, device=dev)
+    T = sum(lens)
+    slots = torch.tensor([2, 0, 1, 3], dtype=torch.int32, device=dev)
+    C = heads * P + 2 * groups * N
+    xbc = (0.5 * torch.randn(T, C, device=dev)).to(dt)
+    proj = torch.randn(T, 5 + heads, device=dev).to(dt)
+    dt_bias, A_log, D = (0.5 * torch.randn(heads, device=dev) for _ in range(3))
+    A_log[0], dt_bias[-1] = 80.0, 6.0
+    state0 = 0.3 * torch.randn(4, heads * P * N, device=dev)
+    assert K.library().li_ssm_chunks_accepts(64, heads, P, N, groups) == 1
+    ref_s, ref_y = state0.clone(), torch.zeros(T, heads * P, device=dev)
+    R.ssm_scan(xbc, proj, 5, dt_bias, A_log, D, ref_s, q_start, slots, ref_y, heads, P, N, groups)
+    for length in (64, 17, 65):
+        s, y = state0.clone(), torch.full((T, heads * P), 7.0, device=dev)
+        K.ssm_scan(xbc, proj, 5, dt_bias, A_log, D, s, q_start, slots, y, heads, P, N, groups, chunks=K.ScanChunks(q_start.tolist(), slots.tolist(), dev, length))
+        _close(y, ref_y, "float32", f"outputs, chunks of {length}")
+        _close(s, ref_s, "float32", f"states, chunks of {length}")
