@@ -253,3 +253,25 @@ def test_rotation_with_tokens_as_columns(heads, tokens, first):
         assert torch.equal(got == 3.0, ref == 3.0)
         T.close(got, ref, torch.bfloat16, "rotation with tokens as columns")
     assert K().library().li_tcgen05_status() == 0
+
+
+@pytest.mark.parametrize("window", [None, 150])
+@pytest.mark.parametrize("dh", [64, 128])
+def test_portions_with_a_cap_and_slopes_on_tensor_memory_tiles(dh, window):
+    """Both changes of a score at once, against the tiles that took them alone before: small scores and ones beyond the cap."""
+    from test_f32_gpu import on_device
+
+    nh, nkv = 6, 2
+    c = on_device(T.make_attention_case([130, 64, 5], [700, 64, 333], nh, nkv, dh, 16, torch.float32, seed=dh))
+    for k in ("qkv", "k_cache", "v_cache"):
+        c[k] = torch.nan_to_num(c[k]).to(torch.bfloat16)
+    slopes = torch.tensor([2.0 ** -(h + 1) for h in range(nh)], device="cuda")
+    outs = []
+    for scale in (dh ** -0.5, 3.0):
+        for implementation in ("prefill_tcgen05", "prefill"):
+            out = torch.full((199, nh * dh), float("nan"), dtype=torch.bfloat16, device="cuda")
+            K().paged_attention(c["qkv"], out, c["k_cache"], c["v_cache"], c["block_table"], c["q_start"], c["ctx_lens"], c["seq_of_token"], c["positions"], nh,
+                                nkv, dh, scale, window, 130, 700, softcap=5.0, slopes=slopes, implementation=implementation)
+            outs.append(out)
+        T.close(outs[-2], outs[-1], torch.bfloat16, f"cap and slopes, scale {scale}")
+    assert K().library().li_tcgen05_status() == 0
