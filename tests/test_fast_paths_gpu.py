@@ -275,3 +275,34 @@ def test_portions_with_a_cap_and_slopes_on_tensor_memory_tiles(dh, window):
             outs.append(out)
         T.close(outs[-2], outs[-1], torch.bfloat16, f"cap and slopes, scale {scale}")
     assert K().library().li_tcgen05_status() == 0
+
+
+@pytest.mark.parametrize("M", [1, 8, 9, 16])
+@pytest.mark.parametrize("N,Kd", [(2384, 1536), (2369, 2048), (4800, 1544), (2400, 1992)])
+def test_streaming_product_of_one_round_gives_the_bits_of_its_parts(M, N, Kd):
+    """More CTAs than multiprocessors, whose warps hold all of their weights at once, against parts of the matrix that go in one wave."""
+    g = torch.Generator(device="cuda").manual_seed(N + Kd + M)
+    a, w = (torch.randn(n, Kd, generator=g, device="cuda").to(torch.bfloat16) for n in (M, N))
+    bias = torch.randn(N, generator=g, device="cuda")
+    outs = {}
+    for dt in (torch.bfloat16, torch.float32):
+        whole = torch.full((M, N), 7.0, device="cuda", dtype=dt)
+        K().linear_with("gemv", a, w, bias, whole)
+        for n0 in range(0, N, 1200):
+            n1 = min(n0 + 1200, N)
+            part = torch.full((M, n1 - n0), 7.0, device="cuda", dtype=dt)
+            K().linear_with("gemv", a, w[n0:n1], bias[n0:n1].clone(), part)
+            assert torch.equal(whole[:, n0:n1], part)
+        outs[dt] = whole
+    # products are exact in float; K + 32 roundings of partial sums that the sum of magnitudes bounds
+    exact = a.double() @ w.double().T + bias.double()
+    bound = (Kd + 32) * 2.0 ** -24 * (a.double().abs() @ w.double().abs().T + bias.double().abs())
+    assert bool(((outs[torch.float32].double() - exact).abs() <= bound).all())
+    if N % 16 == 0:
+        whole = torch.full((M, N // 2), 7.0, device="cuda", dtype=torch.bfloat16)
+        K().linear_with("gemv", a, w, None, whole, epilogue="swiglu")
+        for n0 in range(0, N, 1200):
+            n1 = min(n0 + 1200, N)
+            part = torch.full((M, (n1 - n0) // 2), 7.0, device="cuda", dtype=torch.bfloat16)
+            K().linear_with("gemv", a, w[n0:n1], None, part, epilogue="swiglu")
+            assert torch.equal(whole[:, n0 // 2:n1 // 2], part)
