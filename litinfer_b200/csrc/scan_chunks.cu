@@ -8,10 +8,12 @@
 //     outputs     o_t[c]  = w(t, start) sum over i of q_t[i] S[c, i]  +  sum over s <= t of w(t, s) (q_t . k_s) v_s[c]
 // that is products of a chunk's rows with each other, with the state it starts from and with its values, all in float with packed
 // multiply-adds.  A block of 256 threads takes a chunk of a head's 128 value columns (two heads of 64, which share B and C); 8 x 8
-// outputs a thread for the end state, 4 x 8 for the outputs, operands along the summed index so that pairs of it are the packed
+// outputs a thread for the end state, 4 x 8 for the outputs (the two passes: 18 and 40 us, 24 and 58), operands along the summed index so that pairs of it are the packed
 // pairs.  What bounds them is shared-memory reads (a 16-byte read of a warp takes four cycles, whatever the lanes share).
 // w comes from sums of logarithms in double, or from powers of the head's one decay.
 #include "common.cuh"
+
+#include <type_traits>
 
 namespace {
 
@@ -276,127 +278,135 @@ chunk_output_kernel(const Source<T> src, const int* __restrict__ seg, const floa
     };
     ask(0);
     __syncthreads();
-    {
-        // scores of a token with the earlier ones, weighted: blocks of sixteen tokens on and below the diagonal
-        unsigned long long acc[4][4];
+    // Blocks of sixteen tokens that the chunk has: the last chunk of a portion may have few (777 tokens of 48 heads of 64: 312 blocks, 24 of
+    // them of nine tokens, for 296 places: 68 - 79 -> 58 us).
+    auto with_blocks = [&](auto blocks) {
+        constexpr int A = decltype(blocks)::value;
+        {
+            // scores of a token with the earlier ones, weighted: blocks of sixteen tokens on and below the diagonal
+            unsigned long long acc[A][A];
 #pragma unroll
-        for (int a = 0; a < 4; ++a)
+            for (int a = 0; a < A; ++a)
 #pragma unroll
-            for (int b = 0; b < 4; ++b) acc[a][b] = 0ull;
-        const int quads = (src.d + 3) >> 2;
+                for (int b = 0; b < A; ++b) acc[a][b] = 0ull;
+            const int quads = (src.d + 3) >> 2;
 #pragma unroll 2
-        for (int i = 0; i < quads; ++i) {
-            ulonglong2 q[4];
+            for (int i = 0; i < quads; ++i) {
+                ulonglong2 q[A];
 #pragma unroll
-            for (int a = 0; a < 4; ++a) q[a] = pair4(sm.a + (ty + 16 * a) * kRow + 4 * i);
+                for (int a = 0; a < A; ++a) q[a] = pair4(sm.a + (ty + 16 * a) * kRow + 4 * i);
 #pragma unroll
-            for (int b = 0; b < 4; ++b) {
-                const ulonglong2 k = pair4(sm.b + (tx + 16 * b) * kRow + 4 * i);
+                for (int b = 0; b < A; ++b) {
+                    const ulonglong2 k = pair4(sm.b + (tx + 16 * b) * kRow + 4 * i);
 #pragma unroll
-                for (int a = b; a < 4; ++a) fma2(acc[a][b], q[a].x, k.x), fma2(acc[a][b], q[a].y, k.y);
-            }
-        }
-#pragma unroll
-        for (int a = 0; a < 4; ++a)
-#pragma unroll
-            for (int b = 0; b <= a; ++b) {
-                const int t = ty + 16 * a, s = tx + 16 * b;
-                const float2 x = unpack2(acc[a][b]);
-#pragma unroll
-                for (int hh = 0; hh < OutputSmem<kSsm>::kHeads; ++hh)
-                    if (hh < c.heads_here) sm.p[hh][t * kTokRow + s] = s <= t && t < c.n ? (x.x + x.y) * weight<kSsm>(sm.w, hh, t, s) : 0.0f;
-            }
-    }
-    unsigned long long acc[4][8];
-#pragma unroll
-    for (int a = 0; a < 4; ++a)
-#pragma unroll
-        for (int b = 0; b < 8; ++b) acc[a][b] = 0ull;
-    // queries with the state the chunk starts from
-    const int pieces = (src.d + kPiece - 1) / kPiece;
-    for (int piece = 0; piece < pieces; ++piece) {
-        __syncthreads();                                   // the keys, or the piece before, have been used up
-#pragma unroll
-        for (int r = 0; r < 4; ++r) {
-            const int e = tid + kThreads * r;
-            *reinterpret_cast<float4*>(sm.b + (e >> 3) * kPieceRow + 4 * (e & 7)) = ahead[r];
-        }
-        __syncthreads();
-        if (piece + 1 < pieces) ask(piece + 1);
-#pragma unroll 2
-        for (int i = 0; i < kPiece / 4; ++i) {
-            ulonglong2 q[4];
-#pragma unroll
-            for (int a = 0; a < 4; ++a) q[a] = pair4(sm.a + (ty + 16 * a) * kRow + piece * kPiece + 4 * i);
-#pragma unroll
-            for (int b = 0; b < 8; ++b) {
-                const ulonglong2 s = pair4(sm.b + (tx + 16 * b) * kPieceRow + 4 * i);
-#pragma unroll
-                for (int a = 0; a < 4; ++a) fma2(acc[a][b], q[a].x, s.x), fma2(acc[a][b], q[a].y, s.y);
-            }
-        }
-    }
-    const int second = kSsm ? src.dv : kCols;              // from this column on the tile's second head
-#pragma unroll
-    for (int a = 0; a < 4; ++a)
-#pragma unroll
-        for (int b = 0; b < 8; ++b) {
-            const float2 x = unpack2(acc[a][b]);
-            const int t = ty + 16 * a, hh = tx + 16 * b >= second ? 1 : 0;
-            acc[a][b] = pack2(t < c.n ? (x.x + x.y) * weight_from_start<kSsm>(sm.w, kSsm ? hh : 0, t) : 0.0f, 0.0f);
-        }
-    __syncthreads();                                       // the queries have been used up
-    bool finite = true;
-    stage_rows<T, kSsm>(c.v, src.stride, c.n, c.cols, c.wide(c.v, src.stride), true, [&](int t, int j, const float (&x)[kVec]) {
-#pragma unroll
-        for (int i = 0; i < kVec; ++i) {
-            finite = finite && fabsf(x[i]) < INFINITY;
-            sm.a[(j + i) * kTokRow + t] = x[i];
-        }
-    });
-    // A value that is no finite number must not reach the tokens before it by way of a weight of zero: such a chunk is summed one
-    // by one.
-    const bool one_by_one = __syncthreads_or(!finite);
-    // weighted scores with the values of the tokens
-#pragma unroll
-    for (int sb = 0; sb < 4; ++sb) {
-        if (16 * sb < c.n && !one_by_one) {
-#pragma unroll 1
-            for (int i = 0; i < 4; ++i) {
-                ulonglong2 p[4], p2[4];
-#pragma unroll
-                for (int a = sb; a < 4; ++a) {
-                    p[a] = pair4(sm.p[0] + (ty + 16 * a) * kTokRow + 16 * sb + 4 * i);
-                    if constexpr (kSsm) p2[a] = c.heads_here > 1 ? pair4(sm.p[1] + (ty + 16 * a) * kTokRow + 16 * sb + 4 * i) : p[a];
+                    for (int a = b; a < A; ++a) fma2(acc[a][b], q[a].x, k.x), fma2(acc[a][b], q[a].y, k.y);
                 }
+            }
+#pragma unroll
+            for (int a = 0; a < A; ++a)
+#pragma unroll
+                for (int b = 0; b <= a; ++b) {
+                    const int t = ty + 16 * a, s = tx + 16 * b;
+                    const float2 x = unpack2(acc[a][b]);
+#pragma unroll
+                    for (int hh = 0; hh < OutputSmem<kSsm>::kHeads; ++hh)
+                        if (hh < c.heads_here) sm.p[hh][t * kTokRow + s] = s <= t && t < c.n ? (x.x + x.y) * weight<kSsm>(sm.w, hh, t, s) : 0.0f;
+                }
+        }
+        unsigned long long acc[A][8];
+#pragma unroll
+        for (int a = 0; a < A; ++a)
+#pragma unroll
+            for (int b = 0; b < 8; ++b) acc[a][b] = 0ull;
+        // queries with the state the chunk starts from
+        const int pieces = (src.d + kPiece - 1) / kPiece;
+        for (int piece = 0; piece < pieces; ++piece) {
+            __syncthreads();                                   // the keys, or the piece before, have been used up
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+                const int e = tid + kThreads * r;
+                *reinterpret_cast<float4*>(sm.b + (e >> 3) * kPieceRow + 4 * (e & 7)) = ahead[r];
+            }
+            __syncthreads();
+            if (piece + 1 < pieces) ask(piece + 1);
+#pragma unroll 2
+            for (int i = 0; i < kPiece / 4; ++i) {
+                ulonglong2 q[A];
+#pragma unroll
+                for (int a = 0; a < A; ++a) q[a] = pair4(sm.a + (ty + 16 * a) * kRow + piece * kPiece + 4 * i);
 #pragma unroll
                 for (int b = 0; b < 8; ++b) {
-                    const ulonglong2 v = pair4(sm.a + (tx + 16 * b) * kTokRow + 16 * sb + 4 * i);
+                    const ulonglong2 s = pair4(sm.b + (tx + 16 * b) * kPieceRow + 4 * i);
 #pragma unroll
-                    for (int a = sb; a < 4; ++a) {
-                        const ulonglong2 x = kSsm && b >= 4 ? p2[a] : p[a];      // (two heads are of 64 columns)
-                        fma2(acc[a][b], x.x, v.x), fma2(acc[a][b], x.y, v.y);
+                    for (int a = 0; a < A; ++a) fma2(acc[a][b], q[a].x, s.x), fma2(acc[a][b], q[a].y, s.y);
+                }
+            }
+        }
+        const int second = kSsm ? src.dv : kCols;              // from this column on the tile's second head
+#pragma unroll
+        for (int a = 0; a < A; ++a)
+#pragma unroll
+            for (int b = 0; b < 8; ++b) {
+                const float2 x = unpack2(acc[a][b]);
+                const int t = ty + 16 * a, hh = tx + 16 * b >= second ? 1 : 0;
+                acc[a][b] = pack2(t < c.n ? (x.x + x.y) * weight_from_start<kSsm>(sm.w, kSsm ? hh : 0, t) : 0.0f, 0.0f);
+            }
+        __syncthreads();                                       // the queries have been used up
+        bool finite = true;
+        stage_rows<T, kSsm>(c.v, src.stride, c.n, c.cols, c.wide(c.v, src.stride), true, [&](int t, int j, const float (&x)[kVec]) {
+#pragma unroll
+            for (int i = 0; i < kVec; ++i) {
+                finite = finite && fabsf(x[i]) < INFINITY;
+                sm.a[(j + i) * kTokRow + t] = x[i];
+            }
+        });
+        // A value that is no finite number must not reach the tokens before it by way of a weight of zero: such a chunk is summed one
+        // by one.
+        const bool one_by_one = __syncthreads_or(!finite);
+        // weighted scores with the values of the tokens
+#pragma unroll
+        for (int sb = 0; sb < A; ++sb) {
+            if (16 * sb < c.n && !one_by_one) {
+#pragma unroll 1
+                for (int i = 0; i < 4; ++i) {
+                    ulonglong2 p[A], p2[A];
+#pragma unroll
+                    for (int a = sb; a < A; ++a) {
+                        p[a] = pair4(sm.p[0] + (ty + 16 * a) * kTokRow + 16 * sb + 4 * i);
+                        if constexpr (kSsm) p2[a] = c.heads_here > 1 ? pair4(sm.p[1] + (ty + 16 * a) * kTokRow + 16 * sb + 4 * i) : p[a];
+                    }
+#pragma unroll
+                    for (int b = 0; b < 8; ++b) {
+                        const ulonglong2 v = pair4(sm.a + (tx + 16 * b) * kTokRow + 16 * sb + 4 * i);
+#pragma unroll
+                        for (int a = sb; a < A; ++a) {
+                            const ulonglong2 x = kSsm && b >= 4 ? p2[a] : p[a];      // (two heads are of 64 columns)
+                            fma2(acc[a][b], x.x, v.x), fma2(acc[a][b], x.y, v.y);
+                        }
                     }
                 }
             }
         }
-    }
 #pragma unroll
-    for (int a = 0; a < 4; ++a) {
-        const int t = ty + 16 * a;
-        if (t >= c.n) continue;
-        float* to = out + (size_t)(c.q0 + t) * src.heads * src.dv + c.col0;
+        for (int a = 0; a < A; ++a) {
+            const int t = ty + 16 * a;
+            if (t >= c.n) continue;
+            float* to = out + (size_t)(c.q0 + t) * src.heads * src.dv + c.col0;
 #pragma unroll
-        for (int b = 0; b < 8; ++b) {
-            const int j = tx + 16 * b;
-            const float2 x = unpack2(acc[a][b]);
-            float y = x.x + x.y;
-            if (one_by_one)
-                for (int i = 0; i <= t; ++i) y = fmaf(sm.p[kSsm && j >= second ? 1 : 0][t * kTokRow + i], sm.a[j * kTokRow + i], y);
-            if constexpr (kSsm) y = fmaf(src.skip[c.head + (j >= second ? 1 : 0)], sm.a[j * kTokRow + t], y);
-            if (j < c.cols) to[j] = y;
+            for (int b = 0; b < 8; ++b) {
+                const int j = tx + 16 * b;
+                const float2 x = unpack2(acc[a][b]);
+                float y = x.x + x.y;
+                if (one_by_one)
+                    for (int i = 0; i <= t; ++i) y = fmaf(sm.p[kSsm && j >= second ? 1 : 0][t * kTokRow + i], sm.a[j * kTokRow + i], y);
+                if constexpr (kSsm) y = fmaf(src.skip[c.head + (j >= second ? 1 : 0)], sm.a[j * kTokRow + t], y);
+                if (j < c.cols) to[j] = y;
+            }
         }
-    }
+    };
+    if (c.n > 32) with_blocks(std::integral_constant<int, 4>{});
+    else if (c.n > 16) with_blocks(std::integral_constant<int, 2>{});
+    else with_blocks(std::integral_constant<int, 1>{});
 }
 
 template <typename T, bool kSsm>

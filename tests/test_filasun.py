@@ -646,7 +646,7 @@ def test_decay_scan_in_chunks_as_products(heads, d, dv, dtype):
     assert K.library().li_decay_chunks_accepts(64, d) == 1 and K.library().li_decay_chunks_accepts(65, d) == 0
     ref_s, ref_o = state0.clone(), torch.zeros(T, heads * dv, device=dev)
     R.decay_scan(qkv, *at, decay, ref_s, q_start, slots, ref_o, heads, d, dv)
-    for length in (64, 17, 65):
+    for length in (64, 33, 32, 17, 16, 65):
         s, o = state0.clone(), torch.full((T, heads * dv), 7.0, device=dev)
         K.decay_scan(qkv, *at, decay, s, q_start, slots, o, heads, d, dv, chunks=K.ScanChunks(q_start.tolist(), slots.tolist(), dev, length))
         _close(o, ref_o, "float32", f"outputs, chunks of {length}")
@@ -683,7 +683,7 @@ def test_ssm_scan_in_chunks_as_products(heads, P, N, groups, dtype):
     assert K.library().li_ssm_chunks_accepts(64, heads, P, N, groups) == 1
     ref_s, ref_y = state0.clone(), torch.zeros(T, heads * P, device=dev)
     R.ssm_scan(xbc, proj, 5, dt_bias, A_log, D, ref_s, q_start, slots, ref_y, heads, P, N, groups)
-    for length in (64, 17, 65):
+    for length in (64, 33, 32, 17, 16, 65):
         s, y = state0.clone(), torch.full((T, heads * P), 7.0, device=dev)
         K.ssm_scan(xbc, proj, 5, dt_bias, A_log, D, s, q_start, slots, y, heads, P, N, groups, chunks=K.ScanChunks(q_start.tolist(), slots.tolist(), dev, length))
         _close(y, ref_y, "float32", f"outputs, chunks of {length}")
