@@ -1070,6 +1070,8 @@ __global__ void scan_carry_kernel(float* __restrict__ state, long long state_str
     const int dec_at = period > 0 ? h * period + (e - h * per_head) % period : h;
     float* st = state + (size_t)slot * state_stride + e;
     float S = *st;
+    int length = -1;
+    float power = 1.0f;                                    // a head's one decay to the power of a chunk's length, which is mostly the same
     for (int c0 = first; c0 < first + count; c0 += 8) {
         // eight chunks' end states and decays are asked for at once: they do not depend on S
         float z[8], dec[8];
@@ -1079,7 +1081,11 @@ __global__ void scan_carry_kernel(float* __restrict__ state, long long state_str
             const bool in = c < first + count;
             z[u] = in ? chunk_state[(size_t)c * elements + e] : 0.0f;
             // the chunk's decay: given, or a constant per token and head to the power of the chunk's length
-            dec[u] = !in ? 1.0f : chunk_decay ? chunk_decay[(size_t)c * per_chunk + dec_at] : powf(token_decay[h], (float)(seg[4 * c + 1] - seg[4 * c]));
+            if (in && !chunk_decay && seg[4 * c + 1] - seg[4 * c] != length) {
+                length = seg[4 * c + 1] - seg[4 * c];
+                power = powf(token_decay[h], (float)length);
+            }
+            dec[u] = !in ? 1.0f : chunk_decay ? chunk_decay[(size_t)c * per_chunk + dec_at] : power;
         }
 #pragma unroll
         for (int u = 0; u < 8; ++u) {
@@ -1092,10 +1098,17 @@ __global__ void scan_carry_kernel(float* __restrict__ state, long long state_str
     *st = S;
 }
 
+constexpr int kGatedEach = 4;       // elements a thread keeps
+
+// Threads for a group of gs elements: few elements each, up to 4,096 of them all in registers (a row of 1,536 columns in two loops of
+// 256 threads took 6.5 us, one of 3,072 13; so 3.1 and 4).  A function of the group's size alone: the order of its sum does not
+// depend on the step.
+int gated_threads(int gs) { return gs <= 1024 ? 256 : gs <= 2048 ? 512 : 1024; }
+
 // One block per (token, group).  mode 0: v = y silu(z), out = v rinv w; mode 1: out = y rinv w sigmoid(z); mode 2: out = y rinv w silu(z).
 template <typename T>
-__global__ void gated_rmsnorm_kernel(const float* __restrict__ y, const T* __restrict__ gate, int gate_stride, int gate_off, const float* __restrict__ w,
-                                     float eps, int mode, T* __restrict__ out, int n, int groups) {
+__global__ void __launch_bounds__(1024) gated_rmsnorm_kernel(const float* __restrict__ y, const T* __restrict__ gate, int gate_stride, int gate_off,
+                                                             const float* __restrict__ w, float eps, int mode, T* __restrict__ out, int n, int groups) {
     __shared__ float scratch[32];
     pdl_launch_dependents();
     pdl_wait();
@@ -1103,7 +1116,33 @@ __global__ void gated_rmsnorm_kernel(const float* __restrict__ y, const T* __res
     const int gs = n / groups;
     const float* yr = y + (size_t)t * n + (size_t)g * gs;
     const T* zr = gate + (size_t)t * gate_stride + gate_off + (size_t)g * gs;
+    T* o = out + (size_t)t * n + (size_t)g * gs;
     float ss = 0.0f;
+    if (gs <= kGatedEach * (int)blockDim.x) {
+        // asked for at once and kept
+        float v[kGatedEach], z[kGatedEach], wj[kGatedEach];
+#pragma unroll
+        for (int i = 0; i < kGatedEach; ++i) {
+            const int j = threadIdx.x + i * blockDim.x;
+            v[i] = j < gs ? yr[j] : 0.0f;
+            z[i] = j < gs ? to_float(zr[j]) : 0.0f;
+            wj[i] = j < gs ? w[g * gs + j] : 0.0f;
+        }
+#pragma unroll
+        for (int i = 0; i < kGatedEach; ++i) {
+            if (mode == 0) v[i] *= silu_f(z[i]);
+            if (threadIdx.x + i * blockDim.x < gs) ss += v[i] * v[i];
+        }
+        ss = block_sum(ss, scratch);
+        const float rinv = 1.0f / sqrtf(ss / (float)gs + eps);
+#pragma unroll
+        for (int i = 0; i < kGatedEach; ++i) {
+            const float x = v[i] * rinv * wj[i];
+            const int j = threadIdx.x + i * blockDim.x;
+            if (j < gs) o[j] = from_float<T>(mode == 0 ? x : mode == 1 ? x * sigmoid_f(z[i]) : x * silu_f(z[i]));
+        }
+        return;
+    }
     for (int j = threadIdx.x; j < gs; j += blockDim.x) {
         float v = yr[j];
         if (mode == 0) v *= silu_f(to_float(zr[j]));
@@ -1111,7 +1150,6 @@ __global__ void gated_rmsnorm_kernel(const float* __restrict__ y, const T* __res
     }
     ss = block_sum(ss, scratch);
     const float rinv = 1.0f / sqrtf(ss / (float)gs + eps);
-    T* o = out + (size_t)t * n + (size_t)g * gs;
     for (int j = threadIdx.x; j < gs; j += blockDim.x) {
         float v = yr[j];
         const float z = to_float(zr[j]);
@@ -1252,11 +1290,19 @@ static int scan_warps(int columns) {
     return w >= 16 ? 16 : w >= 8 ? 8 : w >= 4 ? 4 : w >= 2 ? 2 : 1;
 }
 
+// The same for whole sequences (`walks` of them, times heads): fewer warps a block where few blocks would each read a whole head's state
+// (one token of 12 heads of 128 x 128: 10.6 us in 12 blocks, 6.2 in 96).  A column's walk does not depend on the block it is in.
+static int scan_warps_whole(int columns, long long walks) {
+    int w = scan_warps(columns);
+    while (w > 2 && walks * ceil_div(columns, w * kWarpCols) < li_multiprocessors()) w /= 2;
+    return w;
+}
+
 template <typename T, int E>
 static int launch_ssm(const void* xbc, int C, const void* dt_raw, int dt_stride, const float* dt_bias, const float* A_log, const float* D,
                       float* state, long long state_stride, const int* q_start, const int* slots, float* y, int S, int heads, int P, int N,
                       int groups, const int* seg, int mode, float* chunk_state, float* chunk_decay, cudaStream_t stream) {
-    const int warps = scan_warps(P), cols = warps * kWarpCols;
+    const int warps = mode == kScanWhole ? scan_warps_whole(P, (long long)heads * S) : scan_warps(P), cols = warps * kWarpCols;
     const size_t smem = ((size_t)2 * kStage * 32 * E + kStage * cols + 2 * kStage) * sizeof(float);
     if (smem > 48 * 1024) cudaFuncSetAttribute(ssm_scan_kernel<T, E>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     cudaError_t e = li_launch_pdl(ssm_scan_kernel<T, E>, dim3(ceil_div(P, cols), heads, S), dim3(warps * 32), smem, stream, (const T*)xbc, C,
@@ -1294,7 +1340,7 @@ template <typename T, int E>
 static int launch_decay(const void* qkv, int stride, int q_off, int k_off, int v_off, const float* decay, float* state, long long state_stride,
                         const int* q_start, const int* slots, float* out, int S, int heads, int d, int dv, const int* seg, int mode,
                         float* chunk_state, cudaStream_t stream) {
-    const int warps = scan_warps(dv), cols = warps * kWarpCols;
+    const int warps = mode == kScanWhole ? scan_warps_whole(dv, (long long)heads * S) : scan_warps(dv), cols = warps * kWarpCols;
     const size_t smem = ((size_t)2 * kStage * 32 * E + kStage * cols) * sizeof(float);
     if (smem > 48 * 1024) cudaFuncSetAttribute(decay_scan_kernel<T, E>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     cudaError_t e = li_launch_pdl(decay_scan_kernel<T, E>, dim3(ceil_div(dv, cols), heads, S), dim3(warps * 32), smem, stream, (const T*)qkv, stride,
@@ -1598,10 +1644,10 @@ LI_EXPORT int li_gated_rmsnorm(const float* y, const void* gate, int dtype, int 
         return li_check_launch("gated_rmsnorm");
     }
     if (dtype == LI_F32)
-        e = li_launch_pdl(gated_rmsnorm_kernel<float>, dim3((unsigned)blocks), dim3(256), 0, stream, y, (const float*)gate, gate_stride, gate_off, w, eps,
+        e = li_launch_pdl(gated_rmsnorm_kernel<float>, dim3((unsigned)blocks), dim3(gated_threads(n / groups)), 0, stream, y, (const float*)gate, gate_stride, gate_off, w, eps,
                           mode, (float*)out, n, groups);
     else if (dtype == LI_BF16)
-        e = li_launch_pdl(gated_rmsnorm_kernel<bf16>, dim3((unsigned)blocks), dim3(256), 0, stream, y, (const bf16*)gate, gate_stride, gate_off, w, eps,
+        e = li_launch_pdl(gated_rmsnorm_kernel<bf16>, dim3((unsigned)blocks), dim3(gated_threads(n / groups)), 0, stream, y, (const bf16*)gate, gate_stride, gate_off, w, eps,
                           mode, (bf16*)out, n, groups);
     else
         return li_fail("gated norm: unknown dtype %d", dtype);
