@@ -31,9 +31,9 @@ int li_gemv_tcgen05_tiles(int N);
 bool li_gemv_tcgen05_accepts(const void* a, const void* w, int M, int N, int K);
 
 // Whether a product of few rows goes to the tcgen05 kernel with swapped operands rather than to the register-fed one
-// (register-fed / tcgen05, us, 8 and 64 rows: 3072 x 3072, the edge, 8.6 / 7.2 and 19.0 / 12.8; 3584 x 3584 9.4 / 8.1 and 20.8 /
-// 12.6; but 1536 x 3584 4.5 / 7.2 and 10.4 / 12.2, 1536 x 1536 2.9 / 6.2 and 5.8 / 10.6: few short tiles leave a split too little
-// to do).
+// (register-fed / tcgen05, us, 8 and 64 rows: 3072 x 3072, the edge, 8.9 / 6.8 and 19.3 / 9.2; 3584 x 3584 9.8 / 7.9 and 21.2 /
+// 10.2; 1536 x 3584 4.8 / 6.1 and 10.4 / 8.0, 1536 x 1536 2.9 / 4.6 and 5.7 / 6.5: few short tiles leave a split too little to do.
+// One line for every number of rows up to 64, drawn for few of them).
 static bool few_rows_take_tcgen05(int N, int K) {
     const int tiles = (N + 127) / 128, nkb = (K + 63) / 64;
     if (tiles >= 96) return true;                              // fills the GPU without a split of k

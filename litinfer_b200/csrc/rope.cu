@@ -270,9 +270,9 @@ int li_linear_gemv_tcgen05_rope(const void* a, const void* w, const float* bias,
 
 // Whether q|k|v of T <= 64 tokens with heads of 128 goes to the tcgen05 kernel rather than to the register-fed one, which is
 // never split along k here.  With few tiles the merge of the tcgen05 kernel's splits outweighs them however long the rows are:
-// register-fed / tcgen05, us, 8 tokens: 20 tiles of 128 rows, K 4096 9.9 / 8.7, 24 tiles, K 3072 9.1 / 8.3, but 18 tiles, K 4096
-// 5.6 / 8.2, 6 tiles, K 4096 4.5 / 8.8.  With more than 32 tokens the tcgen05 kernel wins from 8,192 columns of k on whatever the
-// tiles (33 tokens, 10 tiles 18.0 / 16.1, with 32 tokens 14.0 / 16.2).
+// register-fed / tcgen05, us, the products of 8 tokens: 20 tiles of 128 rows, K 4096 10.0 / 7.9, 24 tiles, K 3072 8.8 / 6.7, but 18
+// tiles, K 4096 6.1 / 7.2, 6 tiles, K 4096 4.3 / 5.7.  With more than 32 tokens the tcgen05 kernel wins from 8,192 columns of k on whatever the
+// tiles (33 tokens, 10 tiles 21.2 / 10.1; the lines for fewer stand where they were drawn with slower sums of a cluster).
 static bool few_tokens_rope_on_tcgen05(int T, int N, int K) {
     const int tiles = (N + 127) / 128, nkb = (K + 63) / 64;
     if (T > 32 && nkb >= 128) return true;
