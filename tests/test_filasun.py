@@ -688,3 +688,47 @@ def test_ssm_scan_in_chunks_as_products(heads, P, N, groups, dtype):
         K.ssm_scan(xbc, proj, 5, dt_bias, A_log, D, s, q_start, slots, y, heads, P, N, groups, chunks=K.ScanChunks(q_start.tolist(), slots.tolist(), dev, length))
         _close(y, ref_y, "float32", f"outputs, chunks of {length}")
         _close(s, ref_s, "float32", f"states, chunks of {length}")
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", DTYPES)
+def test_a_sequences_recurrence_does_not_depend_on_the_steps_others(dtype):
+    """A single sequence, whose columns go to more and smaller blocks, against the same one beside others: the same bits."""
+    from litinfer_b200 import kernels as K
+
+    dev, dt = torch.device("cuda:0"), _dt(dtype)
+    torch.manual_seed(5)
+    heads, d, S = 4, 64, 80
+    ssm_heads, P, N = 4, 64, 32
+    row, x, pr = (torch.randn(2, n, device=dev).to(dt) for n in (3 * heads * d, ssm_heads * P + 2 * N, ssm_heads))
+    decay = torch.tensor([0.9, 1.0, 0.5, 0.99], device=dev)
+    dt_bias, A_log, D = (0.5 * torch.randn(ssm_heads, device=dev) for _ in range(3))
+    first, first_ssm = torch.randn(1, heads * d * d, device=dev), torch.randn(1, ssm_heads * P * N, device=dev)
+    got = []
+    for n in (1, S):
+        q_start = torch.arange(0, 2 * n + 1, 2, dtype=torch.int32, device=dev)
+        slots = torch.arange(n, dtype=torch.int32, device=dev)
+        state, out = first.repeat(n, 1), torch.empty(2 * n, heads * d, device=dev)
+        K.decay_scan(row.repeat(n, 1), 0, heads * d, 2 * heads * d, decay, state, q_start, slots, out, heads, d, d)
+        state2, y = first_ssm.repeat(n, 1), torch.empty(2 * n, ssm_heads * P, device=dev)
+        K.ssm_scan(x.repeat(n, 1), pr.repeat(n, 1), 0, dt_bias, A_log, D, state2, q_start, slots, y, ssm_heads, P, N, 1)
+        got.append([t[-k:] for t, k in ((state, 1), (out, 2), (state2, 1), (y, 2))])
+    assert all(torch.equal(a, b) for a, b in zip(*got))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("n,groups", [(1024, 1), (1025, 1), (2048, 1), (2049, 1), (4096, 1), (4097, 1), (6144, 3)])
+def test_gated_norm_of_groups_kept_in_registers_and_not(n, groups, dtype):
+    import kernel_refs as R
+    from litinfer_b200 import kernels as K
+
+    dev, dt = torch.device("cuda:0"), _dt(dtype)
+    torch.manual_seed(n)
+    y32, w = torch.randn(3, n, device=dev), torch.randn(n, device=dev)
+    gate = torch.randn(3, n + 9, device=dev).to(dt)
+    for first, act in ((True, "sigmoid"), (False, "sigmoid"), (False, "silu")):
+        a, b = (torch.empty(3, n, device=dev, dtype=dt) for _ in range(2))
+        K.gated_rmsnorm(y32, gate, 4, w, 1e-5, groups, first, a, gate_act=act)
+        R.gated_rmsnorm(y32, gate, 4, w, 1e-5, groups, first, b, gate_act=act)
+        _close(a, b, dtype, f"gated norm, gate first {first}, {act}")
